@@ -1131,15 +1131,11 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     std::vector<SvdPolish> pol;
     std::vector<int> pol_of_sector(nsec, -1);
     DevBuf X, Gm, Wb, cst, cdiag;
-    // the rebuild's FP64 products are small: 16 x 16 tiles spread them over more SMs
-    const int tm = 16, tn = 16;
     auto add_gemm = [&](GemmPlan &g, int64_t c_off, int M, int N, GemmSeg seg) {
         const int sb = (int)g.segs.size();
-        g.tile_m = tm;
-        g.tile_n = tn;
+        g.tile_m = g.tile_n = kFp64Block;
         g.segs.push_back(seg);
-        for (int m0 = 0; m0 < M; m0 += tm)
-            for (int n0 = 0; n0 < N; n0 += tn) g.tiles.push_back({c_off, N, M, N, m0, n0, sb, sb + 1});
+        g.tiles.push_back({c_off, N, M, N, 0, 0, sb, sb + 1});
     };
     auto polish_pass = [&](const std::vector<SvdPolish> &pl_list, const DevBuf &dp, double shift) {
         GemmPlan gram;

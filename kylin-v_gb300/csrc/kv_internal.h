@@ -295,7 +295,12 @@ struct GemmTile {
     int64_t c_off;
     int ldc, M, N, m0, n0;
     int seg_begin, seg_end;
+    short tm = 0, tn = 0;  // FP64 path: outputs per CTA (step)
 };
+// FP64 path, values of GemmPlan::tile_m / tile_n: tiles are made one per output
+// block and cut by fp64_tiles when the plan is uploaded, or (task lists whose
+// size must not grow) made kFp64Coarse square, each CTA walking its tile.
+constexpr int kFp64Block = 1 << 30, kFp64Coarse = 32;
 // Tile shape of the tensor-core path (kv_tc.cu).
 constexpr int kMixedTileM = 128, kMixedTileN = 32;
 
@@ -319,6 +324,7 @@ struct SegX {
 
 struct GemmPlan;
 void plan_mixed(GemmPlan &g);  // slicing jobs of a plan built with the tensor-core tile shape
+void fp64_tiles(GemmPlan &g);  // one tile per output block -> tiles of about equal work
 
 struct GemmPlan {
     std::vector<GemmTile> tiles;
@@ -327,6 +333,7 @@ struct GemmPlan {
     double ref_flops = 0.0;  // sum of 8*M*N*K over the reference's zgemm pairs
     int max_k = 0;
     int tile_m = 0, tile_n = 0;
+    int fp64_threads = 256;  // CTA size of the FP64 path
     // tiles whose segments are all inactive at the launch's step write zeros
     // (false: they write nothing; for intermediates only read by active consumers)
     bool write_inactive = true;
@@ -343,6 +350,7 @@ struct GemmPlan {
     int64_t a_planes = 0, b_planes = 0, a_exps = 0, b_exps = 0;
     DevBuf d_ajobs, d_bjobs, d_xsegs, d_aitems, d_bitems;
     void upload() {
+        if (tile_m == kFp64Block) fp64_tiles(*this);
         d_tiles = upload_vec(tiles);
         d_segs = upload_vec(segs);
         if (tile_m == kMixedTileM && tile_n == kMixedTileN) plan_mixed(*this);

@@ -1,5 +1,8 @@
 // FP64 device kernels of the contraction engine: grouped block-sparse complex
 // GEMM, MPO mixing, block permutation, fills.
+#include <algorithm>
+#include <cmath>
+
 #include "kv_internal.h"
 
 namespace kv {
@@ -17,89 +20,96 @@ __device__ __forceinline__ void cfma(double2 &acc, double2 a, double2 b) {
 }
 
 // ------------------------------------------------------------------ GEMM
-// One CTA per output tile (T x T complex, T = 32 or 16), 256 threads,
-// (T/16) x (T/16) outputs per thread.  Each tile sums all block pairs
-// (segments) that accumulate into it, so no atomics are needed and the
-// summation order is fixed.  GB300 runs FP64 at a few multiply-adds per clock
-// per SM, so a tile's K loop is long in time: the 16 x 16 tiles put four
-// times as many CTAs (SMs) on the same product, for the small products of the
-// SVD's FP64 rebuild.
-constexpr int TK = 16;
+// Grouped FP64 GEMM: one CTA per output tile of tm x tn elements (tm tn <=
+// NT), each output summed by KS = NT / (tm tn) threads that share the tile's
+// K range: the contracted indices of all its segments are numbered
+// consecutively and thread slice ks takes those equal to ks mod KS; the KS
+// partial sums are added in a fixed tree, so the order is fixed and there are
+// no atomics.
+// What bounds it: the FP64 unit, two thread-operations per clock per SM (four
+// per complex multiply-add), so an operand pair read from L1/L2 for every
+// multiply-add (32 B per 2 clocks) is hidden and neither register blocking
+// nor shared-memory staging helps; what matters is that all SMs hold equal
+// shares of the multiply-adds.  The plan (fp64_tiles) therefore sizes tiles
+// by their work, and blocks smaller than a tile leave no thread idle (tm, tn
+// are any integers).  Against 32 x 32 tiles with K walked by the whole CTA
+// (which left most SMs idle): a D = 96 one-site Lanczos exponential 2047 ->
+// 788 us, the energy of 36 such sites 7.73 -> 2.33 ms, the adjoint of a D = 96
+// apply (one output of K ~ 5000 per SM) 6.06 -> 0.61 ms.
+constexpr int kSegBatch = 32;  // segment descriptors staged in shared memory at a time
 
-template <int T>
-__global__ void __launch_bounds__(256) k_gemm_fp64(const GemmTile *__restrict__ tiles,
-                                                   const GemmSeg *__restrict__ segs,
-                                                   const double2 *__restrict__ A,
-                                                   const double2 *__restrict__ B, double2 *__restrict__ C,
-                                                   double alpha, const int *skip, int step, int write_inactive) {
+// v with its sign flipped if flip is 0x80000000 (no FP64 operation)
+__device__ __forceinline__ double flip_sign(double v, int flip) {
+    return __hiloint2double(__double2hiint(v) ^ flip, __double2loint(v));
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ tiles,
+                                                  const GemmSeg *__restrict__ segs, const double2 *__restrict__ A,
+                                                  const double2 *__restrict__ B, double2 *__restrict__ C, double alpha,
+                                                  const int *skip, int step, int write_inactive, int cover) {
     if (skip && *skip) return;
-    constexpr int TM = T, TN = T, R = T / 16;  // R x R outputs per thread
-    constexpr int LOADS = (TM * TK + 255) / 256;
-    __shared__ double2 As[TK][TM + 1];
-    __shared__ double2 Bs[TK][TN + 1];
+    __shared__ GemmSeg sg[kSegBatch];
+    __shared__ double2 red[NT];
     const GemmTile t = tiles[blockIdx.x];
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    double2 acc[R][R] = {};
-    bool any = false;
-    for (int s = t.seg_begin; s < t.seg_end; ++s) {
-        const GemmSeg g = segs[s];
-        if (g.entry > step) continue;  // uniform over the CTA
-        any = true;
-        const double2 *a = A + g.a_off;
-        const double2 *b = B + g.b_off;
-        for (int k0 = 0; k0 < g.K; k0 += TK) {
-#pragma unroll
-            for (int r = 0; r < LOADS; ++r) {
-                int idx = tid + r * 256;
-                int m, k;
-                const bool a_kc = (g.opa == 0 || g.opa == 3);  // contiguous along k
-                if (a_kc) { m = idx / TK; k = idx % TK; }
-                else { m = idx % TM; k = idx / TM; }
-                int gm = t.m0 + m, gk = k0 + k;
-                double2 v = make_double2(0.0, 0.0);
-                if (gm < t.M && gk < g.K) {
-                    v = a_kc ? a[(int64_t)gm * g.lda + gk] : a[(int64_t)gk * g.lda + gm];
-                    if (g.opa == 1 || g.opa == 3) v.y = -v.y;
+    const int tid = threadIdx.x;
+    const int tm = t.tm, tn = t.tn, mn = tm * tn, KS = NT / mn;
+    const int ks = tid / mn, m = (tid % mn) / tn, n = tid % tn;
+    // cover > 0 (coarse task lists): the CTA walks the cover x cover outputs from (m0, n0) in tm x tn steps
+    const int m_end = cover > 0 ? min(t.M, t.m0 + cover) : min(t.M, t.m0 + tm);
+    const int n_end = cover > 0 ? min(t.N, t.n0 + cover) : min(t.N, t.n0 + tn);
+    for (int mb = t.m0; mb < m_end; mb += tm)
+        for (int nb = t.n0; nb < n_end; nb += tn) {
+            const int gm = mb + m, gn = nb + n;
+            const bool on = ks < KS && gm < m_end && gn < n_end;
+            double2 acc = make_double2(0.0, 0.0);
+            bool any = false;
+            int first = ks;  // this slice's first index within the next segment
+            for (int s0 = t.seg_begin; s0 < t.seg_end; s0 += kSegBatch) {
+                const int ns = min(kSegBatch, t.seg_end - s0);
+                __syncthreads();
+                for (int i = tid; i < ns; i += NT) sg[i] = segs[s0 + i];
+                __syncthreads();
+                for (int i = 0; i < ns; ++i) {
+                    if (sg[i].entry > step) continue;  // uniform over the CTA
+                    any = true;
+                    const int K = sg[i].K, lda = sg[i].lda, ldb = sg[i].ldb, opa = sg[i].opa, opb = sg[i].opb;
+                    if (on) {
+                        const bool akc = opa == 0 || opa == 3, bnc = opb == 0 || opb == 3;  // contiguous along k / n
+                        const int fa = (opa == 1 || opa == 3) ? (int)0x80000000 : 0;
+                        const int fb = (opb == 2 || opb == 3) ? (int)0x80000000 : 0;
+                        const int64_t da = akc ? 1 : lda, db = bnc ? ldb : 1;
+                        const double2 *pa = A + sg[i].a_off + (akc ? (int64_t)gm * lda : gm);
+                        const double2 *pb = B + sg[i].b_off + (bnc ? gn : (int64_t)gn * ldb);
+#pragma unroll 4
+                        for (int k = first; k < K; k += KS) {
+                            double2 a = pa[k * da], b = pb[k * db];
+                            a.y = flip_sign(a.y, fa);
+                            b.y = flip_sign(b.y, fb);
+                            cfma(acc, a, b);
+                        }
+                    }
+                    // (first - K) mod KS: the next segment continues the numbering
+                    if (KS > 1) {
+                        first = (first - K) % KS;
+                        if (first < 0) first += KS;
+                    }
                 }
-                As[k][m] = v;
-                int n;
-                const bool b_nc = (g.opb == 0 || g.opb == 3);  // contiguous along n
-                if (b_nc) { n = idx % TN; k = idx / TN; }
-                else { k = idx % TK; n = idx / TK; }
-                int gn = t.n0 + n;
-                gk = k0 + k;
-                double2 w = make_double2(0.0, 0.0);
-                if (gn < t.N && gk < g.K) {
-                    w = b_nc ? b[(int64_t)gk * g.ldb + gn] : b[(int64_t)gn * g.ldb + gk];
-                    if (g.opb == 2 || g.opb == 3) w.y = -w.y;
-                }
-                Bs[k][n] = w;
             }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < TK; ++kk) {
-                double2 a[R], b[R];
-#pragma unroll
-                for (int i = 0; i < R; ++i) {
-                    a[i] = As[kk][ty * R + i];
-                    b[i] = Bs[kk][tx * R + i];
+            for (int live = KS; live > 1;) {
+                const int half = (live + 1) / 2;
+                __syncthreads();
+                if (ks < live) red[tid] = acc;
+                __syncthreads();
+                if (ks < live - half) {
+                    acc.x += red[tid + half * mn].x;
+                    acc.y += red[tid + half * mn].y;
                 }
-#pragma unroll
-                for (int i = 0; i < R; ++i)
-#pragma unroll
-                    for (int j = 0; j < R; ++j) cfma(acc[i][j], a[i], b[j]);
+                live = half;
             }
-            __syncthreads();
-        }
-    }
-    if (!any && !write_inactive) return;
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-            int gm = t.m0 + ty * R + i, gn = t.n0 + tx * R + j;
-            if (gm < t.M && gn < t.N)
-                C[t.c_off + (int64_t)gm * t.ldc + gn] = make_double2(alpha * acc[i][j].x, alpha * acc[i][j].y);
+            if (!any && !write_inactive) return;  // uniform over the CTA
+            if (on && ks == 0)
+                C[t.c_off + (int64_t)gm * t.ldc + gn] = make_double2(alpha * acc.x, alpha * acc.y);
         }
 }
 
@@ -194,17 +204,58 @@ int grid_for(int64_t n, int threads) {
 
 }  // namespace
 
+// Tiles of the FP64 GEMM from one entry per output block (m0 = n0 = 0,
+// covering the block).  A tile's cost is its multiply-adds, outputs x K; tiles
+// are cut so that none exceeds a quarter of an SM's share of the plan, or
+// kMinTile multiply-adds (about 1 us of one SM's FP64 unit, what a CTA costs
+// to start), and never more than 256 outputs.
+void fp64_tiles(GemmPlan &g) {
+    constexpr double kMinTile = 1024.0;
+    std::vector<GemmTile> blocks;
+    blocks.swap(g.tiles);
+    std::vector<double> K(blocks.size(), 0.0);
+    double total = 0.0, top = 0.0;
+    for (size_t i = 0; i < blocks.size(); ++i) {
+        const GemmTile &b = blocks[i];
+        for (int s = b.seg_begin; s < b.seg_end; ++s) K[i] += g.segs[s].K;
+        total += K[i] * b.M * b.N;
+    }
+    const double target = std::max(kMinTile, total / (4.0 * std::max(1, ctx().num_sms)));
+    for (size_t i = 0; i < blocks.size(); ++i) {
+        const GemmTile &b = blocks[i];
+        const int area = (int)std::max(1.0, std::min(256.0, target / std::max(1.0, K[i])));
+        // nearly square, cut into equal parts
+        int tn = std::min(b.N, std::max(1, (int)std::sqrt((double)area)));
+        int tm = std::min(b.M, std::max(1, area / tn));
+        tn = std::min(b.N, std::max(1, area / tm));
+        tm = (b.M + (b.M + tm - 1) / tm - 1) / ((b.M + tm - 1) / tm);
+        tn = (b.N + (b.N + tn - 1) / tn - 1) / ((b.N + tn - 1) / tn);
+        GemmTile t = b;
+        t.tm = (short)tm;
+        t.tn = (short)tn;
+        for (t.m0 = 0; t.m0 < b.M; t.m0 += tm)
+            for (t.n0 = 0; t.n0 < b.N; t.n0 += tn) g.tiles.push_back(t);
+        top = std::max(top, (double)tm * tn * K[i]);
+    }
+    g.fp64_threads = top <= 2.0 * kMinTile ? 64 : 256;
+    if (g.fp64_threads == 64)
+        for (auto &t : g.tiles)
+            if (t.tm * t.tn > 64) { g.fp64_threads = 256; break; }
+}
+
 void launch_gemm_fp64(const GemmPlan &p, const double2 *A, const double2 *B, double2 *C, double alpha,
                       const int *skip, int step) {
     if (p.tiles.empty()) return;
-    KV_REQUIRE(p.tile_m == p.tile_n && (p.tile_m == 32 || p.tile_m == 16 || p.tile_m == 0), KV_EINVAL,
-               "internal: FP64 GEMM tiles are 32 x 32 or 16 x 16");
-    if (p.tile_m == 16)
-        k_gemm_fp64<16><<<(unsigned)p.tiles.size(), 256, 0, ctx().stream>>>(
-            p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C, alpha, skip, step, p.write_inactive ? 1 : 0);
+    KV_REQUIRE(p.tile_m == p.tile_n && (p.tile_m == kFp64Block || p.tile_m == kFp64Coarse), KV_EINVAL,
+               "internal: GEMM plan not prepared for the FP64 path");
+    const int cover = p.tile_m == kFp64Coarse ? kFp64Coarse : 0;
+    const unsigned n = (unsigned)p.tiles.size();
+    if (p.fp64_threads == 64)
+        k_gemm_fp64<64><<<n, 64, 0, ctx().stream>>>(p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C, alpha,
+                                                    skip, step, p.write_inactive ? 1 : 0, cover);
     else
-        k_gemm_fp64<32><<<(unsigned)p.tiles.size(), 256, 0, ctx().stream>>>(
-            p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C, alpha, skip, step, p.write_inactive ? 1 : 0);
+        k_gemm_fp64<256><<<n, 256, 0, ctx().stream>>>(p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C,
+                                                      alpha, skip, step, p.write_inactive ? 1 : 0, cover);
     counted();
     KV_CUDA(cudaGetLastError());
 }

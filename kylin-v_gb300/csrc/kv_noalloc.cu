@@ -100,7 +100,12 @@ void arena_product(Arena &ar, const Meta &A, const double2 *a, const Meta &B, co
     c = static_cast<double2 *>(ar.take(std::max<int64_t>(1, out.nelem) * sizeof(double2)));
     std::vector<int64_t> offs;
     for (auto &blk : out.blocks) offs.push_back(blk.off);
-    build_tiles(P, offs, kTileM(KV_FP64), kTileN(KV_FP64));
+    // coarse tiles: the task list's size is part of the scratch bound
+    build_tiles(P, offs, kFp64Coarse, kFp64Coarse);
+    for (auto &t : P.gemm.tiles) {
+        t.tm = (short)std::min(16, t.M);
+        t.tn = (short)std::min(16, t.N);
+    }
     Views vw;
     put(ar, vw, P.gemm.d_tiles, P.gemm.tiles);
     put(ar, vw, P.gemm.d_segs, P.gemm.segs);
