@@ -974,17 +974,15 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
             SvdSector s{};
             s.m = rows[ri].len;
             s.n = cols[ci].len;
-            // FP64: tall T with accumulated V.  Mixed: T's columns are the
-            // singular vectors the polish needs (right ones for L->R, left
-            // ones for R->L), so no rotations are accumulated; T may be wide.
-            s.transposed = mixed ? (l2r ? 1 : 0) : (s.m < s.n ? 1 : 0);
+            // T's left vectors are, in FP64, the factor kept orthonormal (U for
+            // L->R, V for R->L); mixed: the singular vectors of the other side,
+            // which the polish needs.  T may be wide.
+            s.transposed = mixed == l2r ? 1 : 0;
             s.p = s.transposed ? s.n : s.m;
             s.q = s.transposed ? s.m : s.n;
             s.t_off = P.t_elems;
-            s.v_off = P.v_elems;
             s.s_off = P.s_elems;
             P.t_elems += (int64_t)s.p * s.q;
-            if (!mixed) P.v_elems += (int64_t)s.q * s.q;
             P.s_elems += s.q;
             P.max_q = std::max(P.max_q, s.q);
             rows[ri].kept = std::min(s.m, s.n);
@@ -1001,8 +999,7 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     P.upload();
     const size_t cb = mixed ? sizeof(float2) : sizeof(double2);
     DevBuf T(std::max<int64_t>(1, P.t_elems) * sizeof(double2));
-    DevBuf Us(std::max<int64_t>(1, P.t_elems) * cb), V(std::max<int64_t>(1, P.v_elems) * cb);
-    DevBuf Vs(std::max<int64_t>(1, P.v_elems) * cb);
+    DevBuf Us(std::max<int64_t>(1, P.t_elems) * cb);
     DevBuf S(std::max<int64_t>(1, P.s_elems) * sizeof(double));
     DevBuf status(std::max<size_t>(1, 2 * P.secs.size()) * sizeof(int));  // sweeps, then QR ranks
     svd_gather(P, A.data(), T.as<double2>());
@@ -1036,8 +1033,7 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
             qr_ranks = true;
         }
     } else {
-        svd_jacobi(P, T.as<double2>(), V.as<double2>(), status.as<int>(), 60, 1e-15);
-        svd_finalize(P, T.as<double2>(), V.as<double2>(), Us.as<double2>(), Vs.as<double2>(), S.as<double>());
+        svd_fp64(P, T.as<double2>(), Us.as<double2>(), S.as<double>(), status.as<int>(), 60, 1e-15);
     }
     std::vector<double> sv(P.s_elems);
     std::vector<int> st(2 * P.secs.size());
@@ -1260,15 +1256,42 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     out.U = DTensor::make(mu, extended);  // the added states' other side stays zero
     out.V = DTensor::make(mv, extended);
     if (!mixed) {
-        std::vector<SvdScatter> su, svs;
-        for (size_t i = 0; i < pu.size(); ++i)
-            su.push_back({out.U->meta.blocks[i].off, pu[i].sector, 0, pu[i].pos, pu[i].len, kfin[pu[i].sector],
-                          l2r ? 0 : 1, pu[i].kept});
-        for (size_t i = 0; i < pv.size(); ++i)
-            svs.push_back({out.V->meta.blocks[i].off, pv[i].sector, 1, pv[i].pos, pv[i].len, kfin[pv[i].sector],
-                           l2r ? 1 : 0, pv[i].kept});
-        svd_scatter(su, P, Us.as<double2>(), Vs.as<double2>(), S.as<double>(), out.U->data());
-        svd_scatter(svs, P, Us.as<double2>(), Vs.as<double2>(), S.as<double>(), out.V->data());
+        // the orthonormal factor from T's left vectors; the other one is the
+        // projection of the sector matrix onto them, S V^H = U^H A or U S = A V:
+        // A[i, c] = T[i + c p] (L->R) or conj(T[c + i p]) (R->L), both
+        // contiguous along the contracted index
+        std::vector<SvdScatter> orth;
+        std::vector<SvdDense> dense;
+        std::vector<int64_t> y_off(nsec, 0);
+        int64_t y_elems = 0;
+        GemmPlan other;
+        for (int s_ = 0; s_ < nsec; ++s_) {
+            const SvdSector &sc = P.secs[s_];
+            const int k = kfin[s_];
+            if (k <= 0) continue;
+            y_off[s_] = y_elems;
+            if (l2r) add_gemm(other, y_elems, k, sc.n, GemmSeg{sc.t_off, sc.t_off, sc.m, sc.p, sc.p, 3, 1});
+            else add_gemm(other, y_elems, sc.m, k, GemmSeg{sc.t_off, sc.t_off, sc.n, sc.p, sc.p, 3, 1});
+            y_elems += (int64_t)k * (l2r ? sc.n : sc.m);
+        }
+        DevBuf Y(std::max<int64_t>(1, y_elems) * sizeof(double2));
+        other.upload();
+        if (l2r) launch_gemm_fp64(other, Us.as<double2>(), T.as<double2>(), Y.as<double2>(), 1.0, nullptr);
+        else launch_gemm_fp64(other, T.as<double2>(), Us.as<double2>(), Y.as<double2>(), 1.0, nullptr);
+        for (size_t i = 0; i < pu.size(); ++i) {
+            const int s_ = pu[i].sector, k = kfin[s_];
+            const int64_t o = out.U->meta.blocks[i].off;
+            if (l2r) orth.push_back({o, s_, 0, pu[i].pos, pu[i].len, k, pu[i].kept});
+            else dense.push_back({o, y_off[s_], 0, pu[i].pos, pu[i].len, k, k, 0, pu[i].kept});
+        }
+        for (size_t i = 0; i < pv.size(); ++i) {
+            const int s_ = pv[i].sector, k = kfin[s_];
+            const int64_t o = out.V->meta.blocks[i].off;
+            if (l2r) dense.push_back({o, y_off[s_], 1, pv[i].pos, pv[i].len, k, P.secs[s_].n, 0, 0});
+            else orth.push_back({o, s_, 1, pv[i].pos, pv[i].len, k, 0});
+        }
+        svd_scatter(orth, P, Us.as<double2>(), l2r ? out.U->data() : out.V->data());
+        svd_scatter_dense(dense, Y.as<double2>(), l2r ? out.V->data() : out.U->data());
         if (!extended) return out;
         // ---- SA: the new directions of the kept side (gs_ortho,
         // util/allocation.h:260-320).  Each new vector's entries are drawn
@@ -1302,7 +1325,7 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
         DevBuf Pb(std::max<int64_t>(1, x_elems) * sizeof(double2));
         X = DevBuf(std::max<int64_t>(1, x_elems) * sizeof(double2));
         upload_bytes(X.p, xr.data(), xr.size() * sizeof(double2));
-        sa_basis(sas, P, Us.as<double2>(), Vs.as<double2>(), Bd.as<double2>());
+        sa_basis(sas, P, Us.as<double2>(), Bd.as<double2>());
         GemmPlan proj, back;  // C = B^H X, P = B C
         std::vector<SvdPolish> pl;
         int64_t g_elems = 0;
@@ -1386,15 +1409,15 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     for (size_t i = 0; i < pu.size(); ++i) {
         const int s_ = pu[i].sector;
         const SvdPolish &pl = pol2[pol2_of_sector[s_]];
-        if (side == 0) du.push_back({out.U->meta.blocks[i].off, pl.x_off, 0, pu[i].pos, pu[i].len, pl.k, pl.ldx, 0});
-        else du.push_back({out.U->meta.blocks[i].off, y_off[s_], 0, pu[i].pos, pu[i].len, pl.k, pl.k, 0});
+        if (side == 0) du.push_back({out.U->meta.blocks[i].off, pl.x_off, 0, pu[i].pos, pu[i].len, pl.k, pl.ldx, 0, pl.k});
+        else du.push_back({out.U->meta.blocks[i].off, y_off[s_], 0, pu[i].pos, pu[i].len, pl.k, pl.k, 0, pl.k});
     }
     for (size_t i = 0; i < pv.size(); ++i) {
         const int s_ = pv[i].sector;
         const SvdPolish &pl = pol2[pol2_of_sector[s_]];
         if (side == 0)
-            dv.push_back({out.V->meta.blocks[i].off, y_off[s_], 1, pv[i].pos, pv[i].len, pl.k, P.secs[s_].n, 0});
-        else dv.push_back({out.V->meta.blocks[i].off, pl.x_off, 1, pv[i].pos, pv[i].len, pl.k, pl.ldx, 1});
+            dv.push_back({out.V->meta.blocks[i].off, y_off[s_], 1, pv[i].pos, pv[i].len, pl.k, P.secs[s_].n, 0, 0});
+        else dv.push_back({out.V->meta.blocks[i].off, pl.x_off, 1, pv[i].pos, pv[i].len, pl.k, pl.ldx, 1, 0});
     }
     svd_scatter_dense(du, side == 0 ? X.as<double2>() : Y.as<double2>(), out.U->data());
     svd_scatter_dense(dv, side == 0 ? Y.as<double2>() : X.as<double2>(), out.V->data());

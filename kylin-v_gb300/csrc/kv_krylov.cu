@@ -9,7 +9,6 @@
 #include <cooperative_groups.h>
 #include <mutex>
 #include "kv_internal.h"
-#include "kv_jacobi.cuh"
 
 namespace kv {
 

@@ -2,11 +2,9 @@
 // split (holstein/svd.h:443-614).
 //
 // Each charge sector's dense matrix is gathered as T (p x q, column-major;
-// T = A or T = A^H) and factorised by one CTA:
-//  * FP64 mode: T tall (p >= q), one-sided (Hestenes) Jacobi with round-robin
-//    ordering and accumulated rotations (k_svd_jacobi), sorted by descending
-//    singular value (k_svd_finalize);
-//  * mixed mode: T oriented so the wanted singular vectors are its columns, a
+// T = A or T = A^H) and factorised:
+//  * FP64 mode: kv_svd64.cu;
+//  * mixed mode, one CTA a sector: T oriented so the wanted singular vectors are its columns, a
 //    pivoted Householder reduction of its rows to the numerical rank, then
 //    FP32 one-sided Jacobi on the rank-r factor, all in shared memory
 //    (k_svd_qrj, the Jacobi with the columns in registers); sectors beyond
@@ -26,8 +24,6 @@ namespace kv {
 
 namespace {
 
-constexpr int ST = 256;
-
 __global__ void __launch_bounds__(256) k_svd_gather(const SvdGather *__restrict__ g, const SvdSector *__restrict__ secs,
                                                     const double2 *__restrict__ A, double2 *__restrict__ T) {
     const SvdGather d = g[blockIdx.x];
@@ -39,89 +35,6 @@ __global__ void __launch_bounds__(256) k_svd_gather(const SvdGather *__restrict_
         if (!s.transposed) T[s.t_off + (d.row_off + i) + (int64_t)(d.col_off + j) * s.p] = v;
         else { v.y = -v.y; T[s.t_off + (d.col_off + j) + (int64_t)(d.row_off + i) * s.p] = v; }
     }
-}
-
-template <class R>
-struct Cx;
-template <>
-struct Cx<double> { using T = double2; };
-template <>
-struct Cx<float> { using T = float2; };
-
-template <class R>
-__device__ __forceinline__ void warp_sum3(R &a, R &b, R &cr, R &ci) {
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-        cr += __shfl_xor_sync(0xffffffffu, cr, o);
-        ci += __shfl_xor_sync(0xffffffffu, ci, o);
-    }
-}
-
-// One CTA per sector, NT threads.  status[sector] = sweeps used (negative:
-// no convergence within max_sweeps).
-template <class R, int NT>
-__global__ void __launch_bounds__(NT) k_svd_jacobi(const SvdSector *__restrict__ secs, typename Cx<R>::T *__restrict__ T,
-                                                   typename Cx<R>::T *__restrict__ V, int *status, int max_sweeps,
-                                                   R tol) {
-    using C = typename Cx<R>::T;
-    const SvdSector s = secs[blockIdx.x];
-    const int p = s.p, q = s.q;
-    C *t = T + s.t_off;
-    C *v = V + s.v_off;
-    for (int64_t e = threadIdx.x; e < (int64_t)q * q; e += NT) {
-        C one;
-        one.x = (e % q) == (e / q) ? R(1) : R(0);
-        one.y = R(0);
-        v[e] = one;
-    }
-    __syncthreads();
-    const int qe = q + (q & 1);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = NT / 32;
-    __shared__ int rotated;
-    int sweep = 0;
-    bool converged = (q < 2);
-    for (; sweep < max_sweeps && !converged; ++sweep) {
-        if (threadIdx.x == 0) rotated = 0;
-        __syncthreads();
-        for (int r = 0; r < qe - 1; ++r) {
-            for (int pi = warp; pi < qe / 2; pi += nw) {
-                int c0, c1;
-                kvj::tournament_pair(qe, r, pi, c0, c1);
-                if (c1 >= q) continue;
-                C *x = t + (int64_t)c0 * p, *y = t + (int64_t)c1 * p;
-                R a = 0, b = 0, cr = 0, ci = 0;
-                for (int i = lane; i < p; i += 32) {
-                    C xi = x[i], yi = y[i];
-                    a += xi.x * xi.x + xi.y * xi.y;
-                    b += yi.x * yi.x + yi.y * yi.y;
-                    cr += xi.x * yi.x + xi.y * yi.y;
-                    ci += xi.x * yi.y - xi.y * yi.x;
-                }
-                warp_sum3<R>(a, b, cr, ci);
-                kvj::Rot<R> rot;
-                if (!kvj::make_rotation<R>(a, b, cr, ci, tol, rot)) continue;
-                if (lane == 0) rotated = 1;
-                for (int i = lane; i < p; i += 32) {
-                    C xi = x[i], yi = y[i];
-                    kvj::rotate_pair(rot, xi.x, xi.y, yi.x, yi.y);
-                    x[i] = xi;
-                    y[i] = yi;
-                }
-                C *vx = v + (int64_t)c0 * q, *vy = v + (int64_t)c1 * q;
-                for (int i = lane; i < q; i += 32) {
-                    C xi = vx[i], yi = vy[i];
-                    kvj::rotate_pair(rot, xi.x, xi.y, yi.x, yi.y);
-                    vx[i] = xi;
-                    vy[i] = yi;
-                }
-            }
-            __syncthreads();
-        }
-        converged = (rotated == 0);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) status[blockIdx.x] = converged ? sweep : -sweep;
 }
 
 // Mixed mode: one-sided Jacobi in FP32 without accumulated rotations.  T is
@@ -950,42 +863,34 @@ __global__ void __launch_bounds__(512, 1) k_svd_qr_g(const SvdSector *__restrict
     if (threadIdx.x == 0) ranks[blockIdx.x] = r;
 }
 
-// singular values (as double), descending order, normalised U columns
-template <class R>
-__global__ void __launch_bounds__(256) k_svd_finalize(const SvdSector *__restrict__ secs,
-                                                      const typename Cx<R>::T *__restrict__ T,
-                                                      const typename Cx<R>::T *__restrict__ V,
-                                                      typename Cx<R>::T *__restrict__ Us,
-                                                      typename Cx<R>::T *__restrict__ Vs, double *__restrict__ S) {
-    using C = typename Cx<R>::T;
+// singular values (as double), descending order, normalised columns
+__global__ void __launch_bounds__(256) k_svd_finalize(const SvdSector *__restrict__ secs, const float2 *__restrict__ T,
+                                                      float2 *__restrict__ Us, double *__restrict__ S) {
     const SvdSector s = secs[blockIdx.x];
     const int p = s.p, q = s.q;
-    extern __shared__ unsigned char sv_raw[];  // q norms, in the Jacobi's precision
-    R *sv = reinterpret_cast<R *>(sv_raw);
+    extern __shared__ float sv[];  // q norms
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = 256 / 32;
     for (int j = warp; j < q; j += nw) {
-        R a = 0;
+        float a = 0;
         for (int i = lane; i < p; i += 32) {
-            C x = T[s.t_off + (int64_t)j * p + i];
+            const float2 x = T[s.t_off + (int64_t)j * p + i];
             a += x.x * x.x + x.y * x.y;
         }
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) sv[j] = sqrt(a);
+        if (lane == 0) sv[j] = sqrtf(a);
     }
     __syncthreads();
     for (int j = warp; j < q; j += nw) {
-        const R sj = sv[j];
+        const float sj = sv[j];
         int rank = 0;
         for (int i = 0; i < q; ++i) rank += (sv[i] > sj) || (sv[i] == sj && i < j);
-        const R inv = sj > R(0) ? R(1) / sj : R(0);
+        const float inv = sj > 0.f ? 1.f / sj : 0.f;
         for (int i = lane; i < p; i += 32) {
-            C x = T[s.t_off + (int64_t)j * p + i];
+            float2 x = T[s.t_off + (int64_t)j * p + i];
             x.x *= inv;
             x.y *= inv;
             Us[s.t_off + (int64_t)rank * p + i] = x;
         }
-        if (V)
-            for (int i = lane; i < q; i += 32) Vs[s.v_off + (int64_t)rank * q + i] = V[s.v_off + (int64_t)j * q + i];
         if (lane == 0) S[s.s_off + rank] = sj;
     }
 }
@@ -1122,22 +1027,25 @@ __global__ void k_scatter_dense(const SvdDense *__restrict__ d_, const double2 *
     const int64_t n = (int64_t)d.len * d.kept;
     for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
         double2 v;
+        int64_t dst = e;
         if (d.side == 0) {
             const int i = (int)(e / d.kept), j = (int)(e % d.kept);
+            dst = (int64_t)i * d.out_ld + j;
             v = d.ctrans ? M[d.m_off + (int64_t)j * d.ld + d.pos + i] : M[d.m_off + (int64_t)(d.pos + i) * d.ld + j];
         } else {
             const int j = (int)(e / d.len), c = (int)(e % d.len);
             v = d.ctrans ? M[d.m_off + (int64_t)(d.pos + c) * d.ld + j] : M[d.m_off + (int64_t)j * d.ld + d.pos + c];
         }
         if (d.ctrans) v.y = -v.y;
-        out[d.out_off + e] = v;
+        out[d.out_off + dst] = v;
     }
 }
 
+// FP64 mode: the orthonormal factor's blocks from the sorted left vectors of
+// T (T = A where U is kept, T = A^H where V^H is: V^H[j, r] = conj(V[r, j]))
 __global__ void __launch_bounds__(256) k_svd_scatter(const SvdScatter *__restrict__ d_,
                                                      const SvdSector *__restrict__ secs,
-                                                     const double2 *__restrict__ Us, const double2 *__restrict__ Vs,
-                                                     const double *__restrict__ S, double2 *__restrict__ out) {
+                                                     const double2 *__restrict__ Us, double2 *__restrict__ out) {
     const SvdScatter d = d_[blockIdx.x];
     const SvdSector s = secs[d.sector];
     const int64_t n = (int64_t)d.len * d.kept;
@@ -1146,39 +1054,22 @@ __global__ void __launch_bounds__(256) k_svd_scatter(const SvdScatter *__restric
         int64_t dst;
         if (d.side == 0) { i = (int)(e / d.kept); j = (int)(e % d.kept); dst = (int64_t)i * d.ld + j; }
         else { j = (int)(e / d.len); i = (int)(e % d.len); dst = e; }
-        const int r = d.pos + i;
-        double2 val;
-        if (d.side == 0) {  // U_A[r, j]
-            val = s.transposed ? Vs[s.v_off + (int64_t)j * s.q + r] : Us[s.t_off + (int64_t)j * s.p + r];
-        } else {  // Vt_A[j, r] = conj(V_A[r, j])
-            val = s.transposed ? Us[s.t_off + (int64_t)j * s.p + r] : Vs[s.v_off + (int64_t)j * s.q + r];
-            val.y = -val.y;
-        }
-        if (d.scale_s) {
-            const double sj = S[s.s_off + j];
-            val.x *= sj;
-            val.y *= sj;
-        }
+        double2 val = Us[s.t_off + (int64_t)j * s.p + d.pos + i];
+        if (d.side == 1) val.y = -val.y;
         out[d.out_off + dst] = val;
     }
 }
 
-// SA-1TDVP: B[r, j] = U_A[r, j] (side 0) or conj(V_A[r, j]) (side 1), the
-// sources k_svd_scatter reads
+// SA-1TDVP: B[r, j] = U[r, j] (side 0) or conj(V[r, j]) (side 1), the sources
+// k_svd_scatter reads
 __global__ void __launch_bounds__(256) k_sa_basis(const SaSector *__restrict__ sa, const SvdSector *__restrict__ secs,
-                                                  const double2 *__restrict__ Us, const double2 *__restrict__ Vs,
-                                                  double2 *__restrict__ B) {
+                                                  const double2 *__restrict__ Us, double2 *__restrict__ B) {
     const SaSector d = sa[blockIdx.x];
     const SvdSector s = secs[d.sector];
     for (int64_t e = threadIdx.x; e < (int64_t)d.n * d.kept; e += blockDim.x) {
         const int r = (int)(e / d.kept), j = (int)(e % d.kept);
-        double2 v;
-        if (d.side == 0) {
-            v = s.transposed ? Vs[s.v_off + (int64_t)j * s.q + r] : Us[s.t_off + (int64_t)j * s.p + r];
-        } else {
-            v = s.transposed ? Us[s.t_off + (int64_t)j * s.p + r] : Vs[s.v_off + (int64_t)j * s.q + r];
-            v.y = -v.y;
-        }
+        double2 v = Us[s.t_off + (int64_t)j * s.p + r];
+        if (d.side == 1) v.y = -v.y;
         B[d.b_off + e] = v;
     }
 }
@@ -1270,36 +1161,19 @@ void svd_gather(const SvdPlan &p, const double2 *A, double2 *T) {
     KV_CUDA(cudaGetLastError());
 }
 
-void svd_jacobi(const SvdPlan &p, double2 *T, double2 *V, int *status, int max_sweeps, double tol) {
-    if (p.secs.empty()) return;
-    k_svd_jacobi<double, ST><<<(unsigned)p.secs.size(), ST, 0, ctx().stream>>>(p.d_secs.as<SvdSector>(), T, V,
-                                                                                status, max_sweeps, tol);
-    counted();
-    KV_CUDA(cudaGetLastError());
-}
-
-void svd_finalize(const SvdPlan &p, const double2 *T, const double2 *V, double2 *Us, double2 *Vs, double *S) {
-    if (p.secs.empty()) return;
-    k_svd_finalize<double><<<(unsigned)p.secs.size(), 256, sizeof(double) * p.max_q, ctx().stream>>>(
-        p.d_secs.as<SvdSector>(), T, V, Us, Vs, S);
-    counted();
-    KV_CUDA(cudaGetLastError());
-}
-
-void svd_scatter(const std::vector<SvdScatter> &sc, const SvdPlan &p, const double2 *Us, const double2 *Vs,
-                 const double *S, double2 *out) {
+void svd_scatter(const std::vector<SvdScatter> &sc, const SvdPlan &p, const double2 *Us, double2 *out) {
     if (sc.empty()) return;
     DevBuf d = upload_vec(sc);
     k_svd_scatter<<<(unsigned)sc.size(), 256, 0, ctx().stream>>>(d.as<SvdScatter>(), p.d_secs.as<SvdSector>(), Us,
-                                                                  Vs, S, out);
+                                                                  out);
     counted();
     KV_CUDA(cudaGetLastError());
 }
 
-void sa_basis(const std::vector<SaSector> &v, const SvdPlan &p, const double2 *Us, const double2 *Vs, double2 *B) {
+void sa_basis(const std::vector<SaSector> &v, const SvdPlan &p, const double2 *Us, double2 *B) {
     if (v.empty()) return;
     DevBuf d = upload_vec(v);
-    k_sa_basis<<<(unsigned)v.size(), 256, 0, ctx().stream>>>(d.as<SaSector>(), p.d_secs.as<SvdSector>(), Us, Vs, B);
+    k_sa_basis<<<(unsigned)v.size(), 256, 0, ctx().stream>>>(d.as<SaSector>(), p.d_secs.as<SvdSector>(), Us, B);
     counted();
     KV_CUDA(cudaGetLastError());
 }
@@ -1412,8 +1286,8 @@ bool svd_qrjacobi_f32(const SvdPlan &p, const double2 *T64, float2 *Us, double *
 
 void svd_finalize_f32(const SvdPlan &p, const float2 *T, float2 *Us, double *S) {
     if (p.secs.empty()) return;
-    k_svd_finalize<float><<<(unsigned)p.secs.size(), 256, sizeof(double) * p.max_q, ctx().stream>>>(
-        p.d_secs.as<SvdSector>(), T, nullptr, Us, nullptr, S);
+    k_svd_finalize<<<(unsigned)p.secs.size(), 256, sizeof(double) * p.max_q, ctx().stream>>>(p.d_secs.as<SvdSector>(),
+                                                                                             T, Us, S);
     counted();
     KV_CUDA(cudaGetLastError());
 }

@@ -6,10 +6,9 @@
 namespace kv {
 
 struct SvdSector {
-    int64_t t_off;  // T (p x q, column-major) and its sorted U copy
-    int64_t v_off;  // V (q x q, column-major) and its sorted copy
+    int64_t t_off;  // T (p x q, column-major) and its sorted left singular vectors
     int64_t s_off;  // q singular values
-    int p, q;       // FP64 path: tall orientation, p >= q; mixed path: see op_svd
+    int p, q;       // orientation: see op_svd
     int transposed; // 0: T = A (m = p, n = q); 1: T = A^H (m = q, n = p)
     int m, n;       // sector matrix of A (rows x cols)
 };
@@ -19,9 +18,9 @@ struct SvdGather {  // one block of A into its sector matrix
     int sector, row_off, col_off, nrows, ncols;
 };
 
-struct SvdScatter {  // one output block of U (side 0) or S.V^H / V^H (side 1)
+struct SvdScatter {  // one output block of U (side 0) or V^H (side 1), FP64 mode's orthonormal factor
     int64_t out_off;
-    int sector, side, pos, len, kept, scale_s;
+    int sector, side, pos, len, kept;
     int ld;  // side 0: the block's row length (>= kept; larger where SA-1TDVP adds columns)
 };
 
@@ -43,7 +42,7 @@ struct SaOut {
 struct SvdPlan {
     std::vector<SvdSector> secs;
     std::vector<SvdGather> gathers;
-    int64_t t_elems = 0, v_elems = 0, s_elems = 0;
+    int64_t t_elems = 0, s_elems = 0;
     int max_q = 0;
     DevBuf d_secs, d_gathers;
     void upload() { d_secs = upload_vec(secs); d_gathers = upload_vec(gathers); }
@@ -62,6 +61,7 @@ struct SvdPolish {
 struct SvdDense {
     int64_t out_off, m_off;
     int side, pos, len, kept, ld, ctrans;
+    int out_ld;  // side 0: the block's row length (kept; larger where SA-1TDVP adds columns)
 };
 
 void svd_gather(const SvdPlan &p, const double2 *A, double2 *T);
@@ -93,12 +93,13 @@ void svd_chol(const DevBuf &pol, int npol, double2 *G, int *status, double *diag
 void svd_trsm(const DevBuf &pol, const std::vector<int> &item_pol, const std::vector<int> &item_row0,
               const double2 *G, double2 *X, int kmax);
 void svd_scatter_dense(const std::vector<SvdDense> &d, const double2 *M, double2 *out);
-void svd_jacobi(const SvdPlan &p, double2 *T, double2 *V, int *status, int max_sweeps, double tol);
-void svd_finalize(const SvdPlan &p, const double2 *T, const double2 *V, double2 *Us, double2 *Vs, double *S);
-void svd_scatter(const std::vector<SvdScatter> &sc, const SvdPlan &p, const double2 *Us, const double2 *Vs,
-                 const double *S, double2 *out);
-// FP64 path: the kept vectors of each SA sector into B (after svd_finalize)
-void sa_basis(const std::vector<SaSector> &v, const SvdPlan &p, const double2 *Us, const double2 *Vs, double2 *B);
+// FP64 mode: the min(p, q) left singular vectors of every sector's T,
+// normalised and sorted (column-major p x min(p, q) at t_off), and the singular
+// values (kv_svd64.cu); status[sector] = Jacobi sweeps, negative: no convergence
+void svd_fp64(const SvdPlan &p, const double2 *T, double2 *U, double *S, int *status, int max_sweeps, double tol);
+void svd_scatter(const std::vector<SvdScatter> &sc, const SvdPlan &p, const double2 *Us, double2 *out);
+// FP64 path: the kept vectors of each SA sector into B (after svd_fp64)
+void sa_basis(const std::vector<SaSector> &v, const SvdPlan &p, const double2 *Us, double2 *B);
 // x -= y over n elements
 void sa_subtract(double2 *x, const double2 *y, int64_t n);
 void sa_scatter(const std::vector<SaOut> &v, const double2 *X, double2 *out);

@@ -1,0 +1,613 @@
+// FP64 block SVD (svd_impl's factorisation, holstein/svd.h:296-440, in FP64
+// mode; the SA-1TDVP split, holstein/svd.h:443-614, in every mode): for each
+// charge sector T (p x q, column-major) the p-dimensional left singular
+// vectors and the singular values, sorted.  The caller orients T so that these
+// are the factor it keeps orthonormal and forms the other factor as the
+// projection of the sector matrix onto them.
+//
+// One thread-block cluster per sector:
+//  1. Pivoted Householder reduction of T's rows from the right: at step k the
+//     row with the largest trailing norm is reflected onto its position k and
+//     the reflector applied to the rows not yet pivoted, so T Q = M is
+//     row-pivoted lower triangular (p x r, r <= min(p, q); r is smaller only
+//     if the remaining rows are exactly zero) and T's left vectors are M's.
+//     One-sided Jacobi on such a graded triangular factor converges in fewer
+//     sweeps than on T, and a wide T loses its surplus columns (Drmac and
+//     Veselic, SIAM J. Matrix Anal. Appl. 29 (2008) 1322).
+//  2. One-sided Jacobi on M's columns, round-robin pairs, one barrier a round.
+//  3. Column norms = singular values, sorted; normalised columns = vectors.
+//     Columns of norm exactly zero are completed to an orthonormal set.
+//
+// What bounds it: the FP64 unit.  GB300 issues two FP64 thread-operations per
+// clock per SM, so a warp's FP64 instruction holds its quarter of the SM for
+// 64 clocks, and one SM per sector (17 to 32 sectors on 152 SMs) left most of
+// the chip idle.  Hence: a cluster of SMs per sector, rows (1) and pairs (2)
+// dealt over its SMs, the data in L2 (a round moves a few columns a warp, far
+// less time than its arithmetic); no accumulated rotations; sums of several
+// values reduced together (each shuffle level halves the values a lane
+// carries, then the lanes); and rotation angles from FP32 arithmetic on the
+// mantissas -- an angle off by 1e-7 only leaves 1e-7 of the pair's cosine for
+// the next sweep -- with (cs, s) completed to a unitary pair in FP64.
+// Measured (17 sectors of about 101 x 101, 10 sweeps): 297 ms with one SM a
+// sector, accumulated rotations and FP64 angles, 7.5 ms now; the truncated
+// product's error against numpy 4.1e-14 -> 2.7e-15.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "kv_internal.h"
+#include "kv_svd.h"
+
+namespace kv {
+
+namespace {
+
+constexpr int NT = 256, NW = NT / 32;
+constexpr int kXStage = 4096;  // longest pivot row staged in shared memory
+
+__device__ __forceinline__ double2 ldg2(const double2 *p) { return __ldcg(p); }
+__device__ __forceinline__ void stg2(double2 *p, double2 v) { __stcg(p, v); }
+
+// sums of two / four values over groups of G lanes, every lane of the group
+// receiving them: at the first levels a lane passes on half of its values, so
+// the four sums cost 2 + 1 + ... additions instead of 4 a level
+template <int G>
+__device__ __forceinline__ void group_sum2(double &a, double &b) {
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 1;
+    double keep = hi ? b : a, give = hi ? a : b;
+    keep += __shfl_xor_sync(0xFFFFFFFFu, give, 1);
+#pragma unroll
+    for (int o = 2; o < G; o <<= 1) keep += __shfl_xor_sync(0xFFFFFFFFu, keep, o);
+    const double other = __shfl_xor_sync(0xFFFFFFFFu, keep, 1);
+    a = hi ? other : keep;
+    b = hi ? keep : other;
+}
+template <int G>
+__device__ __forceinline__ void group_sum4(double &a, double &b, double &c, double &d) {
+    const int lane = threadIdx.x & 31;
+    const bool h1 = lane & 1, h2 = lane & 2;
+    double k0 = h1 ? c : a, k1 = h1 ? d : b, g0 = h1 ? a : c, g1 = h1 ? b : d;
+    k0 += __shfl_xor_sync(0xFFFFFFFFu, g0, 1);
+    k1 += __shfl_xor_sync(0xFFFFFFFFu, g1, 1);
+    double v = h2 ? k1 : k0;
+    v += __shfl_xor_sync(0xFFFFFFFFu, h2 ? k0 : k1, 2);
+#pragma unroll
+    for (int o = 4; o < G; o <<= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    // lane bits (h1, h2): (0,0) holds a, (0,1) b, (1,0) c, (1,1) d
+    const int base = lane & ~3;
+    a = __shfl_sync(0xFFFFFFFFu, v, base);
+    c = __shfl_sync(0xFFFFFFFFu, v, base + 1);
+    b = __shfl_sync(0xFFFFFFFFu, v, base + 2);
+    d = __shfl_sync(0xFFFFFFFFu, v, base + 3);
+}
+
+// x = m 2^e with |m| in [1, 2) as FP32 (truncated to 24 bits); zero and
+// subnormal x give m = 0.  Integer operations only.
+__device__ __forceinline__ float mantissa(double x, int &e) {
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const int E = (hi >> 20) & 0x7FF;
+    e = E - 1023;
+    if (E == 0) return 0.f;
+    return __int_as_float((hi & (int)0x80000000) | (127 << 23) | ((hi & 0xFFFFF) << 3) | (int)(lo >> 29));
+}
+// 2^e as FP32, e clamped to [-126, 127]
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((min(max(e, -126), 127) + 127) << 23); }
+// an FP32 value as FP64 (exact; FP32 subnormals as zero).  Integer operations only.
+__device__ __forceinline__ double widen(float x) {
+    const int u = __float_as_int(x), E = (u >> 23) & 0xFF, m = u & 0x7FFFFF;
+    if (E == 0) return 0.0;
+    return __hiloint2double((u & (int)0x80000000) | ((E - 127 + 1023) << 20) | (m >> 3), m << 29);
+}
+
+// The Jacobi rotation of a column pair with |x|^2 = a, |y|^2 = b, x^H y = c
+// != 0 (x' = cs x - conj(s) y, y' = s x + cs y): tau = t c/|c| with
+// t = sign(z) / (|z| + sqrt(1 + z^2)), z = (b - a) / (2|c|), in FP32; then
+// cs = 1 / sqrt(1 + |tau|^2) and s = cs tau in FP64 (two Newton steps on the
+// FP32 reciprocal square root), unitary to FP64 rounding.
+__device__ __forceinline__ void rotation(double a, double b, double cr, double ci, double &cs, double &sr,
+                                         double &si) {
+    int er, ei, ed;
+    const float mr = mantissa(cr, er), mi = mantissa(ci, ei), md = mantissa(b - a, ed);
+    const int ec = mr == 0.f ? ei : mi == 0.f ? er : max(er, ei);
+    const float fr = mr == 0.f ? 0.f : mr * pow2f(er - ec), fi = mi == 0.f ? 0.f : mi * pow2f(ei - ec);
+    const float rn = rsqrtf(fr * fr + fi * fi);  // 1 / (|c| 2^-ec)
+    const float z0 = 0.5f * md * rn;             // z 2^(ec - ed), |z0| < 1
+    const int ez = ed - ec;
+    double tr, ti;
+    if (ez > 60) {  // |z| > 2^58: tau = c / (b - a), which may be below FP32's range
+        const double inv = 1.0 / (b - a);
+        tr = cr * inv;
+        ti = ci * inv;
+    } else {
+        const float z = z0 * pow2f(ez);
+        const float t = copysignf(__fdividef(1.f, fabsf(z) + sqrtf(fmaf(z, z, 1.f))), z);
+        tr = widen(t * fr * rn);
+        ti = widen(t * fi * rn);
+    }
+    const double w = fma(tr, tr, fma(ti, ti, 1.0));  // in [1, 2]
+    int ew;
+    const float fw = mantissa(w, ew);
+    double y = widen(rsqrtf(fw * pow2f(ew)));
+    y = fma(y * 0.5, fma(-w * y, y, 1.0), y);
+    y = fma(y * 0.5, fma(-w * y, y, 1.0), y);
+    cs = y;
+    sr = y * tr;
+    si = y * ti;
+}
+
+struct Svd64Sector {
+    int64_t t_off;   // T, the row workspace and M: p * q elements each
+    int64_t s_off;   // q singular values
+    int64_t k_off;   // min(p, q) diagonal entries and norms
+    int64_t r_off;   // p row flags
+    int p, q;
+};
+
+// candidate of one CTA for the next pivot row
+struct Cand {
+    double v;
+    int row, bad;
+};
+
+template <int G, int EPL>
+__global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ secs, const double2 *__restrict__ T,
+                                              double2 *U, double2 *M, double *S, double2 *alph, double *nrm,
+                                              int *done, Cand *cand, int *flags, int *status,
+                                              int max_sweeps, double tol) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ double2 xs[];  // the pivot row's tail (q <= kXStage)
+    __shared__ double wv[NW];
+    __shared__ int wi[NW], wbad[NW];
+    __shared__ double2 sc[2];  // v0 and (beta, nu) of the step
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int sec = blockIdx.x / C;
+    const Svd64Sector s = secs[sec];
+    const int p = s.p, q = s.q, kmax = min(p, q);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double2 *t = T + s.t_off;
+    double2 *w = U + s.t_off;  // row-major workspace, later the sorted vectors
+    double2 *m = M + s.t_off;  // column-major p x r
+    double2 *al = alph + s.k_off;
+    double *nv = nrm + s.k_off;
+    int *dn = done + s.r_off;  // step a row was the pivot of, or -1
+    Cand *cd = cand + (int64_t)sec * 2 * 16;
+    int *fl = flags + sec * 4;
+
+    // best (value, row) of the CTA into slot b; NaN wins, so it is seen
+    auto publish = [&](double bv, int bi, int bad, int slot) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ov = __shfl_xor_sync(0xFFFFFFFFu, bv, o);
+            const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
+            bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, o);
+            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+        }
+        if (lane == 0) { wv[warp] = bv; wi[warp] = bi; wbad[warp] = bad; }
+        __syncthreads();
+        if (tid == 0) {
+            for (int x = 1; x < NW; ++x) {
+                bad |= wbad[x];
+                if (wv[x] > bv || (wv[x] == bv && wi[x] < bi)) { bv = wv[x]; bi = wi[x]; }
+            }
+            Cand *o = cd + slot * 16 + rank;
+            __stcg(&o->v, bv);
+            __stcg(&o->row, bi);
+            __stcg(&o->bad, bad);
+        }
+    };
+
+    // ---- rows i = rank, rank + C, ... belong to this CTA, row i to warp (i / C) % NW
+    {
+        double bv = -1.0;
+        int bi = 0x7FFFFFFF, bad = 0;
+        for (int i = rank + C * warp; i < p; i += C * NW) {
+            double a = 0.0;
+            for (int c = lane; c < q; c += 32) {
+                const double2 v = t[i + (int64_t)c * p];
+                w[(int64_t)i * q + c] = v;
+                a = fma(v.x, v.x, fma(v.y, v.y, a));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+            if (lane == 0) dn[i] = -1;
+            if (!isfinite(a)) bad = 1;
+            if (a > bv) { bv = a; bi = i; }
+        }
+        if (rank == 0 && tid < 4) fl[tid] = 0;
+        publish(bv, bi, bad, 0);
+    }
+    cl.sync();
+
+    // ---- pivoted Householder on the rows
+    int r = 0;
+    bool nonfinite = false;
+    for (int k = 0;; ++k) {
+        double mv = -1.0;
+        int ip = 0x7FFFFFFF, bad = 0;
+        for (int x = 0; x < C; ++x) {  // the same in every CTA
+            const Cand *o = cd + (k & 1) * 16 + x;
+            const double v = __ldcg(&o->v);
+            const int i = __ldcg(&o->row);
+            bad |= __ldcg(&o->bad);
+            if (v > mv || (v == mv && i < ip)) { mv = v; ip = i; }
+        }
+        if (bad) { nonfinite = true; break; }
+        if (k >= kmax || !(mv > 0.0) || ip >= p) break;
+        r = k + 1;
+        const double2 *xr = w + (int64_t)ip * q;
+        const bool staged = q <= kXStage;
+        if (staged)
+            for (int c = k + tid; c < q; c += NT) xs[c] = ldg2(xr + c);
+        // u = conj(x), alpha = -e^{i phi} |u| (phi = arg u_0), v = u - alpha e_0,
+        // beta = 2 / |v|^2 = 1 / (|u| (|u| + |u_0|))
+        if (warp == 0) {
+            const double2 x0 = ldg2(xr + k);
+            const double nu = sqrt(mv), a0 = sqrt(fma(x0.x, x0.x, x0.y * x0.y));
+            const double ia = a0 > 0.0 ? 1.0 / a0 : 0.0;
+            const double pr = a0 > 0.0 ? x0.x * ia : 1.0, pi = -x0.y * ia;  // e^{i phi}
+            if (lane == 0) {
+                sc[0] = make_double2(pr * (a0 + nu), pi * (a0 + nu));
+                sc[1] = make_double2(1.0 / (nu * (nu + a0)), 0.0);
+                if (ip % C == rank) {
+                    al[k] = make_double2(-pr * nu, pi * nu);  // conj(alpha): the pivot row's entry k
+                    dn[ip] = k;
+                }
+            }
+        }
+        __syncthreads();
+        const double2 v0 = sc[0];
+        const double beta = sc[1].x;
+        double bv = -1.0;
+        int bi = 0x7FFFFFFF, isbad = 0;
+        for (int i = rank + C * warp; i < p; i += C * NW) {
+            if (dn[i] >= 0) continue;  // warp-uniform
+            double2 *wr = w + (int64_t)i * q;
+            double sr = 0.0, si = 0.0;  // sum_c w_c v_c, v_c = conj(x_c) for c > k, v_k = v0
+            for (int c = k + lane; c < q; c += 32) {
+                const double2 xc = staged ? xs[c] : ldg2(xr + c);
+                const double2 vc = c == k ? v0 : make_double2(xc.x, -xc.y);
+                const double2 a = wr[c];
+                sr = fma(a.x, vc.x, fma(-a.y, vc.y, sr));
+                si = fma(a.x, vc.y, fma(a.y, vc.x, si));
+            }
+            group_sum2<32>(sr, si);
+            const double fr = beta * sr, fi = beta * si;
+            double ta = 0.0;
+            for (int c = k + lane; c < q; c += 32) {
+                const double2 xc = staged ? xs[c] : ldg2(xr + c);
+                const double2 cv = c == k ? make_double2(v0.x, -v0.y) : xc;  // conj(v_c)
+                double2 a = wr[c];
+                a.x = fma(-fr, cv.x, fma(fi, cv.y, a.x));
+                a.y = fma(-fr, cv.y, fma(-fi, cv.x, a.y));
+                wr[c] = a;
+                if (c > k) ta = fma(a.x, a.x, fma(a.y, a.y, ta));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ta += __shfl_xor_sync(0xFFFFFFFFu, ta, o);
+            if (!isfinite(ta)) isbad = 1;
+            if (ta > bv) { bv = ta; bi = i; }
+        }
+        publish(bv, bi, isbad, (k + 1) & 1);
+        cl.sync();
+    }
+    if (nonfinite) {  // uniform over the cluster: reported by the host
+        if (rank == 0)
+            for (int j = tid; j < q; j += NT) S[s.s_off + j] = nan("");
+        if (rank == 0 && tid == 0) status[sec] = 0;
+        return;
+    }
+    // ---- M, column-major: a row pivoted at step kk has its entry kk and zeros after it
+    for (int i = rank + C * warp; i < p; i += C * NW) {
+        const int kk = dn[i];
+        for (int c = lane; c < r; c += 32) {
+            double2 v = w[(int64_t)i * q + c];
+            if (kk >= 0 && c >= kk) v = c == kk ? al[kk] : make_double2(0.0, 0.0);
+            stg2(m + (int64_t)c * p + i, v);
+        }
+    }
+    cl.sync();
+
+    // ---- one-sided Jacobi on M's r columns: a round's pairs two (G = 16) or
+    // one (G = 32) a warp, dealt over the CTAs first
+    const int qe = r + (r & 1), m1 = qe - 1, np = qe / 2;
+    constexpr int PW = 32 / G;  // pairs a warp
+    const int gl = lane % G, sub = lane / G;
+    const double tol2 = tol * tol;
+    int sweep = 0;
+    bool converged = r < 2;
+    for (; sweep < max_sweeps && !converged; ++sweep) {
+        if (rank == 0 && tid == 0) __stcg(fl + (sweep + 1) % 3, 0);  // last read two sweeps ago
+        bool rotated = false;
+        for (int rr = 0; rr < m1; ++rr) {
+            for (int wt = rank + C * warp; wt * PW < np; wt += C * NW) {  // warp-uniform
+                const int pi = wt * PW + sub;
+                int c0 = 0, c1 = r;
+                if (pi < np) {
+                    if (pi > 0) { c0 = pi - 1 + rr; if (c0 >= m1) c0 -= m1; ++c0; }
+                    c1 = qe - 2 - pi + rr; if (c1 >= m1) c1 -= m1; ++c1;
+                    if (c0 > c1) { const int x = c0; c0 = c1; c1 = x; }
+                }
+                const bool act = c1 < r;  // group-uniform
+                double2 *x = m + (int64_t)c0 * p, *y = m + (int64_t)(act ? c1 : c0) * p;
+                double a = 0.0, b = 0.0, cr = 0.0, ci = 0.0;
+                double2 xv[EPL > 0 ? EPL : 1], yv[EPL > 0 ? EPL : 1];
+                if constexpr (EPL > 0) {
+#pragma unroll
+                    for (int e = 0; e < EPL; ++e) {
+                        const int i = gl + e * G;
+                        const bool in = act && i < p;
+                        xv[e] = in ? ldg2(x + i) : make_double2(0.0, 0.0);
+                        yv[e] = in ? ldg2(y + i) : make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                    for (int e = 0; e < EPL; ++e) {
+                        if (e * G >= p) break;  // uniform
+                        a = fma(xv[e].x, xv[e].x, fma(xv[e].y, xv[e].y, a));
+                        b = fma(yv[e].x, yv[e].x, fma(yv[e].y, yv[e].y, b));
+                        cr = fma(xv[e].x, yv[e].x, fma(xv[e].y, yv[e].y, cr));
+                        ci = fma(xv[e].x, yv[e].y, fma(-xv[e].y, yv[e].x, ci));
+                    }
+                } else {
+                    if (act)
+                        for (int i = gl; i < p; i += G) {
+                            const double2 xi = ldg2(x + i), yi = ldg2(y + i);
+                            a = fma(xi.x, xi.x, fma(xi.y, xi.y, a));
+                            b = fma(yi.x, yi.x, fma(yi.y, yi.y, b));
+                            cr = fma(xi.x, yi.x, fma(xi.y, yi.y, cr));
+                            ci = fma(xi.x, yi.y, fma(-xi.y, yi.x, ci));
+                        }
+                    __syncwarp();
+                }
+                group_sum4<G>(a, b, cr, ci);
+                const double ac2 = fma(cr, cr, ci * ci);
+                // |c|^2 <= tol^2 a b: the pair is orthogonal to the tolerance
+                if (!act || !(ac2 > tol2 * a * b)) continue;
+                double cs, sr, si;
+                rotation(a, b, cr, ci, cs, sr, si);
+                rotated = true;
+                if constexpr (EPL > 0) {
+#pragma unroll
+                    for (int e = 0; e < EPL; ++e) {
+                        const int i = gl + e * G;
+                        if (e * G >= p) break;
+                        const double2 xo = xv[e], yo = yv[e];
+                        const double nxr = fma(cs, xo.x, -fma(sr, yo.x, si * yo.y));
+                        const double nxi = fma(cs, xo.y, -fma(sr, yo.y, -si * yo.x));
+                        const double nyr = fma(cs, yo.x, fma(sr, xo.x, -si * xo.y));
+                        const double nyi = fma(cs, yo.y, fma(sr, xo.y, si * xo.x));
+                        if (i < p) {
+                            stg2(x + i, make_double2(nxr, nxi));
+                            stg2(y + i, make_double2(nyr, nyi));
+                        }
+                    }
+                } else {
+                    for (int i = gl; i < p; i += G) {
+                        const double2 xo = ldg2(x + i), yo = ldg2(y + i);
+                        stg2(x + i, make_double2(fma(cs, xo.x, -fma(sr, yo.x, si * yo.y)),
+                                                 fma(cs, xo.y, -fma(sr, yo.y, -si * yo.x))));
+                        stg2(y + i, make_double2(fma(cs, yo.x, fma(sr, xo.x, -si * xo.y)),
+                                                 fma(cs, yo.y, fma(sr, xo.y, si * xo.x))));
+                    }
+                }
+            }
+            if (rr == m1 - 1 && rotated) __stcg(fl + sweep % 3, 1);
+            __syncwarp();
+            cl.sync();
+        }
+        converged = __ldcg(fl + sweep % 3) == 0;  // the same in every CTA
+    }
+    if (rank == 0 && tid == 0) status[sec] = converged ? sweep : -sweep;
+
+    // ---- norms, then sorted singular values and normalised columns
+    for (int j = rank + C * warp; j < kmax; j += C * NW) {
+        double a = 0.0;
+        if (j < r)
+            for (int i = lane; i < p; i += 32) {
+                const double2 v = ldg2(m + (int64_t)j * p + i);
+                a = fma(v.x, v.x, fma(v.y, v.y, a));
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+        if (lane == 0) __stcg(nv + j, sqrt(a));
+    }
+    cl.sync();
+    int zeros = 0;  // columns of norm zero, the same in every warp
+    for (int j0 = 0; j0 < kmax; j0 += 32)
+        zeros += __popc(__ballot_sync(0xFFFFFFFFu, j0 + lane < kmax && !(__ldcg(nv + min(j0 + lane, kmax - 1)) > 0.0)));
+    for (int j = rank + C * warp; j < kmax; j += C * NW) {
+        const double sj = __ldcg(nv + j);
+        int pos = 0;
+        for (int i = lane; i < kmax; i += 32) {
+            const double si = __ldcg(nv + i);
+            pos += (si > sj) || (si == sj && i < j);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) pos += __shfl_xor_sync(0xFFFFFFFFu, pos, o);
+        const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
+        if (sj > 0.0)
+            for (int i = lane; i < p; i += 32) {
+                const double2 v = ldg2(m + (int64_t)j * p + i);
+                stg2(w + (int64_t)pos * p + i, make_double2(v.x * inv, v.y * inv));
+            }
+        if (lane == 0) S[s.s_off + pos] = sj;
+    }
+    if (rank == 0)
+        for (int j = kmax + tid; j < q; j += NT) S[s.s_off + j] = 0.0;
+    if (zeros == 0) return;  // uniform over the cluster
+    cl.sync();
+    if (rank != 0) return;
+    // ---- the last `zeros` vectors: unit vectors e_i made orthogonal (twice)
+    // to all before them, i the row those leave the most of e_i in
+    for (int j = kmax - zeros; j < kmax; ++j) {
+        double best = -1.0;
+        int bi = 0x7FFFFFFF;
+        for (int i = tid; i < p; i += NT) {
+            double a = 1.0;
+            for (int c = 0; c < j; ++c) {
+                const double2 v = ldg2(w + (int64_t)c * p + i);
+                a -= fma(v.x, v.x, v.y * v.y);
+            }
+            if (a > best) { best = a; bi = i; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ov = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+            const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
+            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+        }
+        if (lane == 0) { wv[warp] = best; wi[warp] = bi; }
+        __syncthreads();
+        for (int x = 0; x < NW; ++x)
+            if (wv[x] > best || (wv[x] == best && wi[x] < bi)) { best = wv[x]; bi = wi[x]; }
+        double2 *u = w + (int64_t)j * p;
+        for (int i = tid; i < p; i += NT) stg2(u + i, make_double2(i == bi ? 1.0 : 0.0, 0.0));
+        __syncthreads();
+        for (int pass = 0; pass < 2; ++pass)
+            for (int c = 0; c < j; ++c) {
+                double sr = 0.0, si = 0.0;  // u_c^H u, by every warp alike
+                for (int i = lane; i < p; i += 32) {
+                    const double2 a = ldg2(w + (int64_t)c * p + i), b = ldg2(u + i);
+                    sr = fma(a.x, b.x, fma(a.y, b.y, sr));
+                    si = fma(a.x, b.y, fma(-a.y, b.x, si));
+                }
+                group_sum2<32>(sr, si);
+                __syncthreads();
+                for (int i = tid; i < p; i += NT) {
+                    const double2 a = ldg2(w + (int64_t)c * p + i);
+                    double2 b = ldg2(u + i);
+                    b.x -= a.x * sr - a.y * si;
+                    b.y -= a.x * si + a.y * sr;
+                    stg2(u + i, b);
+                }
+                __syncthreads();
+            }
+        double a = 0.0;
+        for (int i = lane; i < p; i += 32) {
+            const double2 b = ldg2(u + i);
+            a = fma(b.x, b.x, fma(b.y, b.y, a));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+        const double inv = 1.0 / sqrt(a);
+        __syncthreads();
+        for (int i = tid; i < p; i += NT) {
+            const double2 b = ldg2(u + i);
+            stg2(u + i, make_double2(b.x * inv, b.y * inv));
+        }
+        __syncthreads();
+    }
+}
+
+constexpr int kMaxDevices = 64;
+constexpr int kXBytes = kXStage * (int)sizeof(double2);
+
+// once per device: the kernels may use kXBytes of dynamic shared memory and
+// clusters of 16; returns whether a cluster of 16 can be resident
+bool svd64_setup(int dev) {
+    static std::mutex mu;
+    static int state[kMaxDevices] = {};  // 0 unknown, 1: clusters of 16, -1: up to 8
+    KV_REQUIRE(dev >= 0 && dev < kMaxDevices, KV_EINVAL, "device index out of range");
+    std::lock_guard<std::mutex> lk(mu);
+    if (state[dev] == 0) {
+        const void *ks[] = {(const void *)k_svd64<16, 4>, (const void *)k_svd64<16, 8>, (const void *)k_svd64<16, 16>,
+                            (const void *)k_svd64<16, 0>, (const void *)k_svd64<32, 2>, (const void *)k_svd64<32, 4>,
+                            (const void *)k_svd64<32, 8>, (const void *)k_svd64<32, 0>};
+        int ok = 1;
+        for (const void *k : ks) {
+            KV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kXBytes));
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+                (void)cudaGetLastError();
+                ok = 0;
+                continue;
+            }
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(16);
+            cfg.blockDim = dim3(NT);
+            cfg.dynamicSmemBytes = kXBytes;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim = {16, 1, 1};
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                n = 0;
+            }
+            if (n < 1) ok = 0;
+        }
+        state[dev] = ok ? 1 : -1;
+    }
+    return state[dev] > 0;
+}
+
+}  // namespace
+
+void svd_fp64(const SvdPlan &P, const double2 *T, double2 *U, double *S, int *status, int max_sweeps, double tol) {
+    if (P.secs.empty()) return;
+    const bool c16 = svd64_setup(ctx().device);
+    const int nsec = (int)P.secs.size();
+    std::vector<Svd64Sector> secs;
+    int64_t k_elems = 0, r_elems = 0;
+    int max_p = 1, max_q = 1, max_k = 1;
+    for (auto &s : P.secs) {
+        secs.push_back({s.t_off, s.s_off, k_elems, r_elems, s.p, s.q});
+        k_elems += std::min(s.p, s.q);
+        r_elems += s.p;
+        max_p = std::max(max_p, s.p);
+        max_q = std::max(max_q, s.q);
+        max_k = std::max(max_k, std::min(s.p, s.q));
+    }
+    // Cluster size: eight pairs keep one CTA's FP64 units busy (two a warp, a
+    // warp per quarter of the SM), and the sectors together should fit one
+    // wave of SMs.  Where four pairs a CTA still fit, one pair a warp (G = 32)
+    // halves a round's time.
+    const int pairs = (max_k + 1) / 2, cmax = c16 ? 16 : 8;
+    int C = 1;
+    while (C < cmax && C * 8 < pairs && nsec * C * 2 <= ctx().num_sms) C *= 2;
+    bool wide = C * 4 >= pairs;
+    if (!wide && C < cmax && C * 8 >= pairs && nsec * C * 2 <= ctx().num_sms) {
+        C *= 2;
+        wide = C * 4 >= pairs;
+    }
+    DevBuf ds = upload_vec(secs);
+    DevBuf M(std::max<int64_t>(1, P.t_elems) * sizeof(double2));
+    DevBuf al(std::max<int64_t>(1, k_elems) * sizeof(double2)), nv(std::max<int64_t>(1, k_elems) * sizeof(double));
+    DevBuf dn(std::max<int64_t>(1, r_elems) * sizeof(int));
+    DevBuf cd((size_t)nsec * 32 * sizeof(Cand)), fl((size_t)nsec * 4 * sizeof(int));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nsec * C));
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = (size_t)std::min(max_q, kXStage) * sizeof(double2);
+    cfg.stream = ctx().stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    auto launch = [&](auto kernel) {
+        KV_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const Svd64Sector *)ds.as<Svd64Sector>(), T, U, M.as<double2>(), S,
+                                   al.as<double2>(), nv.as<double>(), dn.as<int>(), cd.as<Cand>(),
+                                   fl.as<int>(), status, max_sweeps, tol));
+    };
+    // a column's elements stay in registers between the sums and the rotation up to 256 rows
+    if (wide) {
+        if (max_p <= 64) launch(k_svd64<32, 2>);
+        else if (max_p <= 128) launch(k_svd64<32, 4>);
+        else if (max_p <= 256) launch(k_svd64<32, 8>);
+        else launch(k_svd64<32, 0>);
+    } else {
+        if (max_p <= 64) launch(k_svd64<16, 4>);
+        else if (max_p <= 128) launch(k_svd64<16, 8>);
+        else if (max_p <= 256) launch(k_svd64<16, 16>);
+        else launch(k_svd64<16, 0>);
+    }
+    counted();
+}
+
+}  // namespace kv
