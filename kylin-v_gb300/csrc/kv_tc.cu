@@ -23,9 +23,9 @@
 //     planes of a panel contiguous, so a pipeline stage is one bulk copy per
 //     operand.
 //  2. Products (k_gemm_tc).  T1 = Ar Br, T2 = Ai Bi, T3 = As Bs are formed as
-//     digit-pair products of orders o = i + j <= 4 (15 per real product, 45
-//     tcgen05.mma.kind::f16 of M=128, N=32, K=16 per K panel) into 15 FP32
-//     accumulators in tensor memory.  Every digit product is an integer of
+//     digit-pair products of orders o = i + j <= 4 (15 per real product; 15
+//     tcgen05.mma.kind::f16 of M=128, N=32..160, K=16 per K panel, see
+//     mma_panel) into 15 FP32 accumulators in tensor memory.  Every digit product is an integer of
 //     at most 2^14 in magnitude, an order sums at most 2^16 of them per K
 //     step, and at most 240 K-steps are accumulated between drains, so every
 //     accumulator is an integer below 2^24 and the FP32 accumulation is
@@ -348,45 +348,50 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
 
 // instruction descriptor, kind::f16: D = F32 (bits 4-5 = 1), A = B = F16
 // (bits 7-9, 10-12 = 0), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+constexpr uint32_t idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); }
 
-// D (+)= A B with the accumulate flag fixed at compile time (no per-MMA predicate set-up)
-template <bool ACC>
+// D (+)= A B over N columns with the accumulate flag fixed at compile time (no per-MMA predicate set-up)
+template <bool ACC, int N>
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc) {
     if constexpr (ACC)
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 1, 1;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "n"(IDESC));
+            "l"(adesc), "l"(bdesc), "n"(idesc(N)));
     else
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, 1, 1;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "n"(IDESC));
+            "l"(adesc), "l"(bdesc), "n"(idesc(N)));
 }
 
-// The 45 MMAs of one K panel.  Shared-memory descriptors are the stage's
-// plane-0 descriptors plus compile-time plane offsets (a plane offset is a
-// multiple of 16 bytes, and no address leaves the 14-bit field, so adding
-// offset / 16 to the descriptor is adding it to the address).  FIRST: the
-// panel opens a drain group, so each order's first digit pair overwrites its
-// accumulator.
-template <bool FIRST>
-__device__ __forceinline__ void mma_panel(uint32_t tmem, uint64_t da, uint64_t db) {
+// The MMAs of one K panel.  A's digit plane i meets B's planes 0 .. 4-i: those
+// planes are consecutive in shared memory (one N axis of 32 (5-i) rows) and
+// their orders i .. 4 are consecutive accumulators, so one MMA of N = 32 (5-i)
+// does 5-i digit pairs: 15 MMAs a panel, each reading its A plane once (45 of
+// N = 32 read A 45 times, and shared memory bounds them: D = 512 two-site
+// Lanczos exponential, us a launch: 365 -> 212; D = 128: 34.6 -> 27.2).
+// Shared-memory descriptors are the stage's plane-0 descriptors plus
+// compile-time plane offsets (a plane offset is a multiple of 16 bytes, and no
+// address leaves the 14-bit field, so adding offset / 16 to the descriptor is
+// adding it to the address).  FIRST: the panel opens a drain group, so A's
+// plane 0, which reaches every order, overwrites the accumulators.
+template <bool FIRST, int I>
+__device__ __forceinline__ void mma_plane(uint32_t tmem, uint64_t da, uint64_t db) {
 #pragma unroll
     for (int c = 0; c < NCOMP; ++c)
-#pragma unroll
-        for (int o = 0; o < NORD; ++o) {
-            const uint32_t d = tmem + (uint32_t)((c * NORD + o) * BN);
-#pragma unroll
-            for (int i = (o > NDIG - 1 ? o - (NDIG - 1) : 0); i <= (o < NDIG - 1 ? o : NDIG - 1); ++i) {
-                const int jj = o - i;
-                const uint64_t ad = da + (uint64_t)(((c * NDIG + i) * PLANE_A) >> 4);
-                const uint64_t bd = db + (uint64_t)(((c * NDIG + jj) * PLANE_B) >> 4);
-                if (FIRST && i == (o > NDIG - 1 ? o - (NDIG - 1) : 0)) mma_f16<false>(d, ad, bd);
-                else mma_f16<true>(d, ad, bd);
-            }
-        }
+        mma_f16<!(FIRST && I == 0), BN *(NORD - I)>(tmem + (uint32_t)((c * NORD + I) * BN),
+                                                    da + (uint64_t)(((c * NDIG + I) * PLANE_A) >> 4),
+                                                    db + (uint64_t)(((c * NDIG) * PLANE_B) >> 4));
+}
+template <bool FIRST>
+__device__ __forceinline__ void mma_panel(uint32_t tmem, uint64_t da, uint64_t db) {
+    static_assert(NDIG == 5 && NORD == 5, "one call per digit plane of A");
+    mma_plane<FIRST, 0>(tmem, da, db);
+    mma_plane<FIRST, 1>(tmem, da, db);
+    mma_plane<FIRST, 2>(tmem, da, db);
+    mma_plane<FIRST, 3>(tmem, da, db);
+    mma_plane<FIRST, 4>(tmem, da, db);
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
