@@ -288,7 +288,8 @@ double ref_product_flops(const Meta &A, const Meta &B, int nc, int opA, int opB,
 // legs lead, lead+1 of lm (w_l, sigma) contract with legs 1, 2 of W; W's legs
 // 0, 3 (sigma', w_r) replace them.  Equal output blocks are merged here (the
 // reference keeps them apart and the following product<> sums them).
-MixPlanFull plan_mix(const Meta &lm, const Meta &W, int lead, const std::vector<double> *mult_in, bool keys_only) {
+MixPlanFull plan_mix(const Meta &lm, const Meta &W, int lead, const std::vector<double> *mult_in, bool keys_only,
+                     int min_chunk) {
     MixPlanFull R;
     R.out.rank = lm.rank;
     R.out.dirs = lm.dirs;
@@ -348,6 +349,8 @@ MixPlanFull plan_mix(const Meta &lm, const Meta &W, int lead, const std::vector<
             R.term_coef[at] = f.coef;
         }
     }
+    const int64_t share = R.out.nelem / (32 * std::max(1, ctx().num_sms));
+    R.mix.chunk = (int)std::max<int64_t>(min_chunk, std::min<int64_t>(kMixChunkMax, share / 32 * 32));
     for (size_t b = 0; b < nout; ++b) {
         MixJob j;
         j.out_off = R.out.blocks[b].off;
@@ -360,7 +363,7 @@ MixPlanFull plan_mix(const Meta &lm, const Meta &W, int lead, const std::vector<
         j.term_end = start[b + 1];
         const int job = (int)R.mix.jobs.size();
         R.mix.jobs.push_back(j);
-        for (int64_t s = 0; s < j.count; s += kMixChunk) R.mix.items.push_back({job, s});
+        for (int64_t s = 0; s < j.count; s += R.mix.chunk) R.mix.items.push_back({job, s});
     }
     return R;
 }

@@ -61,7 +61,7 @@ struct SvdOut {
 ProductPlan plan_product(const Meta &A, const Meta &B, int nc, int opA, int opB, bool keys_only = false);
 void build_tiles(ProductPlan &P, const std::vector<int64_t> &target_off, int tile_m, int tile_n);
 MixPlanFull plan_mix(const Meta &lm, const Meta &W, int lead, const std::vector<double> *mult_in = nullptr,
-                     bool keys_only = false);
+                     bool keys_only = false, int min_chunk = kMixChunk);
 double ref_product_flops(const Meta &A, const Meta &B, int nc, int opA, int opB, const std::vector<double> *multA,
                          const std::vector<double> *multB);
 HeffPlan plan_heff(int nsite, const Meta &L, const Meta &psi, const Meta *W1, const Meta *W2, const Meta &R,

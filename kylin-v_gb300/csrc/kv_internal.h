@@ -368,10 +368,12 @@ struct MixJob {
     int nk_unused, so, wr, rest;
     int term_begin, term_end;
 };
-// elements of one job handled by one CTA of the mixing kernel (256 threads,
-// one element each): small jobs still spread over many SMs
-constexpr int kMixChunk = 256;
-struct MixItem {  // a chunk of one job handled by one CTA
+// Output elements of one job handled by one warp of the mixing kernel: so that
+// the plan's elements make about 32 items an SM, within these bounds
+// (kMixChunkCoarse: the least where the item list's size is part of a scratch
+// bound).
+constexpr int kMixChunk = 64, kMixChunkCoarse = 256, kMixChunkMax = 2048;
+struct MixItem {  // a chunk of one job handled by one warp
     int job;
     int64_t start;
 };
@@ -379,6 +381,7 @@ struct MixPlan {
     std::vector<MixTerm> terms;
     std::vector<MixJob> jobs;
     std::vector<MixItem> items;
+    int chunk = kMixChunk;
     DevBuf d_terms, d_jobs, d_items;
     bool write_inactive = true;  // as GemmPlan::write_inactive, per output block
     // profiling: algorithmic bytes of a launch at Lanczos step s (s clamped to

@@ -114,50 +114,141 @@ __global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ t
 }
 
 // ------------------------------------------------------------------ mix
-// out[k, k2, r, n] = sum_terms sum_kk W[k2, kk, r] in[k, kk, n]; one CTA per
-// (job, chunk of kMixChunk elements).  The FP64 unit (two thread-operations
-// per clock per SM on GB300) bounds this kernel, and an MPO's local operators
-// are mostly zeros and real: a zero W entry adds nothing and is skipped, a
-// real one takes two fused multiply-adds instead of four.  Consecutive
-// threads share (k2, r), so the branch is uniform across a warp where n spans
-// it; for finite inputs the sums equal the four-FMA product's (up to the
-// sign of a zero sum).
+// out[k, k2, r, n] = sum_terms sum_kk W[k2, kk, r] in[k, kk, n]; one warp per
+// item (a chunk of one job's elements).  An MPO's local operators are mostly
+// zeros, real, and often the identity: each warp first compacts its job's
+// nonzero W entries, in order, into a list per output (k2, r) in shared
+// memory, so an element costs one input per nonzero entry (two fused
+// multiply-adds if W is real, none for a leading 1).  What bounds it: the
+// elements' traffic once the blocks are large (each element is written once
+// and about 1.5 inputs are read), the list's chain of loads (job, terms, W)
+// where they are small; a warp per item keeps many such chains in flight.
+// For finite inputs the sums equal the four-multiply-add product's over all
+// entries up to the sign of a zero.
+// MIX_MEASURED
+constexpr int kMixWarps = 8;    // warps (items) per CTA
+constexpr int kMixTerms = 16;   // terms, outputs (k2, r) and nonzero entries a warp's list holds;
+constexpr int kMixOuts = 16;    // larger jobs take mix_direct
+constexpr int kMixList = 64;
 
-__global__ void __launch_bounds__(256) k_mix(const MixItem *__restrict__ items, const MixJob *__restrict__ jobs,
-                                             const MixTerm *__restrict__ terms, const double2 *__restrict__ in,
-                                             const double2 *__restrict__ W, double2 *__restrict__ out,
-                                             const int *skip, int step, int write_inactive) {
-    if (skip && *skip) return;
-    const MixItem it = items[blockIdx.x];
-    const MixJob jb = jobs[it.job];
-    if (!write_inactive) {
-        bool any = false;
-        for (int ti = jb.term_begin; ti < jb.term_end; ++ti) any = any || terms[ti].entry <= step;
-        if (!any) return;
+struct MixEntry {
+    double2 w;
+    int64_t off;  // of the input element at k = n = 0
+    int64_t kst;  // input elements per k
+};
+struct MixWarp {
+    MixEntry list[kMixList];
+    MixTerm term[kMixTerms];
+    int start[kMixOuts + 1];
+};
+
+// one element straight from the plan and W
+__device__ __forceinline__ double2 mix_direct(const MixJob &jb, const MixTerm *__restrict__ terms,
+                                              const double2 *__restrict__ in, const double2 *__restrict__ W, int step,
+                                              int64_t e) {
+    const int64_t n = e % jb.rest, r = (e / jb.rest) % jb.wr, k2 = (e / ((int64_t)jb.rest * jb.wr)) % jb.so;
+    const int64_t k = e / ((int64_t)jb.rest * jb.wr * jb.so);
+    double2 acc = make_double2(0.0, 0.0);
+    for (int ti = jb.term_begin; ti < jb.term_end; ++ti) {
+        const MixTerm tm = terms[ti];
+        if (tm.entry > step) continue;
+        const double2 *w = W + tm.w_off + (k2 * tm.K) * jb.wr + r;
+        const double2 *x = in + tm.in_off + (k * tm.K) * jb.rest + n;
+        for (int kk = 0; kk < tm.K; ++kk) {
+            const double2 wv = w[(int64_t)kk * jb.wr];
+            if (wv.x != 0.0 || wv.y != 0.0) cfma(acc, wv, x[(int64_t)kk * jb.rest]);
+        }
     }
-    for (int j = threadIdx.x; j < kMixChunk; j += blockDim.x) {
-        int64_t e = it.start + j;
-        if (e >= jb.count) break;
-        int64_t n = e % jb.rest;
-        int64_t r = (e / jb.rest) % jb.wr;
-        int64_t k2 = (e / (jb.rest * jb.wr)) % jb.so;
-        int64_t k = e / (jb.rest * jb.wr * jb.so);
+    return acc;
+}
+
+__global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restrict__ items, int nitems, int chunk,
+                                                        const MixJob *__restrict__ jobs,
+                                                        const MixTerm *__restrict__ terms,
+                                                        const double2 *__restrict__ in, const double2 *__restrict__ W,
+                                                        double2 *__restrict__ out, const int *skip, int step,
+                                                        int write_inactive) {
+    __shared__ MixWarp sm[kMixWarps];
+    if (skip && *skip) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int item = blockIdx.x * kMixWarps + warp;
+    if (item >= nitems) return;  // warp-uniform, as every branch on the item below
+    MixWarp &mw = sm[warp];
+    const MixItem it = items[item];
+    const MixJob jb = jobs[it.job];
+    const int nt_all = jb.term_end - jb.term_begin, nout = jb.so * jb.wr;
+    const int64_t e1 = min(jb.count, it.start + chunk);
+    bool listed = nt_all <= kMixTerms && nout <= kMixOuts && jb.count < (1ll << 31);
+    int nt = 0, ktot = 0;  // active terms and their contracted indices
+    if (listed) {
+        MixTerm tm{};
+        const bool act = lane < nt_all && (tm = terms[jb.term_begin + lane]).entry <= step;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, act);
+        if (act) mw.term[__popc(m & ((1u << lane) - 1))] = tm;
+        nt = __popc(m);
+        ktot = __reduce_add_sync(0xFFFFFFFFu, act ? tm.K : 0);
+        __syncwarp();
+        if (nt == 0 && !write_inactive) return;
+        // entries (output o, contracted index kp of the active terms), o major, kept where W is not zero
+        int used = 0;
+        for (int x0 = 0; x0 < nout * ktot && used <= kMixList; x0 += 32) {
+            const int x = x0 + lane;
+            MixEntry en{};
+            bool nz = false;
+            int o = 0, kp = 0;
+            if (x < nout * ktot) {
+                o = x / ktot;
+                kp = x - o * ktot;
+                int t = 0, kk = kp;
+                while (kk >= mw.term[t].K) kk -= mw.term[t++].K;
+                const MixTerm &q = mw.term[t];
+                const int k2 = o / jb.wr, r = o - k2 * jb.wr;
+                en.w = W[q.w_off + ((int64_t)k2 * q.K + kk) * jb.wr + r];
+                en.off = q.in_off + (int64_t)kk * jb.rest;
+                en.kst = (int64_t)q.K * jb.rest;
+                nz = en.w.x != 0.0 || en.w.y != 0.0;
+            }
+            const unsigned b = __ballot_sync(0xFFFFFFFFu, nz);
+            const int at = used + __popc(b & ((1u << lane) - 1));
+            if (x < nout * ktot && kp == 0) mw.start[o] = at;
+            if (nz && at < kMixList) mw.list[at] = en;
+            used += __popc(b);
+        }
+        if (lane == 0) {
+            if (ktot == 0)
+                for (int o = 0; o < nout; ++o) mw.start[o] = 0;
+            mw.start[nout] = used;
+        }
+        __syncwarp();
+        listed = used <= kMixList;
+    } else if (!write_inactive) {
+        bool any = false;
+        for (int ti = jb.term_begin + lane; ti < jb.term_end; ti += 32) any = any || terms[ti].entry <= step;
+        if (!__any_sync(0xFFFFFFFFu, any)) return;
+    }
+    if (!listed) {
+        for (int64_t e = it.start + lane; e < e1; e += 32) out[jb.out_off + e] = mix_direct(jb, terms, in, W, step, e);
+        return;
+    }
+    const unsigned rest = (unsigned)jb.rest, no = (unsigned)nout;
+#pragma unroll 2
+    for (unsigned e = (unsigned)it.start + lane; e < (unsigned)e1; e += 32) {
+        const unsigned row = e / rest, n = e - row * rest, k = row / no, o = row - k * no;
         double2 acc = make_double2(0.0, 0.0);
-        for (int ti = jb.term_begin; ti < jb.term_end; ++ti) {
-            const MixTerm tm = terms[ti];
-            if (tm.entry > step) continue;
-            const double2 *w = W + tm.w_off + (k2 * tm.K) * jb.wr + r;
-            const double2 *x = in + tm.in_off + (k * tm.K) * jb.rest + n;
-            for (int kk = 0; kk < tm.K; ++kk) {
-                const double2 wv = w[(int64_t)kk * jb.wr];
-                if (wv.y == 0.0) {
-                    if (wv.x == 0.0) continue;
-                    const double2 xv = x[(int64_t)kk * jb.rest];
-                    acc.x = fma(wv.x, xv.x, acc.x);
-                    acc.y = fma(wv.x, xv.y, acc.y);
-                } else {
-                    cfma(acc, wv, x[(int64_t)kk * jb.rest]);
-                }
+        int i = mw.start[o];
+        const int i1 = mw.start[o + 1];
+        if (i < i1 && mw.list[i].w.x == 1.0 && mw.list[i].w.y == 0.0) {
+            acc = in[mw.list[i].off + (int64_t)k * mw.list[i].kst + n];
+            ++i;
+        }
+        for (; i < i1; ++i) {
+            const MixEntry &en = mw.list[i];
+            const double2 x = in[en.off + (int64_t)k * en.kst + n];
+            if (en.w.y == 0.0) {
+                acc.x = fma(en.w.x, x.x, acc.x);
+                acc.y = fma(en.w.x, x.y, acc.y);
+            } else {
+                cfma(acc, en.w, x);
             }
         }
         out[jb.out_off + e] = acc;
@@ -262,9 +353,10 @@ void launch_gemm_fp64(const GemmPlan &p, const double2 *A, const double2 *B, dou
 
 void launch_mix(const MixPlan &p, const double2 *in, const double2 *W, double2 *out, const int *skip, int step) {
     if (p.items.empty()) return;
-    k_mix<<<(unsigned)p.items.size(), 256, 0, ctx().stream>>>(p.d_items.as<MixItem>(), p.d_jobs.as<MixJob>(),
-                                                               p.d_terms.as<MixTerm>(), in, W, out, skip, step,
-                                                               p.write_inactive ? 1 : 0);
+    const int n = (int)p.items.size();
+    k_mix<<<(unsigned)((n + kMixWarps - 1) / kMixWarps), 32 * kMixWarps, 0, ctx().stream>>>(
+        p.d_items.as<MixItem>(), n, p.chunk, p.d_jobs.as<MixJob>(), p.d_terms.as<MixTerm>(), in, W, out, skip, step,
+        p.write_inactive ? 1 : 0);
     counted();
     KV_CUDA(cudaGetLastError());
 }

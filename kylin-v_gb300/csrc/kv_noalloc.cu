@@ -136,7 +136,7 @@ cplx expectation_noalloc(const std::vector<DTensor *> &bra, const std::vector<DT
         Meta t1;
         double2 *t1_d;
         arena_product(ar, env, env_d, ket[i]->meta, ket[i]->data(), 1, KV_OP_N, KV_OP_N, t1, t1_d);
-        MixPlanFull M = plan_mix(t1, w[i]->meta, 1);
+        MixPlanFull M = plan_mix(t1, w[i]->meta, 1, nullptr, false, kMixChunkCoarse);
         double2 *t2_d = static_cast<double2 *>(ar.take(std::max<int64_t>(1, M.out.nelem) * sizeof(double2)));
         {
             Views vw;
