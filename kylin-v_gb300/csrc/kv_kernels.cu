@@ -134,8 +134,21 @@ constexpr int kMixList = 64;
 struct MixEntry {
     double2 w;
     int64_t off;  // of the input element at k = n = 0
-    int64_t kst;  // input elements per k
+    int kst;      // input elements per k
+    int kind;     // kUnit, kReal or kComplex (an FP64 comparison per element would cost as much as its sum)
 };
+enum MixKind { kUnit = 0, kReal = 1, kComplex = 2 };
+// acc (first: nothing summed yet) plus the entry's share
+__device__ __forceinline__ void mix_add(double2 &acc, const MixEntry &en, double2 x, bool first) {
+    if (en.kind == kComplex) {
+        cfma(acc, en.w, x);
+    } else if (first && en.kind == kUnit) {
+        acc = x;
+    } else {
+        acc.x = fma(en.w.x, x.x, acc.x);
+        acc.y = fma(en.w.x, x.y, acc.y);
+    }
+}
 struct MixWarp {
     MixEntry list[kMixList];
     MixTerm term[kMixTerms];
@@ -205,7 +218,8 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
                 const int k2 = o / jb.wr, r = o - k2 * jb.wr;
                 en.w = W[q.w_off + ((int64_t)k2 * q.K + kk) * jb.wr + r];
                 en.off = q.in_off + (int64_t)kk * jb.rest;
-                en.kst = (int64_t)q.K * jb.rest;
+                en.kst = q.K * jb.rest;
+                en.kind = en.w.y != 0.0 ? kComplex : en.w.x == 1.0 ? kUnit : kReal;
                 nz = en.w.x != 0.0 || en.w.y != 0.0;
             }
             const unsigned b = __ballot_sync(0xFFFFFFFFu, nz);
@@ -230,26 +244,40 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
         for (int64_t e = it.start + lane; e < e1; e += 32) out[jb.out_off + e] = mix_direct(jb, terms, in, W, step, e);
         return;
     }
-    const unsigned rest = (unsigned)jb.rest, no = (unsigned)nout;
+    const unsigned rest = (unsigned)jb.rest, no = (unsigned)nout, ee = (unsigned)e1;
+    if (rest >= 32) {  // row by row: each entry is read once for up to 4 elements a lane
+        for (unsigned e = (unsigned)it.start; e < ee;) {
+            const unsigned row = e / rest, n0 = e - row * rest, k = row / no, o = row - k * no;
+            const unsigned len = min(min(rest - n0, ee - e), 128u);
+            const int i0 = mw.start[o], i1 = mw.start[o + 1];
+            double2 acc[4] = {};
+            for (int i = i0; i < i1; ++i) {
+                const MixEntry &en = mw.list[i];
+                const double2 *x = in + en.off + (int64_t)k * en.kst + n0;
+                double2 v[4] = {};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (lane + 32 * j < len) v[j] = x[lane + 32 * j];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (32 * j < len) mix_add(acc[j], en, v[j], i == i0);
+            }
+            double2 *y = out + jb.out_off + e;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (lane + 32 * j < len) y[lane + 32 * j] = acc[j];
+            e += len;
+        }
+        return;
+    }
 #pragma unroll 2
-    for (unsigned e = (unsigned)it.start + lane; e < (unsigned)e1; e += 32) {
+    for (unsigned e = (unsigned)it.start + lane; e < ee; e += 32) {
         const unsigned row = e / rest, n = e - row * rest, k = row / no, o = row - k * no;
         double2 acc = make_double2(0.0, 0.0);
-        int i = mw.start[o];
-        const int i1 = mw.start[o + 1];
-        if (i < i1 && mw.list[i].w.x == 1.0 && mw.list[i].w.y == 0.0) {
-            acc = in[mw.list[i].off + (int64_t)k * mw.list[i].kst + n];
-            ++i;
-        }
-        for (; i < i1; ++i) {
+        const int i0 = mw.start[o], i1 = mw.start[o + 1];
+        for (int i = i0; i < i1; ++i) {
             const MixEntry &en = mw.list[i];
-            const double2 x = in[en.off + (int64_t)k * en.kst + n];
-            if (en.w.y == 0.0) {
-                acc.x = fma(en.w.x, x.x, acc.x);
-                acc.y = fma(en.w.x, x.y, acc.y);
-            } else {
-                cfma(acc, en.w, x);
-            }
+            mix_add(acc, en, in[en.off + (int64_t)k * en.kst + n], i == i0);
         }
         out[jb.out_off + e] = acc;
     }
