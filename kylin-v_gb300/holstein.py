@@ -444,6 +444,8 @@ def random_mps_structure(chain: HolsteinChain, D: int) -> list:
                 if not progressed:
                     break
             while rem < 0:
+                if max(alloc.values()) == 1:
+                    break  # more sectors than D: one state each
                 for q in sorted(alloc, key=lambda q: (alloc[q], q), reverse=True):
                     if rem == 0:
                         break
