@@ -1130,9 +1130,14 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     std::vector<SvdPolish> pol;
     std::vector<int> pol_of_sector(nsec, -1);
     DevBuf X, Gm, Wb, cst, cdiag;
+    // The mixed rebuild sums over k in order: the last bit of its result decides,
+    // through the next FP32 SVD's cut-offs, which noise-level states a one-site
+    // sweep keeps (populations of D = 64 chains move by up to 7e-8 a step with
+    // another order), so its order of summation does not follow the tiling.
     auto add_gemm = [&](GemmPlan &g, int64_t c_off, int M, int N, GemmSeg seg) {
         const int sb = (int)g.segs.size();
         g.tile_m = g.tile_n = kFp64Block;
+        g.serial_k = mixed;
         g.segs.push_back(seg);
         g.tiles.push_back({c_off, N, M, N, 0, 0, sb, sb + 1});
     };

@@ -334,6 +334,7 @@ struct GemmPlan {
     int max_k = 0;
     int tile_m = 0, tile_n = 0;
     int fp64_threads = 256;  // CTA size of the FP64 path
+    bool serial_k = false;   // FP64 path: each output summed by one thread over k in order (else K may be split)
     // tiles whose segments are all inactive at the launch's step write zeros
     // (false: they write nothing; for intermediates only read by active consumers)
     bool write_inactive = true;

@@ -26,10 +26,11 @@ __device__ __forceinline__ void cfma(double2 &acc, double2 a, double2 b) {
 // consecutively and thread slice ks takes those equal to ks mod KS; the KS
 // partial sums are added in a fixed tree, so the order is fixed and there are
 // no atomics.
-// What bounds it: the FP64 unit, two thread-operations per clock per SM (four
-// per complex multiply-add), so an operand pair read from L1/L2 for every
-// multiply-add (32 B per 2 clocks) is hidden and neither register blocking
-// nor shared-memory staging helps; what matters is that all SMs hold equal
+// What bounds it: the FP64 unit.  Measured on GB300: a warp's FP64 instruction
+// takes 19 clocks of the SM (64 of one warp's time), whatever its active
+// lanes, and a complex multiply-add is four, so an operand pair read from
+// L1/L2 for every multiply-add is hidden and neither register blocking nor
+// shared-memory staging helps; what matters is that all SMs hold equal
 // shares of the multiply-adds.  The plan (fp64_tiles) therefore sizes tiles
 // by their work, and blocks smaller than a tile leave no thread idle (tm, tn
 // are any integers).  Against 32 x 32 tiles with K walked by the whole CTA
@@ -47,13 +48,14 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ tiles,
                                                   const GemmSeg *__restrict__ segs, const double2 *__restrict__ A,
                                                   const double2 *__restrict__ B, double2 *__restrict__ C, double alpha,
-                                                  const int *skip, int step, int write_inactive, int cover) {
+                                                  const int *skip, int step, int write_inactive, int cover,
+                                                  int serial_k) {
     if (skip && *skip) return;
     __shared__ GemmSeg sg[kSegBatch];
     __shared__ double2 red[NT];
     const GemmTile t = tiles[blockIdx.x];
     const int tid = threadIdx.x;
-    const int tm = t.tm, tn = t.tn, mn = tm * tn, KS = NT / mn;
+    const int tm = t.tm, tn = t.tn, mn = tm * tn, KS = serial_k ? 1 : NT / mn;
     const int ks = tid / mn, m = (tid % mn) / tn, n = tid % tn;
     // cover > 0 (coarse task lists): the CTA walks the cover x cover outputs from (m0, n0) in tm x tn steps
     const int m_end = cover > 0 ? min(t.M, t.m0 + cover) : min(t.M, t.m0 + tm);
@@ -81,8 +83,36 @@ __global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ t
                         const int64_t da = akc ? 1 : lda, db = bnc ? ldb : 1;
                         const double2 *pa = A + sg[i].a_off + (akc ? (int64_t)gm * lda : gm);
                         const double2 *pb = B + sg[i].b_off + (bnc ? gn : (int64_t)gn * ldb);
-#pragma unroll 4
-                        for (int k = first; k < K; k += KS) {
+                        // UL operand pairs are read ahead of the UL being multiplied
+                        constexpr int UL = NT == 32 ? 8 : 4;
+                        const int64_t sa = (int64_t)KS * da, sb = (int64_t)KS * db;
+                        const double2 *qa = pa + first * da, *qb = pb + first * db;
+                        int k = first;
+                        if (k + (UL - 1) * KS < K) {
+                            double2 a[UL], b[UL];
+#pragma unroll
+                            for (int u = 0; u < UL; ++u) { a[u] = qa[u * sa]; b[u] = qb[u * sb]; }
+                            for (; k + (UL - 1) * KS < K; k += UL * KS) {
+                                double2 an[UL], bn[UL];
+                                qa += UL * sa;
+                                qb += UL * sb;
+                                const bool more = k + (2 * UL - 1) * KS < K;
+#pragma unroll
+                                for (int u = 0; u < UL; ++u) {
+                                    an[u] = more ? qa[u * sa] : make_double2(0.0, 0.0);
+                                    bn[u] = more ? qb[u * sb] : make_double2(0.0, 0.0);
+                                }
+#pragma unroll
+                                for (int u = 0; u < UL; ++u) {
+                                    a[u].y = flip_sign(a[u].y, fa);
+                                    b[u].y = flip_sign(b[u].y, fb);
+                                    cfma(acc, a[u], b[u]);
+                                    a[u] = an[u];
+                                    b[u] = bn[u];
+                                }
+                            }
+                        }
+                        for (; k < K; k += KS) {
                             double2 a = pa[k * da], b = pb[k * db];
                             a.y = flip_sign(a.y, fa);
                             b.y = flip_sign(b.y, fb);
@@ -327,13 +357,16 @@ int grid_for(int64_t n, int threads) {
 // covering the block).  A tile's cost is its multiply-adds, outputs x K; tiles
 // are cut so that none exceeds a quarter of an SM's share of the plan, or
 // kMinTile multiply-adds (about 1 us of one SM's FP64 unit, what a CTA costs
-// to start), and never more than 256 outputs.
+// to start), and never more than 256 outputs.  serial_k plans (one thread per
+// output, so each sum runs over k in order) take one warp a tile, shaped to
+// need the fewest warps.
 void fp64_tiles(GemmPlan &g) {
     constexpr double kMinTile = 1024.0;
     std::vector<GemmTile> blocks;
     blocks.swap(g.tiles);
     std::vector<double> K(blocks.size(), 0.0);
     double total = 0.0, top = 0.0;
+    int most = 1;
     for (size_t i = 0; i < blocks.size(); ++i) {
         const GemmTile &b = blocks[i];
         for (int s = b.seg_begin; s < b.seg_end; ++s) K[i] += g.segs[s].K;
@@ -347,19 +380,27 @@ void fp64_tiles(GemmPlan &g) {
         int tn = std::min(b.N, std::max(1, (int)std::sqrt((double)area)));
         int tm = std::min(b.M, std::max(1, area / tn));
         tn = std::min(b.N, std::max(1, area / tm));
-        tm = (b.M + (b.M + tm - 1) / tm - 1) / ((b.M + tm - 1) / tm);
-        tn = (b.N + (b.N + tn - 1) / tn - 1) / ((b.N + tn - 1) / tn);
+        if (g.serial_k) {
+            int64_t fewest = INT64_MAX;
+            for (int x = 1; x <= std::min(32, b.N); ++x) {
+                const int y = std::min(b.M, 32 / x);
+                const int64_t warps = (int64_t)((b.M + y - 1) / y) * ((b.N + x - 1) / x);
+                if (warps < fewest) { fewest = warps; tn = x; tm = y; }
+            }
+        } else {
+            tm = (b.M + (b.M + tm - 1) / tm - 1) / ((b.M + tm - 1) / tm);
+            tn = (b.N + (b.N + tn - 1) / tn - 1) / ((b.N + tn - 1) / tn);
+        }
         GemmTile t = b;
         t.tm = (short)tm;
         t.tn = (short)tn;
         for (t.m0 = 0; t.m0 < b.M; t.m0 += tm)
             for (t.n0 = 0; t.n0 < b.N; t.n0 += tn) g.tiles.push_back(t);
         top = std::max(top, (double)tm * tn * K[i]);
+        most = std::max(most, tm * tn);
     }
-    g.fp64_threads = top <= 2.0 * kMinTile ? 64 : 256;
-    if (g.fp64_threads == 64)
-        for (auto &t : g.tiles)
-            if (t.tm * t.tn > 64) { g.fp64_threads = 256; break; }
+    if (g.serial_k) g.fp64_threads = 32;
+    else g.fp64_threads = top <= 2.0 * kMinTile && most <= 64 ? 64 : 256;
 }
 
 void launch_gemm_fp64(const GemmPlan &p, const double2 *A, const double2 *B, double2 *C, double alpha,
@@ -369,12 +410,13 @@ void launch_gemm_fp64(const GemmPlan &p, const double2 *A, const double2 *B, dou
                "internal: GEMM plan not prepared for the FP64 path");
     const int cover = p.tile_m == kFp64Coarse ? kFp64Coarse : 0;
     const unsigned n = (unsigned)p.tiles.size();
-    if (p.fp64_threads == 64)
-        k_gemm_fp64<64><<<n, 64, 0, ctx().stream>>>(p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C, alpha,
-                                                    skip, step, p.write_inactive ? 1 : 0, cover);
-    else
-        k_gemm_fp64<256><<<n, 256, 0, ctx().stream>>>(p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C,
-                                                      alpha, skip, step, p.write_inactive ? 1 : 0, cover);
+    auto launch = [&](auto kernel, int threads) {
+        kernel<<<n, threads, 0, ctx().stream>>>(p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C, alpha, skip,
+                                                step, p.write_inactive ? 1 : 0, cover, p.serial_k ? 1 : 0);
+    };
+    if (p.fp64_threads == 32) launch(k_gemm_fp64<32>, 32);
+    else if (p.fp64_threads == 64) launch(k_gemm_fp64<64>, 64);
+    else launch(k_gemm_fp64<256>, 256);
     counted();
     KV_CUDA(cudaGetLastError());
 }
