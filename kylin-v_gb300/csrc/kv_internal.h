@@ -304,26 +304,44 @@ constexpr int kFp64Block = 1 << 30, kFp64Coarse = 32;
 // Tile shape of the tensor-core path (kv_tc.cu).
 constexpr int kMixedTileM = 128, kMixedTileN = 32;
 
-// Tensor-core path: one operand block viewed as GEMM rows x K, sliced into
-// fixed-point digit panels (dst_off: FP16 elements into the panel buffer,
-// exp_off: first of its per-row exponents).
+// Tensor-core path.  An operand view is one operand block as GEMM rows x K (A:
+// rows m; B: rows n).  A pack stacks row pieces of several views with the same
+// K (pieces start at multiples of 8) into one panel: up to 128 rows for A,
+// stored with as many rows as it holds, and 32 for B; a tile multiplies one A
+// pack by one B pack per segment and its outputs go to several output blocks.
+// One slicing job is one piece: fixed-point digits of its rows into the panel
+// (dst_off: FP16 elements into the panel buffer, exp_off: its first per-row
+// exponent).
 struct SliceJob {
     int64_t src_off, dst_off;
-    int rows, K, ld;
-    int trans;  // 0: (row, k) at src[row*ld + k]; 1: at src[k*ld + row]
-    int conj;   // negate the imaginary part
+    int row0, rows;  // the piece within its view
+    int r0, tr;      // its first row within the panel, and the panel's rows
+    int K, ld;
+    int trans;       // 0: (row, k) at src[row*ld + k]; 1: at src[k*ld + row]
+    int conj;        // negate the imaginary part
     int exp_off, nkc;
-    int entry;  // first step at which a segment reading this block is active
-    int ks_off; // balanced plans: first of this view's K power-of-two scale entries (-1: none)
+    int entry;       // first step at which a segment reading this pack is active
+    int ks_off;      // balanced plans: first of this view's K power-of-two scale entries (-1: none)
 };
-// Tensor-core path: a segment's sliced A and B blocks.
+// A tile's segment: its sliced A and B packs.
 struct SegX {
     int64_t a_pan, b_pan;
     int nkc, a_exp, b_exp, entry;
 };
+struct TcTile {
+    int rows;                // rows of the A packs (a multiple of 8)
+    int seg_begin, seg_end;
+    int rowmap, colmap;      // 128 and 32 entries (piece, row or column of its block; piece -1: padding)
+    int pair, ncol;          // output of (row piece i, column piece j): pairs[pair + i * ncol + j]
+};
+struct TcPair {
+    int64_t c_off;  // output block, or -1
+    int ldc;
+    int entry;      // first step at which the pair is active
+};
 
 struct GemmPlan;
-void plan_mixed(GemmPlan &g);  // slicing jobs of a plan built with the tensor-core tile shape
+void plan_mixed(GemmPlan &g);  // tiles, packs and slicing jobs of a plan built with the tensor-core tile shape
 void fp64_tiles(GemmPlan &g);  // one tile per output block -> tiles of about equal work
 
 struct GemmPlan {
@@ -345,16 +363,18 @@ struct GemmPlan {
     // whose magnitudes vary along k (MPO channels) keep their precision.
     bool balance_k = false;
     int64_t k_scales = 0;  // entries of the per-k maxima arrays
-    std::vector<SliceJob> ajobs, bjobs;
-    std::vector<SegX> xsegs;
-    std::vector<int2> aitems, bitems;  // (job, first of 8 rows) per slicing CTA
+    int tc_tiles = 0, na_items = 0, nb_items = 0;
     int64_t a_planes = 0, b_planes = 0, a_exps = 0, b_exps = 0;
-    DevBuf d_ajobs, d_bjobs, d_xsegs, d_aitems, d_bitems;
+    // items: (job, first of 8 rows) per slicing CTA
+    DevBuf d_tctiles, d_xsegs, d_maps, d_pairs, d_ajobs, d_bjobs, d_aitems, d_bitems;
     void upload() {
+        if (tile_m == kMixedTileM && tile_n == kMixedTileN) {
+            plan_mixed(*this);
+            return;
+        }
         if (tile_m == kFp64Block) fp64_tiles(*this);
         d_tiles = upload_vec(tiles);
         d_segs = upload_vec(segs);
-        if (tile_m == kMixedTileM && tile_n == kMixedTileN) plan_mixed(*this);
     }
 };
 

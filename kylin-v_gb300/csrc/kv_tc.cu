@@ -57,6 +57,8 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <unordered_map>
@@ -95,7 +97,7 @@ constexpr int SMEM_BYTES = STAGES * (A_BYTES + B_BYTES) + SMEM_ALIGN + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "pipeline stages exceed the shared memory of one CTA");
 
 static_assert(NACC * BN <= (int)TMEM_COLS, "accumulators exceed tensor memory");
-static_assert(EPI_COLS % 4 == 0, "the drain loads 4 columns per accumulator at once");
+static_assert(EPI_COLS == 8, "a warp's columns are one multiple of 8 (one piece), loaded 4 at a time");
 static_assert(A_BYTES + B_BYTES < (1 << 20), "transaction count per stage");
 
 // ----------------------------------------------------------- slicing
@@ -121,8 +123,7 @@ __device__ __forceinline__ void digits(long long X, int d[NDIG]) {
     d[0] = (int)X;
 }
 
-// element offset of (row r, k) inside one plane of a TR x 16 panel
-template <int TR>
+// element offset of (row r, k) inside one plane of a panel 16 deep
 __device__ __forceinline__ int panel_off(int r, int k) {
     return (r >> 3) * 128 + (k >> 3) * 64 + (r & 7) * 8 + (k & 7);
 }
@@ -186,7 +187,8 @@ __device__ __forceinline__ void kmax_item(const SliceJob *__restrict__ ajobs, co
         const int k = k0 + lane;
         unsigned long long m = 0;
         if (r < j.rows && k < j.K) {
-            const double2 v = s[j.trans ? (int64_t)k * j.ld + r : (int64_t)r * j.ld + k];
+            const int64_t row = j.row0 + r;
+            const double2 v = s[j.trans ? (int64_t)k * j.ld + row : row * j.ld + k];
             const unsigned long long br = (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFull;
             const unsigned long long bi = (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFull;
             m = max(br, bi);
@@ -216,7 +218,6 @@ __global__ void __launch_bounds__(256) k_kmax(const SliceJob *__restrict__ ajobs
 // an Inf or NaN sets bit kErrNonFinite of *err: fixed point has no code for
 // it, and the digits written for that row are meaningless.  Warps return on
 // their own; there is no barrier here.
-template <int TR>
 __device__ __forceinline__ void slice_item(const SliceJob *__restrict__ jobs, int2 it, const double2 *__restrict__ src,
                                            __half *__restrict__ dst, int *__restrict__ exps, double alpha, int step,
                                            int *err, const unsigned long long *kmax, int64_t kscales, int b_side) {
@@ -224,15 +225,16 @@ __device__ __forceinline__ void slice_item(const SliceJob *__restrict__ jobs, in
     if (j.entry > step) return;  // no active segment reads this block
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = it.y + warp;
-    // rows past the block (up to the panel's TR) are not written: they only
+    // rows past the piece (up to a multiple of 8) are not written: they only
     // reach output rows / columns the GEMM epilogue never stores
     if (r >= j.rows) return;
+    const int64_t row = j.row0 + r;
     const int kpad = j.nkc * BKC;
     const double2 *s = src + j.src_off;
     const bool scale = alpha != 1.0;
     const bool bal = kmax != nullptr && j.ks_off >= 0;
     auto load = [&](int k) {
-        double2 v = s[j.trans ? (int64_t)k * j.ld + r : (int64_t)r * j.ld + k];
+        double2 v = s[j.trans ? (int64_t)k * j.ld + row : row * j.ld + k];
         if (scale) { v.x *= alpha; v.y *= alpha; }
         if (j.conj) v.y = -v.y;
         if (bal) {  // exact power-of-two balancing of the contracted index
@@ -256,8 +258,8 @@ __device__ __forceinline__ void slice_item(const SliceJob *__restrict__ jobs, in
         exps[j.exp_off + r] = e;
         if (mx >= 0x7FF0000000000000ull) atomicOr(err, kErrNonFinite);
     }
-    __half *pan = dst + j.dst_off + (int64_t)(r / TR) * j.nkc * (NPL * TR * BKC);
-    const int rr = r % TR;
+    __half *pan = dst + j.dst_off;
+    const int rr = j.r0 + r, plane = j.tr * BKC;  // elements of a digit plane
     for (int k = 2 * lane; k < kpad; k += 64) {  // k even: k and k + 1 are adjacent in the panel
         long long x[2][NCOMP];
 #pragma unroll
@@ -272,7 +274,7 @@ __device__ __forceinline__ void slice_item(const SliceJob *__restrict__ jobs, in
             x[h][1] = xi;
             x[h][2] = xr + xi;
         }
-        __half *p = pan + (int64_t)(k / BKC) * (NPL * TR * BKC) + panel_off<TR>(rr, k & (BKC - 1));
+        __half *p = pan + (int64_t)(k / BKC) * (NPL * plane) + panel_off(rr, k & (BKC - 1));
 #pragma unroll
         for (int c = 0; c < NCOMP; ++c) {
             int d0[NDIG], d1[NDIG];
@@ -280,7 +282,7 @@ __device__ __forceinline__ void slice_item(const SliceJob *__restrict__ jobs, in
             digits(x[1][c], d1);
 #pragma unroll
             for (int i = 0; i < NDIG; ++i)
-                *reinterpret_cast<__half2 *>(p + (c * NDIG + i) * (TR * BKC)) = digits2(d0[i], d1[i]);
+                *reinterpret_cast<__half2 *>(p + (c * NDIG + i) * plane) = digits2(d0[i], d1[i]);
         }
     }
 }
@@ -296,8 +298,8 @@ __global__ void __launch_bounds__(256) k_slice_ab(const SliceJob *__restrict__ a
                                                   int *err, const unsigned long long *kmax, int64_t kscales) {
     if (skip && *skip) return;
     const int bid = (int)blockIdx.x;
-    if (bid < na) slice_item<BM>(ajobs, aitems[bid], A, ap, ae, 1.0, step, err, kmax, kscales, 0);
-    else slice_item<BN>(bjobs, bitems[bid - na], B, bp, be, alpha, step, err, kmax, kscales, 1);
+    if (bid < na) slice_item(ajobs, aitems[bid], A, ap, ae, 1.0, step, err, kmax, kscales, 0);
+    else slice_item(bjobs, bitems[bid - na], B, bp, be, alpha, step, err, kmax, kscales, 1);
 }
 
 // The balanced slicing as one cooperative launch: zero the per-index maxima,
@@ -326,8 +328,8 @@ __global__ void __launch_bounds__(256) k_slice_coop(const SliceJob *__restrict__
         grid.sync();
     }
     for (int bid = blockIdx.x; bid < nitems; bid += gridDim.x) {
-        if (bid < na) slice_item<BM>(ajobs, aitems[bid], A, ap, ae, 1.0, step, err, kmax, kscales, 0);
-        else slice_item<BN>(bjobs, bitems[bid - na], B, bp, be, alpha, step, err, kmax, kscales, 1);
+        if (bid < na) slice_item(ajobs, aitems[bid], A, ap, ae, 1.0, step, err, kmax, kscales, 0);
+        else slice_item(bjobs, bitems[bid - na], B, bp, be, alpha, step, err, kmax, kscales, 1);
     }
 }
 
@@ -371,27 +373,29 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
 // does 5-i digit pairs: 15 MMAs a panel, each reading its A plane once (45 of
 // N = 32 read A 45 times, and shared memory bounds them: D = 512 two-site
 // Lanczos exponential, us a launch: 365 -> 212; D = 128: 34.6 -> 27.2).
-// Shared-memory descriptors are the stage's plane-0 descriptors plus
-// compile-time plane offsets (a plane offset is a multiple of 16 bytes, and no
-// address leaves the 14-bit field, so adding offset / 16 to the descriptor is
-// adding it to the address).  FIRST: the panel opens a drain group, so A's
+// Shared-memory descriptors are the stage's plane-0 descriptors plus plane
+// offsets (multiples of 16 bytes, and no address leaves the 14-bit field, so
+// adding offset / 16 to the descriptor is adding it to the address); pa: an A
+// plane's bytes / 16.  An A plane of fewer than 128 rows is followed by the
+// next one, so the MMA's rows beyond it multiply other digits and reach only
+// output rows that are not stored.  FIRST: the panel opens a drain group, so A's
 // plane 0, which reaches every order, overwrites the accumulators.
 template <bool FIRST, int I>
-__device__ __forceinline__ void mma_plane(uint32_t tmem, uint64_t da, uint64_t db) {
+__device__ __forceinline__ void mma_plane(uint32_t tmem, uint64_t da, uint64_t db, uint32_t pa) {
 #pragma unroll
     for (int c = 0; c < NCOMP; ++c)
         mma_f16<!(FIRST && I == 0), BN *(NORD - I)>(tmem + (uint32_t)((c * NORD + I) * BN),
-                                                    da + (uint64_t)(((c * NDIG + I) * PLANE_A) >> 4),
+                                                    da + (uint64_t)((uint32_t)(c * NDIG + I) * pa),
                                                     db + (uint64_t)(((c * NDIG) * PLANE_B) >> 4));
 }
 template <bool FIRST>
-__device__ __forceinline__ void mma_panel(uint32_t tmem, uint64_t da, uint64_t db) {
+__device__ __forceinline__ void mma_panel(uint32_t tmem, uint64_t da, uint64_t db, uint32_t pa) {
     static_assert(NDIG == 5 && NORD == 5, "one call per digit plane of A");
-    mma_plane<FIRST, 0>(tmem, da, db);
-    mma_plane<FIRST, 1>(tmem, da, db);
-    mma_plane<FIRST, 2>(tmem, da, db);
-    mma_plane<FIRST, 3>(tmem, da, db);
-    mma_plane<FIRST, 4>(tmem, da, db);
+    mma_plane<FIRST, 0>(tmem, da, db, pa);
+    mma_plane<FIRST, 1>(tmem, da, db, pa);
+    mma_plane<FIRST, 2>(tmem, da, db, pa);
+    mma_plane<FIRST, 3>(tmem, da, db, pa);
+    mma_plane<FIRST, 4>(tmem, da, db, pa);
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
@@ -484,14 +488,15 @@ __device__ __forceinline__ long long combine(const float *p) {
 // Persistent: CTA b takes tiles b, b + gridDim.x, ...; each role walks the
 // same tile sequence and keeps its mbarrier phase counters across tiles, so
 // the producer streams the next tile's panels while the current tile drains.
-__device__ __forceinline__ bool tile_active(const GemmTile &t, const SegX *segs, int step) {
+__device__ __forceinline__ bool tile_active(const TcTile &t, const SegX *segs, int step) {
     for (int s = t.seg_begin; s < t.seg_end; ++s)
         if (segs[s].entry <= step) return true;
     return false;
 }
 
-__global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restrict__ tiles, int ntiles,
-                                                    const SegX *__restrict__ segs,
+__global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const TcTile *__restrict__ tiles, int ntiles,
+                                                    const SegX *__restrict__ segs, const int2 *__restrict__ maps,
+                                                    const TcPair *__restrict__ pairs,
                                                     const __half *__restrict__ Apl, const __half *__restrict__ Bpl,
                                                     const int *__restrict__ Aexp, const int *__restrict__ Bexp,
                                                     double2 *__restrict__ C, const int *skip, int *err, int step,
@@ -536,19 +541,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restr
             int uses[STAGES] = {0, 0, 0};
             bool ok = true;
             for (int ti = blockIdx.x; ti < ntiles && ok; ti += gridDim.x) {
-                const GemmTile t = tiles[ti];
-                const int rt = t.m0 / BM, nt = t.n0 / BN;
+                const TcTile t = tiles[ti];
+                const int a_panel = NPL * BKC * t.rows;  // FP16 elements of one K panel of A
                 for (int s = t.seg_begin; s < t.seg_end && ok; ++s) {
                     const SegX g = segs[s];
                     if (g.entry > step) continue;
-                    const __half *ap = Apl + g.a_pan + (int64_t)rt * g.nkc * A_PANEL;
-                    const __half *bp = Bpl + g.b_pan + (int64_t)nt * g.nkc * B_PANEL;
+                    const __half *ap = Apl + g.a_pan;
+                    const __half *bp = Bpl + g.b_pan;
                     for (int kc = 0; kc < g.nkc && !no_copies; ++kc, ++it) {
                         const int st = it % STAGES;
                         const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
                         if (!mbar_wait(smem_u32(empty + st), ph ^ 1u, wait_limit)) { ok = false; break; }
-                        mbar_expect_tx(smem_u32(full + st), (uint32_t)(A_BYTES + B_BYTES));
-                        bulk_g2s(smem_u32(sA + st * A_BYTES), ap + (int64_t)kc * A_PANEL, A_BYTES,
+                        mbar_expect_tx(smem_u32(full + st), (uint32_t)(2 * a_panel + B_BYTES));
+                        bulk_g2s(smem_u32(sA + st * A_BYTES), ap + (int64_t)kc * a_panel, (uint32_t)(2 * a_panel),
                                  smem_u32(full + st));
                         bulk_g2s(smem_u32(sB + st * B_BYTES), bp + (int64_t)kc * B_PANEL, B_BYTES,
                                  smem_u32(full + st));
@@ -569,7 +574,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restr
             int it = 0, grp = 0;
             bool ok = true;
             for (int ti = blockIdx.x; ti < ntiles && ok; ti += gridDim.x) {
-                const GemmTile t = tiles[ti];
+                const TcTile t = tiles[ti];
+                const uint32_t pa = (uint32_t)(t.rows * BKC * 2) >> 4;
                 for (int s = t.seg_begin; s < t.seg_end && ok; ++s) {
                     if (segs[s].entry > step) continue;
                     const int nkc = segs[s].nkc;
@@ -585,8 +591,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restr
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             const uint64_t da = desc_a0 + (uint64_t)(st * (A_BYTES >> 4));
                             const uint64_t db = desc_b0 + (uint64_t)(st * (B_BYTES >> 4));
-                            if (kc == kc0) mma_panel<true>(tmem, da, db);
-                            else mma_panel<false>(tmem, da, db);
+                            if (t.rows == BM) {  // plane offsets known at compile time
+                                if (kc == kc0) mma_panel<true>(tmem, da, db, PLANE_A >> 4);
+                                else mma_panel<false>(tmem, da, db, PLANE_A >> 4);
+                            } else {
+                                if (kc == kc0) mma_panel<true>(tmem, da, db, pa);
+                                else mma_panel<false>(tmem, da, db, pa);
+                            }
                             mma_commit(smem_u32(empty + st));  // stage free once these MMAs are done
                         }
                         if (!ok) break;
@@ -611,17 +622,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restr
         bool ok = true;  // warp-uniform; after a timed-out wait the warp stops waiting but keeps the barriers
         int grp = 0;
         for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
-            const GemmTile t = tiles[ti];
+            const TcTile t = tiles[ti];
             const bool act = tile_active(t, segs, step);
+            const bool used = q * 32 < t.rows;  // warp-uniform: some row of this quarter is stored
             if (!act && !write_inactive) continue;  // the same for every epilogue warp
             const int nseg = t.seg_end - t.seg_begin;
+            // where this thread's row and the warp's 8 columns go (pieces start at
+            // multiples of 8, so the columns belong to one): read ahead of the drain
+            const int2 rm = maps[t.rowmap + m];  // (row piece, row of its block)
+            const int2 cm = maps[t.colmap + c_lo + (lane & (EPI_COLS - 1))];
+            const int ncol = __popc(__ballot_sync(0xFFFFFFFFu, lane < EPI_COLS && cm.x >= 0));
+            const int cpiece = __shfl_sync(0xFFFFFFFFu, cm.x, 0), col0 = __shfl_sync(0xFFFFFFFFu, cm.y, 0);
+            TcPair pr{-1, 0, kAllSteps};
+            if (rm.x >= 0 && cpiece >= 0) pr = pairs[t.pair + (int64_t)rm.x * t.ncol + cpiece];
+            const bool live = act && pr.entry <= step;
+            const bool mine = pr.c_off >= 0 && (live || write_inactive);
             int erow = kZeroExp;
             for (int s = t.seg_begin; s < t.seg_end; ++s)
-                if (segs[s].entry <= step) erow = max(erow, Aexp[segs[s].a_exp + t.m0 + m]);
+                if (segs[s].entry <= step) erow = max(erow, Aexp[segs[s].a_exp + m]);
             if (warp == 2) {
                 int ec = kZeroExp;
                 for (int s = t.seg_begin; s < t.seg_end; ++s)
-                    if (segs[s].entry <= step) ec = max(ec, Bexp[segs[s].b_exp + t.n0 + lane]);
+                    if (segs[s].entry <= step) ec = max(ec, Bexp[segs[s].b_exp + lane]);
                 s_ecol[lane] = ec;
             }
             epi_bar();  // s_ecol written; reached by every epilogue warp for every tile
@@ -632,15 +654,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restr
                 const SegX g = segs[t.seg_begin + sl];
                 if (g.entry > step) continue;
                 // column shifts of this segment, into the warp's own shared-memory slots
-                if (lane < EPI_COLS) fw[lane] = s_ecol[c_lo + lane] - Bexp[g.b_exp + t.n0 + c_lo + lane];
+                if (lane < EPI_COLS) fw[lane] = s_ecol[c_lo + lane] - Bexp[g.b_exp + c_lo + lane];
                 __syncwarp();
-                const int shr = erow - Aexp[g.a_exp + t.m0 + m];
+                const int shr = erow - Aexp[g.a_exp + m];
                 for (int kc0 = 0; kc0 < g.nkc; kc0 += GKC, ++grp) {
                     // warp-uniform decision: tcgen05.ld below is a warp-wide instruction
                     if (ok && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(accf), (uint32_t)grp & 1u, wait_limit)))
                         ok = false;
                     if (!ok) continue;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (used)
 #pragma unroll
                     for (int c0 = 0; c0 < EPI_COLS; c0 += 4) {
                         long long I[NCOMP][4];
@@ -672,22 +695,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const GemmTile *__restr
                 }
                 __syncwarp();  // fw is rewritten for the next segment
             }
-            const int gm = t.m0 + m;
-            if (ok && gm < t.M) {
-                double2 *crow = C + t.c_off + (int64_t)gm * t.ldc;
+            if (ok && mine) {
+                double2 *crow = C + pr.c_off + (int64_t)rm.y * pr.ldc + col0;
 #pragma unroll
                 for (int c = 0; c < EPI_COLS; ++c) {
-                    const int gn = t.n0 + c_lo + c;
-                    if (gn < t.N) {
-                        const int ec = s_ecol[c_lo + c];
-                        const int sc = erow + ec - 2 * FRAC + COMB_SHIFT;
-                        // a row or column holding Inf or NaN (slicer exponent above the
-                        // FP64 range) gives NaN, as the FP64 product would
-                        crow[gn] = (erow > kMaxFiniteExp || ec > kMaxFiniteExp)
-                                       ? make_double2(__longlong_as_double(0x7FF8000000000000ll),
-                                                      __longlong_as_double(0x7FF8000000000000ll))
-                                       : make_double2(i64_ldexp(cr[c], sc), i64_ldexp(ci[c], sc));
-                    }
+                    if (c >= ncol) break;  // warp-uniform
+                    const int ec = s_ecol[c_lo + c];
+                    const int sc = erow + ec - 2 * FRAC + COMB_SHIFT;
+                    // a row or column holding Inf or NaN (slicer exponent above the
+                    // FP64 range) gives NaN, as the FP64 product would
+                    crow[c] = !live ? make_double2(0.0, 0.0)
+                              : (erow > kMaxFiniteExp || ec > kMaxFiniteExp)
+                                  ? make_double2(__longlong_as_double(0x7FF8000000000000ll),
+                                                 __longlong_as_double(0x7FF8000000000000ll))
+                                  : make_double2(i64_ldexp(cr[c], sc), i64_ldexp(ci[c], sc));
                 }
             }
             epi_bar();  // every warp has used s_ecol before the next tile rewrites it
@@ -726,80 +747,97 @@ int *device_err_word(int dev) {
 
 }  // namespace
 
-// Slicing jobs and per-segment panel addresses of a mixed-precision plan:
-// one job per distinct (block, operation) view of A and of B.
+// Tiles, packs and slicing jobs of a tensor-core plan (GemmPlan::tiles holds the
+// output blocks; only a block's first entry, m0 = n0 = 0, is read).
+//
+// A U(1) block-sparse product is a set of dense products cut into small blocks
+// (8 x 8 at a D = 128 bond of 17 sectors), and a 128 x 32 tile per output block
+// costs the same however little of it is used.  Blocks are therefore packed:
+//  * blocks of one segment: A views that meet the same list of B views form a
+//    complete bipartite group; their rows and the B views' columns are stacked.
+//  * blocks of several segments: blocks with the same list of (B view, entry)
+//    share their columns; their rows are stacked (segment by segment).
+// Every output element keeps its own segments, row and column exponents, so
+// packing does not change a bit of the result.
+// The rows a tile takes (128, 64 or 32) follow a cost model: fewer rows make
+// more tiles for the SMs to share and smaller operand panels.
+// Measured, both GEMM launches of a D = 128 apply over 2992 blocks of 8 x 8 x 8
+// (8704 tiles before): 160 -> 32 us; over 62 blocks of 64 x 64: 27.2 -> 23.4 us
+// a launch; at D = 512, where blocks fill their tiles: 212 -> 215.
+namespace {
+
+struct Pack {
+    std::vector<std::array<int, 3>> pieces;  // view, first row, rows
+    int rows = 0;                            // with every piece padded to a multiple of 8
+};
+
+int pad8(int n) { return (n + 7) & ~7; }
+
+// rows of the views in order, cut into packs of at most `most` rows; unit[p] = index of each piece's view in `views`
+void make_packs(const std::vector<int> &views, const std::vector<int> &view_rows, int most, std::vector<Pack> *packs,
+                std::vector<std::vector<int>> *unit) {
+    Pack cur;
+    std::vector<int> cu;
+    auto flush = [&] {
+        if (cur.pieces.empty()) return;
+        packs->push_back(cur);
+        unit->push_back(cu);
+        cur = Pack{};
+        cu.clear();
+    };
+    for (size_t u = 0; u < views.size(); ++u)
+        for (int r = 0; r < view_rows[u];) {
+            if (cur.rows == most) flush();
+            const int n = std::min(view_rows[u] - r, most - cur.rows);
+            cur.pieces.push_back({views[u], r, n});
+            cu.push_back((int)u);
+            cur.rows += pad8(n);
+            r += n;
+        }
+    flush();
+}
+
+}  // namespace
+
 void plan_mixed(GemmPlan &g) {
-    g.ajobs.clear();
-    g.bjobs.clear();
-    g.xsegs.assign(g.segs.size(), SegX{});
-    g.a_planes = g.b_planes = 0;
-    g.a_exps = g.b_exps = 0;
-    std::vector<std::pair<int, int>> seg_mn(g.segs.size(), {0, 0});
-    std::vector<std::pair<int, int>> seg_job(g.segs.size(), {0, 0});  // (A view, B view) of each segment
-    for (auto &t : g.tiles)
-        for (int s = t.seg_begin; s < t.seg_end; ++s) seg_mn[s] = {t.M, t.N};
-    // one job per distinct (block offset, operation) of each operand
+    struct View {
+        int64_t off;
+        int rows, K, ld, trans, conj, ks = -1;
+    };
+    std::vector<View> av, bv;
     std::unordered_map<int64_t, int> amap, bmap;
+    struct Block {
+        int64_t c_off;
+        int ldc, M, N, sb, se;
+    };
+    std::vector<Block> blocks;
+    for (auto &t : g.tiles)
+        if (t.m0 == 0 && t.n0 == 0) blocks.push_back({t.c_off, t.ldc, t.M, t.N, t.seg_begin, t.seg_end});
+    // ---- views: one per distinct (block offset, operation) of each operand
+    std::vector<int> sa(g.segs.size(), -1), sb(g.segs.size(), -1);  // views of each segment
     amap.reserve(2 * g.segs.size());
     bmap.reserve(2 * g.segs.size());
-    for (size_t s = 0; s < g.segs.size(); ++s) {
-        const GemmSeg &sg = g.segs[s];
-        const int M = seg_mn[s].first, N = seg_mn[s].second;
-        if (M == 0) continue;  // segment of no tile
-        const int nkc = (sg.K + BKC - 1) / BKC;
-        auto ia = amap.find(sg.a_off * 4 + sg.opa);
-        if (ia == amap.end()) {
-            SliceJob j{};
-            j.src_off = sg.a_off;
-            j.dst_off = g.a_planes;
-            j.rows = M;
-            j.K = sg.K;
-            j.ld = sg.lda;
-            j.trans = (sg.opa == 1 || sg.opa == 2) ? 1 : 0;
-            j.conj = (sg.opa == 1 || sg.opa == 3) ? 1 : 0;
-            j.exp_off = (int)g.a_exps;
-            j.nkc = nkc;
-            j.entry = kAllSteps;
-            j.ks_off = -1;
-            const int nrt = (M + BM - 1) / BM;
-            g.a_planes += (int64_t)nrt * nkc * A_PANEL;
-            g.a_exps += (int64_t)nrt * BM;
-            ia = amap.emplace(sg.a_off * 4 + sg.opa, (int)g.ajobs.size()).first;
-            g.ajobs.push_back(j);
+    for (auto &b : blocks)
+        for (int s = b.sb; s < b.se; ++s) {
+            const GemmSeg &sg = g.segs[s];
+            auto ia = amap.emplace(sg.a_off * 4 + sg.opa, (int)av.size());
+            if (ia.second)
+                av.push_back({sg.a_off, b.M, sg.K, sg.lda, (sg.opa == 1 || sg.opa == 2) ? 1 : 0,
+                              (sg.opa == 1 || sg.opa == 3) ? 1 : 0});
+            auto ib = bmap.emplace(sg.b_off * 4 + sg.opb, (int)bv.size());
+            if (ib.second)  // B element (n, k) at b[k*ldb + n] for opb 0 and 3
+                bv.push_back({sg.b_off, b.N, sg.K, sg.ldb, (sg.opb == 0 || sg.opb == 3) ? 1 : 0,
+                              (sg.opb == 2 || sg.opb == 3) ? 1 : 0});
+            sa[s] = ia.first->second;
+            sb[s] = ib.first->second;
+            KV_REQUIRE(av[sa[s]].rows == b.M && bv[sb[s]].rows == b.N && av[sa[s]].K == sg.K && bv[sb[s]].K == sg.K,
+                       KV_EINVAL, "internal: inconsistent block views in a mixed-precision plan");
         }
-        auto ib = bmap.find(sg.b_off * 4 + sg.opb);
-        if (ib == bmap.end()) {
-            SliceJob j{};
-            j.src_off = sg.b_off;
-            j.dst_off = g.b_planes;
-            j.rows = N;
-            j.K = sg.K;
-            j.ld = sg.ldb;
-            j.trans = (sg.opb == 0 || sg.opb == 3) ? 1 : 0;  // B element (n, k) at b[k*ldb + n]
-            j.conj = (sg.opb == 2 || sg.opb == 3) ? 1 : 0;
-            j.exp_off = (int)g.b_exps;
-            j.nkc = nkc;
-            j.entry = kAllSteps;
-            j.ks_off = -1;
-            const int nnt = (N + BN - 1) / BN;
-            g.b_planes += (int64_t)nnt * nkc * B_PANEL;
-            g.b_exps += (int64_t)nnt * BN;
-            ib = bmap.emplace(sg.b_off * 4 + sg.opb, (int)g.bjobs.size()).first;
-            g.bjobs.push_back(j);
-        }
-        seg_job[s] = {ia->second, ib->second};
-        const SliceJob &ja = g.ajobs[ia->second], &jb = g.bjobs[ib->second];
-        KV_REQUIRE(ja.rows == M && jb.rows == N && ja.K == sg.K && jb.K == sg.K, KV_EINVAL,
-                   "internal: inconsistent block views in a mixed-precision plan");
-        g.xsegs[s] = SegX{ja.dst_off, jb.dst_off, nkc, ja.exp_off, jb.exp_off, sg.entry};
-        g.ajobs[ia->second].entry = std::min(g.ajobs[ia->second].entry, sg.entry);
-        g.bjobs[ib->second].entry = std::min(g.bjobs[ib->second].entry, sg.entry);
-    }
-    // balancing: A and B views joined by a segment share one vector of
+    // ---- balancing: A and B views joined by a segment share one vector of
     // per-k scales, so the views of each connected component get one range
     g.k_scales = 0;
     if (g.balance_k) {
-        const int na = (int)g.ajobs.size(), nb = (int)g.bjobs.size();
+        const int na = (int)av.size(), nb = (int)bv.size();
         std::vector<int> parent(na + nb);
         for (int i = 0; i < na + nb; ++i) parent[i] = i;
         auto root = [&](int x) {
@@ -807,38 +845,282 @@ void plan_mixed(GemmPlan &g) {
             return x;
         };
         for (size_t s = 0; s < g.segs.size(); ++s) {
-            if (seg_mn[s].first == 0) continue;
-            const int a = root(seg_job[s].first), b = root(na + seg_job[s].second);
+            if (sa[s] < 0) continue;
+            const int a = root(sa[s]), b = root(na + sb[s]);
             if (a != b) parent[a] = b;
         }
         std::vector<int64_t> comp_off(na + nb, -1);
         std::vector<int> comp_k(na + nb, -1);
-        auto assign = [&](SliceJob &j, int id) {
+        auto assign = [&](View &v, int id) {
             const int c = root(id);
             if (comp_off[c] < 0) {
                 comp_off[c] = g.k_scales;
-                comp_k[c] = j.K;
-                g.k_scales += j.K;
+                comp_k[c] = v.K;
+                g.k_scales += v.K;
             }
-            KV_REQUIRE(comp_k[c] == j.K, KV_EINVAL, "internal: views of one segment component differ in K");
-            j.ks_off = (int)comp_off[c];
+            KV_REQUIRE(comp_k[c] == v.K, KV_EINVAL, "internal: views of one segment component differ in K");
+            v.ks = (int)comp_off[c];
         };
-        for (int i = 0; i < na; ++i) assign(g.ajobs[i], i);
-        for (int i = 0; i < nb; ++i) assign(g.bjobs[i], na + i);
+        for (int i = 0; i < na; ++i) assign(av[i], i);
+        for (int i = 0; i < nb; ++i) assign(bv[i], na + i);
         KV_REQUIRE(g.k_scales < (1ll << 31), KV_EINVAL, "mixed-precision plan too large");
     }
-    g.aitems.clear();
-    g.bitems.clear();
-    for (size_t i = 0; i < g.ajobs.size(); ++i)
-        for (int r0 = 0; r0 < g.ajobs[i].rows; r0 += 8) g.aitems.push_back({(int)i, r0});
-    for (size_t i = 0; i < g.bjobs.size(); ++i)
-        for (int r0 = 0; r0 < g.bjobs[i].rows; r0 += 8) g.bitems.push_back({(int)i, r0});
-    KV_REQUIRE(g.a_exps < (1ll << 31) && g.b_exps < (1ll << 31), KV_EINVAL, "mixed-precision plan too large");
-    g.d_ajobs = upload_vec(g.ajobs);
-    g.d_bjobs = upload_vec(g.bjobs);
-    g.d_xsegs = upload_vec(g.xsegs);
-    g.d_aitems = upload_vec(g.aitems);
-    g.d_bitems = upload_vec(g.bitems);
+    // ---- groups
+    struct Group {
+        std::vector<int> rblk;                // row units: A views (one segment) or blocks (several)
+        std::vector<int> cview;               // column units: B views (one segment); several: the views per segment
+        std::vector<int> grid;                // one segment: block of (row unit, column unit)
+        bool multi;
+    };
+    std::vector<Group> groups;
+    std::vector<int> zero_blocks;
+    {
+        struct Hash {
+            size_t operator()(const std::vector<int> &v) const {
+                uint64_t h = 1469598103934665603ull;
+                for (int x : v) { h ^= (uint64_t)(uint32_t)x; h *= 1099511628211ull; }
+                return (size_t)h;
+            }
+        };
+        std::unordered_map<std::vector<int>, int, Hash> single, multi;
+        std::vector<std::vector<int>> alist(av.size());  // one-segment blocks of each A view, in block order
+        for (size_t b = 0; b < blocks.size(); ++b) {
+            const int n = blocks[b].se - blocks[b].sb;
+            if (n == 0) zero_blocks.push_back((int)b);
+            else if (n == 1) alist[sa[blocks[b].sb]].push_back((int)b);
+            else {
+                std::vector<int> key;
+                for (int s = blocks[b].sb; s < blocks[b].se; ++s) {
+                    key.push_back(sb[s]);
+                    key.push_back(g.segs[s].entry);
+                }
+                auto it = multi.emplace(key, (int)groups.size());
+                if (it.second) {
+                    Group gr;
+                    gr.multi = true;
+                    for (int s = blocks[b].sb; s < blocks[b].se; ++s) gr.cview.push_back(sb[s]);
+                    groups.push_back(gr);
+                }
+                groups[it.first->second].rblk.push_back((int)b);
+            }
+        }
+        for (size_t a = 0; a < av.size(); ++a) {
+            if (alist[a].empty()) continue;
+            std::vector<int> key;
+            for (int b : alist[a]) key.push_back(sb[blocks[b].sb]);
+            auto it = single.emplace(key, (int)groups.size());
+            if (it.second) {
+                Group gr;
+                gr.multi = false;
+                gr.cview = key;
+                groups.push_back(gr);
+            }
+            Group &gr = groups[it.first->second];
+            gr.rblk.push_back((int)a);
+            gr.grid.insert(gr.grid.end(), alist[a].begin(), alist[a].end());
+        }
+    }
+    // ---- rows per tile: estimated clocks of the busiest SM.  A K panel costs
+    // its operand bytes at about 45 B per clock or the MMAs' shared-memory
+    // reads, a drain about 1800 clocks, a tile 600 more (measured on GB300).
+    auto group_rows = [&](const Group &gr) {
+        int r = 0;
+        for (int u : gr.rblk) r += pad8(gr.multi ? blocks[u].M : av[u].rows);
+        return r;
+    };
+    auto group_cols = [&](const Group &gr) {
+        if (gr.multi) return bv[gr.cview[0]].rows;
+        int c = 0;
+        for (int v : gr.cview) c += pad8(bv[v].rows);
+        return c;
+    };
+    int most = BM;
+    {
+        double best = 0.0;
+        const double sms = std::max(1, ctx().num_sms);
+        for (int R : {128, 64, 32}) {
+            const double panel = std::max(800.0, (R + BN) * NPL * BKC * 2 / 45.0);
+            double sum = 0.0, top = 0.0, n = 0.0;
+            for (auto &gr : groups) {
+                const int s0 = gr.multi ? blocks[gr.rblk[0]].sb : blocks[gr.grid[0]].sb, ns = gr.multi ? (int)gr.cview.size() : 1;
+                double cost = 600.0;
+                for (int s = s0; s < s0 + ns; ++s) {
+                    const int nkc = (g.segs[s].K + BKC - 1) / BKC;
+                    cost += nkc * panel + ((nkc + GKC - 1) / GKC) * 1800.0;
+                }
+                const double tiles = (double)((group_rows(gr) + R - 1) / R) * ((group_cols(gr) + BN - 1) / BN);
+                sum += tiles * cost;
+                n += tiles;
+                top = std::max(top, cost);
+            }
+            const double t = std::max(top, n > 0 ? std::ceil(n / sms) * (sum / n) : 0.0);
+            if (R == 128 || t < 0.97 * best) {
+                best = t;
+                most = R;
+            }
+        }
+    }
+    // ---- packs (shared where the same pieces recur), tiles, maps, pairs
+    std::vector<SliceJob> ajobs, bjobs;
+    std::vector<SegX> xsegs;
+    std::vector<TcTile> tiles;
+    std::vector<TcPair> pairs;
+    std::vector<int2> maps;
+    g.a_planes = g.b_planes = g.a_exps = g.b_exps = 0;
+    struct Panel {
+        int64_t pan;
+        int exp;
+        int job0, njobs;
+    };
+    std::unordered_map<int64_t, Panel> bpanels;  // single-piece B packs by (view, first column)
+    auto add_pack = [&](const Pack &p, bool is_b) {
+        Panel o;
+        const std::vector<View> &vw = is_b ? bv : av;
+        std::vector<SliceJob> &jobs = is_b ? bjobs : ajobs;
+        const int tr = is_b ? BN : p.rows, K = vw[p.pieces[0][0]].K, nkc = (K + BKC - 1) / BKC;
+        o.pan = is_b ? g.b_planes : g.a_planes;
+        o.exp = (int)(is_b ? g.b_exps : g.a_exps);
+        o.job0 = (int)jobs.size();
+        int r0 = 0;
+        for (auto &pc : p.pieces) {
+            const View &v = vw[pc[0]];
+            KV_REQUIRE(v.K == K, KV_EINVAL, "internal: a pack's views differ in K");
+            jobs.push_back(SliceJob{v.off, o.pan, pc[1], pc[2], r0, tr, v.K, v.ld, v.trans, v.conj, o.exp + r0, nkc,
+                                    kAllSteps, v.ks});
+            r0 += pad8(pc[2]);
+        }
+        o.njobs = (int)jobs.size() - o.job0;
+        (is_b ? g.b_planes : g.a_planes) += (int64_t)nkc * NPL * BKC * tr;
+        (is_b ? g.b_exps : g.a_exps) += is_b ? BN : BM;
+        return o;
+    };
+    // a pair reads the pack's piece from step `entry` on (before that its block
+    // may not hold data yet)
+    auto seen = [&](const Panel &p, bool is_b, int piece, int entry) {
+        SliceJob &j = (is_b ? bjobs : ajobs)[p.job0 + piece];
+        j.entry = std::min(j.entry, entry);
+    };
+    auto add_map = [&](const Pack &p, int n) {  // (piece, row) of each of n panel rows
+        const int at = (int)maps.size();
+        for (size_t i = 0; i < p.pieces.size(); ++i) {
+            for (int r = 0; r < p.pieces[i][2]; ++r) maps.push_back(make_int2((int)i, p.pieces[i][1] + r));
+            for (int r = p.pieces[i][2]; r < pad8(p.pieces[i][2]); ++r) maps.push_back(make_int2(-1, 0));
+        }
+        while ((int)maps.size() < at + n) maps.push_back(make_int2(-1, 0));
+        return at;
+    };
+    for (auto &gr : groups) {
+        std::vector<Pack> rp, cp;
+        std::vector<std::vector<int>> ru, cu;
+        std::vector<int> rows;
+        if (!gr.multi) {
+            for (int a : gr.rblk) rows.push_back(av[a].rows);
+            make_packs(gr.rblk, rows, most, &rp, &ru);
+            std::vector<int> cols;
+            for (int v : gr.cview) cols.push_back(bv[v].rows);
+            make_packs(gr.cview, cols, BN, &cp, &cu);
+            std::vector<Panel> ap, bp;
+            std::vector<int> rmap, cmap;
+            for (auto &p : rp) { ap.push_back(add_pack(p, false)); rmap.push_back(add_map(p, BM)); }
+            for (auto &p : cp) { bp.push_back(add_pack(p, true)); cmap.push_back(add_map(p, BN)); }
+            const int nc = (int)gr.cview.size();
+            // kColBatch column packs meet every row pack before the next ones, so
+            // the panels of the tiles in flight stay in L2 (all columns a row pack
+            // at a time read B's panels from HBM once per row pack)
+            constexpr size_t kColBatch = 16;
+            std::vector<std::pair<size_t, size_t>> order;
+            for (size_t j0 = 0; j0 < cp.size(); j0 += kColBatch)
+                for (size_t i = 0; i < rp.size(); ++i)
+                    for (size_t j = j0; j < std::min(cp.size(), j0 + kColBatch); ++j) order.push_back({i, j});
+            {
+                for (auto [i, j] : order) {
+                    TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + 1, rmap[i], cmap[j], (int)pairs.size(),
+                             (int)cp[j].pieces.size()};
+                    int entry = kAllSteps;
+                    for (size_t u = 0; u < ru[i].size(); ++u)
+                        for (size_t v = 0; v < cu[j].size(); ++v) {
+                            const Block &b = blocks[gr.grid[(size_t)ru[i][u] * nc + cu[j][v]]];
+                            const int e = g.segs[b.sb].entry;
+                            pairs.push_back({b.c_off, b.ldc, e});
+                            entry = std::min(entry, e);
+                            seen(ap[i], false, (int)u, e);
+                            seen(bp[j], true, (int)v, e);
+                        }
+                    xsegs.push_back(SegX{ap[i].pan, bp[j].pan, (av[gr.rblk[0]].K + BKC - 1) / BKC, ap[i].exp, bp[j].exp,
+                                         entry});
+                    tiles.push_back(t);
+                }
+            continue;
+        }
+        for (int b : gr.rblk) rows.push_back(blocks[b].M);
+        make_packs(gr.rblk, rows, most, &rp, &ru);  // pieces name blocks here
+        const int ns = (int)gr.cview.size(), N = bv[gr.cview[0]].rows;
+        for (size_t i = 0; i < rp.size(); ++i) {
+            std::vector<Panel> ap;
+            const int rmap = add_map(rp[i], BM);
+            for (int s = 0; s < ns; ++s) {
+                Pack p = rp[i];
+                for (auto &pc : p.pieces) pc[0] = sa[blocks[pc[0]].sb + s];
+                ap.push_back(add_pack(p, false));
+            }
+            for (int n0 = 0; n0 < N; n0 += BN) {
+                Pack c;
+                c.pieces.push_back({0, n0, std::min(BN, N - n0)});
+                TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + ns, rmap, add_map(c, BN), (int)pairs.size(),
+                         1};
+                int entry = kAllSteps;
+                for (int s = 0; s < ns; ++s) {
+                    const GemmSeg &sg = g.segs[blocks[gr.rblk[0]].sb + s];
+                    const int64_t key = (int64_t)gr.cview[s] * (1 << 20) + n0 / BN;
+                    KV_REQUIRE(n0 / BN < (1 << 20), KV_EINVAL, "mixed-precision plan too large");
+                    auto it = bpanels.find(key);
+                    if (it == bpanels.end()) {
+                        c.pieces[0][0] = gr.cview[s];
+                        it = bpanels.emplace(key, add_pack(c, true)).first;
+                    }
+                    xsegs.push_back(SegX{ap[s].pan, it->second.pan, (sg.K + BKC - 1) / BKC, ap[s].exp, it->second.exp,
+                                         sg.entry});
+                    for (int x = 0; x < ap[s].njobs; ++x) seen(ap[s], false, x, sg.entry);
+                    seen(it->second, true, 0, sg.entry);
+                    entry = std::min(entry, sg.entry);
+                }
+                for (int u : ru[i]) pairs.push_back({blocks[gr.rblk[u]].c_off, blocks[gr.rblk[u]].ldc, entry});
+                tiles.push_back(t);
+            }
+        }
+    }
+    for (int z : zero_blocks) {  // written as zeros (or skipped) by tiles without segments
+        const Block &b = blocks[z];
+        for (int m0 = 0; m0 < b.M; m0 += BM)
+            for (int n0 = 0; n0 < b.N; n0 += BN) {
+                Pack r, c;
+                r.pieces.push_back({0, m0, std::min(BM, b.M - m0)});
+                c.pieces.push_back({0, n0, std::min(BN, b.N - n0)});
+                const int rm = add_map(r, BM), cm = add_map(c, BN);
+                tiles.push_back(TcTile{pad8(r.pieces[0][2]), (int)xsegs.size(), (int)xsegs.size(), rm, cm,
+                                       (int)pairs.size(), 1});
+                pairs.push_back({b.c_off, b.ldc, kAllSteps});
+            }
+    }
+    std::vector<int2> aitems, bitems;
+    for (size_t i = 0; i < ajobs.size(); ++i)
+        for (int r0 = 0; r0 < ajobs[i].rows; r0 += 8) aitems.push_back({(int)i, r0});
+    for (size_t i = 0; i < bjobs.size(); ++i)
+        for (int r0 = 0; r0 < bjobs[i].rows; r0 += 8) bitems.push_back({(int)i, r0});
+    KV_REQUIRE(g.a_exps < (1ll << 31) && g.b_exps < (1ll << 31) && maps.size() < (1ull << 31) &&
+                   pairs.size() < (1ull << 31),
+               KV_EINVAL, "mixed-precision plan too large");
+    g.tc_tiles = (int)tiles.size();
+    g.na_items = (int)aitems.size();
+    g.nb_items = (int)bitems.size();
+    g.d_tctiles = upload_vec(tiles);
+    g.d_xsegs = upload_vec(xsegs);
+    g.d_maps = upload_vec(maps);
+    g.d_pairs = upload_vec(pairs);
+    g.d_ajobs = upload_vec(ajobs);
+    g.d_bjobs = upload_vec(bjobs);
+    g.d_aitems = upload_vec(aitems);
+    g.d_bitems = upload_vec(bitems);
 }
 
 // Grid of the cooperative slicing launch on a device: every CTA resident at
@@ -861,17 +1143,17 @@ static int slice_coop_grid(int device) {
 void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, double2 *C, double alpha,
                        const int *skip, int step) {
     if (p.tiles.empty()) return;
-    KV_REQUIRE(p.tile_m == BM && p.tile_n == BN && p.xsegs.size() == p.segs.size(), KV_EINVAL,
+    KV_REQUIRE(p.tile_m == BM && p.tile_n == BN && p.tc_tiles > 0, KV_EINVAL,
                "internal: GEMM plan not prepared for the tensor-core path");
     auto &c = ctx();
     int *err = device_err_word(c.device);
     DevBuf ap(std::max<int64_t>(1, p.a_planes) * sizeof(__half)), bp(std::max<int64_t>(1, p.b_planes) * sizeof(__half));
     DevBuf ae(std::max<int64_t>(1, p.a_exps) * sizeof(int)), be(std::max<int64_t>(1, p.b_exps) * sizeof(int));
     int n = 0;
-    const bool bal = p.balance_k && p.k_scales > 0 && !p.aitems.empty() && !p.bitems.empty();
+    const bool bal = p.balance_k && p.k_scales > 0 && p.na_items > 0 && p.nb_items > 0;
     DevBuf kmax(bal ? 2 * (size_t)p.k_scales * sizeof(unsigned long long) : 8);
     unsigned long long *km = bal ? kmax.as<unsigned long long>() : nullptr;
-    int na = (int)p.aitems.size(), nb = (int)p.bitems.size();
+    int na = p.na_items, nb = p.nb_items;
     const int grid = slice_coop_grid(c.device);
     if (na + nb > 0 && &c == &main_ctx() && grid > 0) {
         // one cooperative launch (zero, maxima, slicing); only on the main
@@ -903,9 +1185,9 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
         ++n;
     }
     // persistent: one CTA per SM at most (the kernel holds all of an SM's tensor memory)
-    const int ntiles = (int)p.tiles.size();
+    const int ntiles = p.tc_tiles;
     k_gemm_tc<<<(unsigned)std::min(ntiles, c.num_sms), NTHREADS, SMEM_BYTES, c.stream>>>(
-        p.d_tiles.as<GemmTile>(), ntiles, p.d_xsegs.as<SegX>(), ap.as<__half>(), bp.as<__half>(), ae.as<int>(),
+        p.d_tctiles.as<TcTile>(), ntiles, p.d_xsegs.as<SegX>(), p.d_maps.as<int2>(), p.d_pairs.as<TcPair>(), ap.as<__half>(), bp.as<__half>(), ae.as<int>(),
         be.as<int>(), C, skip, err, step, p.write_inactive ? 1 : 0, g_stall_test ? (1ll << 10) : WAIT_LIMIT,
         g_stall_test);
     KV_CUDA(cudaGetLastError());
