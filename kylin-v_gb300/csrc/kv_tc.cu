@@ -1032,24 +1032,23 @@ void plan_mixed(GemmPlan &g) {
             for (size_t j0 = 0; j0 < cp.size(); j0 += kColBatch)
                 for (size_t i = 0; i < rp.size(); ++i)
                     for (size_t j = j0; j < std::min(cp.size(), j0 + kColBatch); ++j) order.push_back({i, j});
-            {
-                for (auto [i, j] : order) {
-                    TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + 1, rmap[i], cmap[j], (int)pairs.size(),
-                             (int)cp[j].pieces.size()};
-                    int entry = kAllSteps;
-                    for (size_t u = 0; u < ru[i].size(); ++u)
-                        for (size_t v = 0; v < cu[j].size(); ++v) {
-                            const Block &b = blocks[gr.grid[(size_t)ru[i][u] * nc + cu[j][v]]];
-                            const int e = g.segs[b.sb].entry;
-                            pairs.push_back({b.c_off, b.ldc, e});
-                            entry = std::min(entry, e);
-                            seen(ap[i], false, (int)u, e);
-                            seen(bp[j], true, (int)v, e);
-                        }
-                    xsegs.push_back(SegX{ap[i].pan, bp[j].pan, (av[gr.rblk[0]].K + BKC - 1) / BKC, ap[i].exp, bp[j].exp,
-                                         entry});
-                    tiles.push_back(t);
-                }
+            for (auto [i, j] : order) {
+                TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + 1, rmap[i], cmap[j], (int)pairs.size(),
+                         (int)cp[j].pieces.size()};
+                int entry = kAllSteps;
+                for (size_t u = 0; u < ru[i].size(); ++u)
+                    for (size_t v = 0; v < cu[j].size(); ++v) {
+                        const Block &b = blocks[gr.grid[(size_t)ru[i][u] * nc + cu[j][v]]];
+                        const int e = g.segs[b.sb].entry;
+                        pairs.push_back({b.c_off, b.ldc, e});
+                        entry = std::min(entry, e);
+                        seen(ap[i], false, (int)u, e);
+                        seen(bp[j], true, (int)v, e);
+                    }
+                xsegs.push_back(SegX{ap[i].pan, bp[j].pan, (av[gr.rblk[0]].K + BKC - 1) / BKC, ap[i].exp, bp[j].exp,
+                                     entry});
+                tiles.push_back(t);
+            }
             continue;
         }
         for (int b : gr.rblk) rows.push_back(blocks[b].M);
