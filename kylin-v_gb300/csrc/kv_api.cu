@@ -123,6 +123,9 @@ void context_close(Context &c) {
     c.stop_host = c.stop_dev = nullptr;
     for (auto &e : c.ev_free) cudaEventDestroy(e);
     c.ev_free.clear();
+    if (c.kmax) cudaFreeAsync(c.kmax, c.stream);
+    c.kmax = nullptr;
+    c.kmax_n = 0;
     KV_CUDA(cudaStreamSynchronize(c.stream));
     KV_CUDA(cudaStreamDestroy(c.stream));
     c.stream = nullptr;

@@ -84,6 +84,9 @@ struct Context {
     cudaEvent_t ring_ev[kRingChunks] = {};
     bool ring_live[kRingChunks] = {};
     PlanCache *plans = nullptr;
+    // balancing maxima of the tensor-core GEMM's slicing (kv_tc.cu), zero between calls
+    int *kmax = nullptr;
+    int64_t kmax_n = 0;
     // charge sectors through the mixed/FP64 SVD: count, columns, rank
     // reached by the QR reduction (else min(rows, columns)), Jacobi sweeps
     struct SvdStats {

@@ -14,9 +14,8 @@
 //     the exact integer sum X_re + X_im).  Integer arithmetic only.  Where
 //     the contracted index runs over parts of very different magnitude (MPO
 //     channels, Schmidt values), it is first balanced by exact powers of two
-//     (kmax_item, GemmPlan::balance_k; on the main stream the maxima and the
-//     slicing are one cooperative launch, k_slice_coop, with grid barriers
-//     between zeroing, maxima and slicing).  The digits are written directly in the
+//     (kmax_item, GemmPlan::balance_k; the maxima and the slicing are one
+//     launch with a barrier between them, k_slice_coop or k_slice_cluster).  The digits are written directly in the
 //     tensor cores' shared-memory panel layout (K-major, no swizzle: 8-row x
 //     16-byte core matrices, K-adjacent core matrices 128 B apart, 8-row
 //     groups 256 B apart), one 16-deep K panel after another, all 15 digit
@@ -114,38 +113,39 @@ __device__ __forceinline__ long long fixq(double x, int e) {
     return (u >> 63) ? -X : X;
 }
 
-__device__ __forceinline__ void digits(long long X, int d[NDIG]) {
-#pragma unroll
-    for (int i = NDIG - 1; i > 0; --i) {
-        d[i] = (int)(((X + 128) & 255) - 128);
-        X = (X - d[i]) >> 8;  // exact
-    }
-    d[0] = (int)X;
-}
-
 // element offset of (row r, k) inside one plane of a panel 16 deep
 __device__ __forceinline__ int panel_off(int r, int k) {
     return (r >> 3) * 128 + (k >> 3) * 64 + (r & 7) * 8 + (k & 7);
 }
 
-// two digits (|d| <= 512) as FP16: 1536 + d in the binade [1024, 2048) has
-// unit spacing, so its bits are 0x6600 + d; subtracting 1536 is exact
-__device__ __forceinline__ __half2 digits2(int d0, int d1) {
-    const uint32_t u = (uint32_t)(0x6600 + d0) | ((uint32_t)(0x6600 + d1) << 16);
-    __half2 h;
-    memcpy(&h, &u, sizeof(h));
-    return __hsub2(h, __float2half2_rn(1536.f));
+// The five balanced base-256 digits of X0 and X1 as FP16 pairs.  Adding 128 at
+// each of the four low digits makes the digits plus 128 the bytes of Y.  Two
+// digits |d| <= 512 as FP16: 1536 + d in the binade [1024, 2048) has unit
+// spacing, so its bits are 0x6600 + d; subtracting 1536 is exact.
+__device__ __forceinline__ void digit_pairs(long long X0, long long X1, __half2 out[NDIG]) {
+    static_assert(NDIG == 5, "four bytes and a leading digit");
+    const long long Y0 = X0 + 0x80808080ll, Y1 = X1 + 0x80808080ll;
+    const uint32_t l0 = (uint32_t)Y0, l1 = (uint32_t)Y1;
+    auto half2_of = [](uint32_t u) {
+        __half2 h;
+        memcpy(&h, &u, sizeof(h));
+        return __hsub2(h, __float2half2_rn(1536.f));
+    };
+    const uint32_t h0 = (uint32_t)(0x6600 + (int)(Y0 >> 32)), h1 = (uint32_t)(0x6600 + (int)(Y1 >> 32));
+    out[0] = half2_of(__byte_perm(h0, h1, 0x5410));
+    out[1] = half2_of((__byte_perm(l0, l1, 0x0703) & 0x00FF00FFu) + 0x65806580u);
+    out[2] = half2_of((__byte_perm(l0, l1, 0x0602) & 0x00FF00FFu) + 0x65806580u);
+    out[3] = half2_of((__byte_perm(l0, l1, 0x0501) & 0x00FF00FFu) + 0x65806580u);
+    out[4] = half2_of((__byte_perm(l0, l1, 0x0400) & 0x00FF00FFu) + 0x65806580u);
 }
 
-// One CTA per (job, 8 consecutive rows); one warp per row: pass 1 finds the
-// row exponent, pass 2 writes the digits of two adjacent K positions per lane.
-// Balancing of the contracted index k: kmax[k] holds the largest |re|, |im|
-// of A's column k over the A views of a segment component, kmax[kscales + k]
-// that of B's row k.  A's column is scaled by 2^s, B's row by 2^-s, with
-// s = floor((E_B - E_A) / 2) from their binary exponents, so both reach about
+// Balancing of the contracted index k: kmax[k] holds the largest binary
+// exponent (biased, 0: none) of re, im in A's column k over the A views of a
+// segment component, kmax[kscales + k] that of B's row k.  A's column is scaled
+// by 2^s, B's row by 2^-s, with s = floor((E_B - E_A) / 2), so both reach about
 // sqrt(max_A max_B) and every digit product is resolved at the same scale.
-__device__ __forceinline__ int balance_shift(const unsigned long long *kmax, int64_t kscales, int64_t k, int b_side) {
-    const int ea = (int)(kmax[k] >> 52), eb = (int)(kmax[kscales + k] >> 52);
+__device__ __forceinline__ int balance_shift(const int *kmax, int64_t kscales, int64_t k, int b_side) {
+    const int ea = __ldcg(kmax + k), eb = __ldcg(kmax + kscales + k);
     if (ea == 0 || eb == 0) return 0;
     const int sh = (eb - ea) >> 1;
     return b_side ? -sh : sh;
@@ -166,171 +166,216 @@ __device__ __forceinline__ double scale_exp(double x, int sh) {
     return __longlong_as_double((long long)((u & ~(0x7FFull << 52)) | ((unsigned long long)En << 52)));
 }
 
-// Per-k maxima for balancing: one CTA per (view, 8 rows), one warp per row;
-// the 8 rows' values are reduced in shared memory, then one atomicMax per k
-// (non-negative doubles order like their bit patterns).
-// item bid of the A items followed by the B items (CTA-uniform)
-__device__ __forceinline__ void kmax_item(const SliceJob *__restrict__ ajobs, const int2 *__restrict__ aitems, int na,
-                                          const SliceJob *__restrict__ bjobs, const int2 *__restrict__ bitems,
-                                          const double2 *__restrict__ A, const double2 *__restrict__ B,
-                                          unsigned long long *kmax, int64_t kscales, int step, int bid) {
-    __shared__ unsigned long long red[8][33];
-    const bool is_b = bid >= na;
-    const int2 it = is_b ? bitems[bid - na] : aitems[bid];
-    const SliceJob j = is_b ? bjobs[it.x] : ajobs[it.x];
-    if (j.entry > step || j.ks_off < 0) return;  // uniform over the CTA
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = it.y + warp;
-    const double2 *s = (is_b ? B : A) + j.src_off;
-    unsigned long long *dst = kmax + (is_b ? kscales : 0) + j.ks_off;
-    for (int k0 = 0; k0 < j.K; k0 += 32) {
-        const int k = k0 + lane;
-        unsigned long long m = 0;
-        if (r < j.rows && k < j.K) {
-            const int64_t row = j.row0 + r;
-            const double2 v = s[j.trans ? (int64_t)k * j.ld + row : row * j.ld + k];
-            const unsigned long long br = (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFull;
-            const unsigned long long bi = (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFull;
-            m = max(br, bi);
-        }
-        red[warp][lane] = m;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long x = 0;
+// the high word of |x| with its last bit set if only the low word is nonzero:
+// ordered by magnitude up to the exponent, zero only for x = 0
+__device__ __forceinline__ int magnitude(double x) {
+    return (__double2hiint(x) & 0x7FFFFFFF) | (__double2loint(x) != 0 ? 1 : 0);
+}
+
+// Slicing works on items of 8 rows (one core matrix high), GW warps an item
+// splitting its K range in steps of 8.  Lane l of a warp holds row l / 4 and
+// the K positions 2 (l % 4) and + 1 of a step: a step's digits of one plane are
+// one 128-byte core matrix, written by one coalesced store (a row a warp wrote
+// 16-byte pieces of eight lines), and both operand orders are read in 64 or
+// 128-byte pieces.
+struct SliceArgs {
+    const SliceJob *ajobs, *bjobs;
+    const int2 *aitems, *bitems;
+    int na, nb;
+    const double2 *A, *B;
+    __half *ap, *bp;
+    int *ae, *be;
+    double alpha;
+    int step;
+    int *err;
+    int *kmax;  // null: no balancing
+    int64_t kscales;
+};
+
+struct SliceLane {
+    SliceJob j;
+    const double2 *src;
+    int64_t base;  // element (row, 0)
+    int64_t kst;   // elements per k
+    bool on;       // the lane's row exists
+    bool is_b;
+    int rr;        // row within the panel
+};
+// the item's job and this lane's row; false: no active segment reads it
+__device__ __forceinline__ bool slice_open(const SliceArgs &a, int item, SliceLane &x) {
+    x.is_b = item >= a.na;
+    const int2 it = x.is_b ? a.bitems[item - a.na] : a.aitems[item];
+    x.j = x.is_b ? a.bjobs[it.x] : a.ajobs[it.x];
+    if (x.j.entry > a.step) return false;
+    const int r = it.y + ((threadIdx.x & 31) >> 2);
+    x.on = r < x.j.rows;
+    x.rr = x.j.r0 + r;
+    const int64_t row = x.j.row0 + r;
+    x.src = (x.is_b ? a.B : a.A) + x.j.src_off;
+    x.base = x.j.trans ? row : row * x.j.ld;
+    x.kst = x.j.trans ? x.j.ld : 1;
+    return true;
+}
+__device__ __forceinline__ double2 slice_raw(const SliceLane &x, int k) {
+    return x.on && k < x.j.K ? x.src[x.base + k * x.kst] : make_double2(0.0, 0.0);
+}
+
+// largest exponents per k over the item's rows, into kmax
+__device__ __forceinline__ void kmax_item(const SliceArgs &a, int item, int w, int GW) {
+    SliceLane x;
+    if (!slice_open(a, item, x) || x.j.ks_off < 0) return;  // uniform over the item's warps
+    const int lane = threadIdx.x & 31;
+    int *dst = a.kmax + (x.is_b ? a.kscales : 0) + x.j.ks_off;
+    for (int k0 = 8 * w; k0 < x.j.K; k0 += 8 * GW) {
+        const int k = k0 + 2 * (lane & 3);
+        const double2 v0 = slice_raw(x, k), v1 = slice_raw(x, k + 1);
+        const int e0 = max(__double2hiint(v0.x) & 0x7FFFFFFF, __double2hiint(v0.y) & 0x7FFFFFFF) >> 20;
+        const int e1 = max(__double2hiint(v1.x) & 0x7FFFFFFF, __double2hiint(v1.y) & 0x7FFFFFFF) >> 20;
+        unsigned m = (unsigned)e0 | ((unsigned)e1 << 16);
 #pragma unroll
-            for (int w = 0; w < 8; ++w) x = max(x, red[w][lane]);
-            if (x && k < j.K) atomicMax(dst + k, x);
+        for (int o = 4; o < 32; o <<= 1) m = __vmaxu2(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+        if (lane < 4) {
+            if (k < x.j.K && (m & 0xFFFF)) atomicMax(dst + k, (int)(m & 0xFFFF));
+            if (k + 1 < x.j.K && (m >> 16)) atomicMax(dst + k + 1, (int)(m >> 16));
         }
-        __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(256) k_kmax(const SliceJob *__restrict__ ajobs, const int2 *__restrict__ aitems,
-                                              int na, const SliceJob *__restrict__ bjobs,
-                                              const int2 *__restrict__ bitems, const double2 *__restrict__ A,
-                                              const double2 *__restrict__ B, unsigned long long *kmax,
-                                              int64_t kscales, const int *skip, int step) {
-    if (skip && *skip) return;
-    kmax_item(ajobs, aitems, na, bjobs, bitems, A, B, kmax, kscales, step, (int)blockIdx.x);
-}
-
-// One slicing item (a job's 8 rows from it.y, one per warp).  A row holding
-// an Inf or NaN sets bit kErrNonFinite of *err: fixed point has no code for
-// it, and the digits written for that row are meaningless.  Warps return on
-// their own; there is no barrier here.
-__device__ __forceinline__ void slice_item(const SliceJob *__restrict__ jobs, int2 it, const double2 *__restrict__ src,
-                                           __half *__restrict__ dst, int *__restrict__ exps, double alpha, int step,
-                                           int *err, const unsigned long long *kmax, int64_t kscales, int b_side) {
-    const SliceJob j = jobs[it.x];
-    if (j.entry > step) return;  // no active segment reads this block
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = it.y + warp;
-    // rows past the piece (up to a multiple of 8) are not written: they only
-    // reach output rows / columns the GEMM epilogue never stores
-    if (r >= j.rows) return;
-    const int64_t row = j.row0 + r;
-    const int kpad = j.nkc * BKC;
-    const double2 *s = src + j.src_off;
-    const bool scale = alpha != 1.0;
-    const bool bal = kmax != nullptr && j.ks_off >= 0;
+// One item's digits.  A row holding an Inf or NaN sets bit kErrNonFinite of
+// *err: fixed point has no code for it, and the digits written for that row are
+// meaningless.  red: [GW][8] shared words of the item's warps; bar: their
+// named barrier.
+__device__ __forceinline__ void slice_item(const SliceArgs &a, int item, int w, int GW, int (*red)[8], int bar) {
+    SliceLane x;
+    if (!slice_open(a, item, x)) return;  // uniform over the item's warps
+    const int lane = threadIdx.x & 31;
+    const bool scale = x.is_b && a.alpha != 1.0, bal = a.kmax != nullptr && x.j.ks_off >= 0;
+    const int nst = 2 * x.j.nkc;  // steps of 8, zero-padded past K
     auto load = [&](int k) {
-        double2 v = s[j.trans ? (int64_t)k * j.ld + row : row * j.ld + k];
-        if (scale) { v.x *= alpha; v.y *= alpha; }
-        if (j.conj) v.y = -v.y;
-        if (bal) {  // exact power-of-two balancing of the contracted index
-            const int sh = balance_shift(kmax, kscales, j.ks_off + k, b_side);
+        double2 v = slice_raw(x, k);
+        if (scale) { v.x *= a.alpha; v.y *= a.alpha; }
+        if (x.j.conj) v.y = __hiloint2double(__double2hiint(v.y) ^ (int)0x80000000, __double2loint(v.y));
+        if (bal && k < x.j.K) {  // exact power-of-two balancing of the contracted index
+            const int sh = balance_shift(a.kmax, a.kscales, x.j.ks_off + k, x.is_b ? 1 : 0);
             v.x = scale_exp(v.x, sh);
             v.y = scale_exp(v.y, sh);
         }
         return v;
     };
-    unsigned long long mx = 0;
-    for (int k = lane; k < j.K; k += 32) {
-        const double2 v = load(k);
-        const unsigned long long br = (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFull;
-        const unsigned long long bi = (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFull;
-        mx = max(mx, max(br, bi));
-    }
+    constexpr int KEEP = 4;  // steps whose elements stay in registers between the two passes
+    double2 kept[KEEP][2];
+    int mx = 0;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) mx = max(mx, (unsigned long long)__shfl_xor_sync(0xFFFFFFFFu, mx, o));
-    const int e = mx ? (int)(mx >> 52) - 1022 : kZeroExp;
-    if (lane == 0) {
-        exps[j.exp_off + r] = e;
-        if (mx >= 0x7FF0000000000000ull) atomicOr(err, kErrNonFinite);
+    for (int i = 0; i < KEEP; ++i) {
+        const int st = w + i * GW;
+        if (st >= nst) break;  // warp-uniform
+        const int k = 8 * st + 2 * (lane & 3);
+        kept[i][0] = load(k);
+        kept[i][1] = load(k + 1);
+        mx = max(mx, max(max(magnitude(kept[i][0].x), magnitude(kept[i][0].y)),
+                         max(magnitude(kept[i][1].x), magnitude(kept[i][1].y))));
     }
-    __half *pan = dst + j.dst_off;
-    const int rr = j.r0 + r, plane = j.tr * BKC;  // elements of a digit plane
-    for (int k = 2 * lane; k < kpad; k += 64) {  // k even: k and k + 1 are adjacent in the panel
-        long long x[2][NCOMP];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            long long xr = 0, xi = 0;
-            if (k + h < j.K) {
-                const double2 v = load(k + h);
-                xr = fixq(v.x, e);
-                xi = fixq(v.y, e);
-            }
-            x[h][0] = xr;
-            x[h][1] = xi;
-            x[h][2] = xr + xi;
-        }
-        __half *p = pan + (int64_t)(k / BKC) * (NPL * plane) + panel_off(rr, k & (BKC - 1));
+    for (int st = w + KEEP * GW; st < nst; st += GW) {
+        const int k = 8 * st + 2 * (lane & 3);
+        const double2 v0 = load(k), v1 = load(k + 1);
+        mx = max(mx, max(max(magnitude(v0.x), magnitude(v0.y)), max(magnitude(v1.x), magnitude(v1.y))));
+    }
+    mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+    mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+    if (GW > 1) {
+        if ((lane & 3) == 0) red[w][lane >> 2] = mx;
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * GW) : "memory");
+        for (int i = 0; i < GW; ++i) mx = max(mx, red[i][lane >> 2]);
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * GW) : "memory");  // red is free for the next item
+    }
+    const int e = mx ? (mx >> 20) - 1022 : kZeroExp;
+    if (w == 0 && (lane & 3) == 0 && x.on) {
+        (x.is_b ? a.be : a.ae)[x.j.exp_off + x.rr - x.j.r0] = e;
+        if (mx >= 0x7FF00000) atomicOr(a.err, kErrNonFinite);
+    }
+    // rows past the piece are not written: they only reach output rows /
+    // columns the GEMM epilogue never stores
+    if (!x.on) return;
+    const int plane = x.j.tr * BKC;  // elements of a digit plane
+    __half *pan = (x.is_b ? a.bp : a.ap) + x.j.dst_off;
+    auto put = [&](int st, double2 v0, double2 v1) {
+        const int k = 8 * st + 2 * (lane & 3);
+        long long X[2][NCOMP];
+        X[0][0] = fixq(v0.x, e);
+        X[0][1] = fixq(v0.y, e);
+        X[0][2] = X[0][0] + X[0][1];
+        X[1][0] = fixq(v1.x, e);
+        X[1][1] = fixq(v1.y, e);
+        X[1][2] = X[1][0] + X[1][1];
+        __half *p = pan + (int64_t)(k / BKC) * (NPL * plane) + panel_off(x.rr, k & (BKC - 1));
 #pragma unroll
         for (int c = 0; c < NCOMP; ++c) {
-            int d0[NDIG], d1[NDIG];
-            digits(x[0][c], d0);
-            digits(x[1][c], d1);
+            __half2 d[NDIG];
+            digit_pairs(X[0][c], X[1][c], d);
 #pragma unroll
-            for (int i = 0; i < NDIG; ++i)
-                *reinterpret_cast<__half2 *>(p + (c * NDIG + i) * plane) = digits2(d0[i], d1[i]);
+            for (int i = 0; i < NDIG; ++i) *reinterpret_cast<__half2 *>(p + (c * NDIG + i) * plane) = d[i];
         }
+    };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) {
+        const int st = w + i * GW;
+        if (st >= nst) break;
+        put(st, kept[i][0], kept[i][1]);
+    }
+    for (int st = w + KEEP * GW; st < nst; st += GW) {
+        const int k = 8 * st + 2 * (lane & 3);
+        put(st, load(k), load(k + 1));
     }
 }
 
-// Both operands' slicing in one launch: CTAs [0, na) take the A items, the
-// rest the B items.
-__global__ void __launch_bounds__(256) k_slice_ab(const SliceJob *__restrict__ ajobs, const int2 *__restrict__ aitems,
-                                                  int na, const SliceJob *__restrict__ bjobs,
-                                                  const int2 *__restrict__ bitems, const double2 *__restrict__ A,
-                                                  const double2 *__restrict__ B, __half *__restrict__ ap,
-                                                  __half *__restrict__ bp, int *__restrict__ ae,
-                                                  int *__restrict__ be, double alpha, const int *skip, int step,
-                                                  int *err, const unsigned long long *kmax, int64_t kscales) {
-    if (skip && *skip) return;
-    const int bid = (int)blockIdx.x;
-    if (bid < na) slice_item(ajobs, aitems[bid], A, ap, ae, 1.0, step, err, kmax, kscales, 0);
-    else slice_item(bjobs, bitems[bid - na], B, bp, be, alpha, step, err, kmax, kscales, 1);
+constexpr int kSliceWarps = 8;
+
+// Both operands' slicing (the A items, then the B items), CTA `cta` of `ctas`.
+// MAX: the balancing maxima only; otherwise the digits.
+template <bool MAX>
+__device__ __forceinline__ void slice_walk(const SliceArgs &a, int GW, int cta, int ctas) {
+    __shared__ int red[kSliceWarps][8];
+    const int warp = threadIdx.x >> 5, per = kSliceWarps / GW, grp = warp / GW, w = warp % GW;
+    for (int item = cta * per + grp; item < a.na + a.nb; item += ctas * per) {
+        if constexpr (MAX) kmax_item(a, item, w, GW);
+        else slice_item(a, item, w, GW, red + grp * GW, 1 + grp);
+    }
 }
 
-// The balanced slicing as one cooperative launch: zero the per-index maxima,
-// grid barrier, the maxima of every contracted index (k_kmax's work), grid
-// barrier, both operands' slicing (k_slice_ab's work); each CTA walks the
-// items with a stride of the grid.  kmax == nullptr: no balancing, no barrier.
-__global__ void __launch_bounds__(256) k_slice_coop(const SliceJob *__restrict__ ajobs,
-                                                    const int2 *__restrict__ aitems, int na,
-                                                    const SliceJob *__restrict__ bjobs,
-                                                    const int2 *__restrict__ bitems, int nb,
-                                                    const double2 *__restrict__ A, const double2 *__restrict__ B,
-                                                    __half *__restrict__ ap, __half *__restrict__ bp,
-                                                    int *__restrict__ ae, int *__restrict__ be, double alpha,
-                                                    const int *skip, int step, int *err, unsigned long long *kmax,
-                                                    int64_t kscales) {
-    namespace cg = cooperative_groups;
+// One launch: the maxima of every contracted index, a barrier, the digits; the
+// maxima start from zero (k_gemm_tc of the previous call cleared them).
+//  * a grid barrier (cooperative launch) on the main context's stream;
+//  * a cluster barrier for few items: a cluster is scheduled whole, so worker
+//    streams can use it too.
+//  * two launches (k_slice_max, k_slice_put) for many items on worker streams.
+// What bounds it: integer instructions and the chain maxima, barrier, row
+// maxima for small operands; the panels' traffic (30 B written a complex
+// element) for large ones.  Measured (us a launch, a row per warp and three
+// grid barriers before): D = 32 12.5 -> 8.8, D = 128 two-site 30.2 -> 24.1 and
+// over 8 x 8 blocks 28.2 -> 13.1, D = 512 204 -> 127.
+__global__ void __launch_bounds__(32 * kSliceWarps) k_slice_coop(SliceArgs a, int GW, const int *skip) {
     if (skip && *skip) return;  // uniform over the grid: nothing in this launch writes it
-    const int nitems = na + nb;
-    if (kmax) {
-        cg::grid_group grid = cg::this_grid();
-        for (int64_t e = blockIdx.x * 256ll + threadIdx.x; e < 2 * kscales; e += (int64_t)gridDim.x * 256)
-            kmax[e] = 0;
-        grid.sync();
-        for (int bid = blockIdx.x; bid < nitems; bid += gridDim.x)
-            kmax_item(ajobs, aitems, na, bjobs, bitems, A, B, kmax, kscales, step, bid);
-        grid.sync();
+    if (a.kmax) {
+        slice_walk<true>(a, GW, (int)blockIdx.x, (int)gridDim.x);
+        cooperative_groups::this_grid().sync();
     }
-    for (int bid = blockIdx.x; bid < nitems; bid += gridDim.x) {
-        if (bid < na) slice_item(ajobs, aitems[bid], A, ap, ae, 1.0, step, err, kmax, kscales, 0);
-        else slice_item(bjobs, bitems[bid - na], B, bp, be, alpha, step, err, kmax, kscales, 1);
+    slice_walk<false>(a, GW, (int)blockIdx.x, (int)gridDim.x);
+}
+__global__ void __launch_bounds__(32 * kSliceWarps) k_slice_cluster(SliceArgs a, int GW, const int *skip) {
+    if (skip && *skip) return;
+    if (a.kmax) {
+        slice_walk<true>(a, GW, (int)blockIdx.x, (int)gridDim.x);
+        cooperative_groups::this_cluster().sync();
     }
+    slice_walk<false>(a, GW, (int)blockIdx.x, (int)gridDim.x);
+}
+__global__ void __launch_bounds__(32 * kSliceWarps) k_slice_max(SliceArgs a, int GW, const int *skip) {
+    if (skip && *skip) return;
+    slice_walk<true>(a, GW, (int)blockIdx.x, (int)gridDim.x);
+}
+__global__ void __launch_bounds__(32 * kSliceWarps) k_slice_put(SliceArgs a, int GW, const int *skip) {
+    if (skip && *skip) return;
+    slice_walk<false>(a, GW, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // -------------------------------------------------------- tensor-core GEMM
@@ -500,8 +545,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const TcTile *__restric
                                                     const __half *__restrict__ Apl, const __half *__restrict__ Bpl,
                                                     const int *__restrict__ Aexp, const int *__restrict__ Bexp,
                                                     double2 *__restrict__ C, const int *skip, int *err, int step,
-                                                    int write_inactive, long long wait_limit, int no_copies) {
+                                                    int write_inactive, long long wait_limit, int no_copies,
+                                                    int *kmax, int nkmax) {
     if (skip && *skip) return;
+    // the balancing maxima are used up: zero for the next call's slicing
+    for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < nkmax; i += (int)(gridDim.x * blockDim.x))
+        kmax[i] = 0;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + SMEM_ALIGN - 1) & ~(uintptr_t)(SMEM_ALIGN - 1));
     uint8_t *sA = smem;
@@ -1122,21 +1171,56 @@ void plan_mixed(GemmPlan &g) {
     g.d_bitems = upload_vec(bitems);
 }
 
-// Grid of the cooperative slicing launch on a device: every CTA resident at
-// once (0: cooperative launches unavailable).  Checked once per device.
-static int slice_coop_grid(int device) {
+// Per device: the cooperative slicing grid (every CTA resident at once; 0:
+// cooperative launches unavailable) and the largest slicing cluster (16, else 8).
+struct SliceLimits {
+    int grid = 0, cluster = 0;
+};
+static SliceLimits slice_limits(int device) {
     static std::mutex mu;
-    static int grid[kMaxDevices] = {};  // 0 unknown, > 0 the grid, -1 unavailable
-    if (device < 0 || device >= kMaxDevices) return 0;
+    static SliceLimits lim[kMaxDevices];
+    KV_REQUIRE(device >= 0 && device < kMaxDevices, KV_EINVAL, "device index out of range");
     std::lock_guard<std::mutex> lk(mu);
-    if (grid[device] == 0) {
+    SliceLimits &l = lim[device];
+    if (l.cluster == 0) {
         int coop = 0, per_sm = 0, sms = 0;
         KV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
         KV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        KV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_slice_coop, 256, 0));
-        grid[device] = (coop && per_sm > 0) ? per_sm * sms : -1;
+        KV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_slice_coop, 32 * kSliceWarps, 0));
+        l.grid = coop ? per_sm * sms : 0;
+        int n = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(32 * kSliceWarps);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 16;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const bool ok = cudaFuncSetAttribute((const void *)k_slice_cluster,
+                                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, (const void *)k_slice_cluster, &cfg) == cudaSuccess && n > 0;
+        if (!ok) (void)cudaGetLastError();
+        l.cluster = ok ? 16 : 8;
     }
-    return std::max(0, grid[device]);
+    return l;
+}
+
+// The context's balancing maxima, at least n of them, all zero between calls:
+// k_gemm_tc clears what its slicing filled.  Freed with the context.
+static int *context_kmax(int64_t n) {
+    Context &c = ctx();
+    if (c.kmax_n < n) {
+        if (c.kmax) KV_CUDA(cudaFreeAsync(c.kmax, c.stream));
+        c.kmax = nullptr;
+        c.kmax_n = 0;
+        const int64_t want = std::max<int64_t>(2 * n, 4096);
+        KV_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&c.kmax), want * sizeof(int), c.stream));
+        KV_CUDA(cudaMemsetAsync(c.kmax, 0, want * sizeof(int), c.stream));
+        c.kmax_n = want;
+    }
+    return c.kmax;
 }
 
 void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, double2 *C, double alpha,
@@ -1150,45 +1234,61 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
     DevBuf ae(std::max<int64_t>(1, p.a_exps) * sizeof(int)), be(std::max<int64_t>(1, p.b_exps) * sizeof(int));
     int n = 0;
     const bool bal = p.balance_k && p.k_scales > 0 && p.na_items > 0 && p.nb_items > 0;
-    DevBuf kmax(bal ? 2 * (size_t)p.k_scales * sizeof(unsigned long long) : 8);
-    unsigned long long *km = bal ? kmax.as<unsigned long long>() : nullptr;
-    int na = p.na_items, nb = p.nb_items;
-    const int grid = slice_coop_grid(c.device);
-    if (na + nb > 0 && &c == &main_ctx() && grid > 0) {
-        // one cooperative launch (zero, maxima, slicing); only on the main
-        // context's stream, whose kernels never overlap, so its grid barrier
-        // waits on no other launch of this library
-        const SliceJob *aj = p.d_ajobs.as<SliceJob>(), *bj = p.d_bjobs.as<SliceJob>();
-        const int2 *ai = p.d_aitems.as<int2>(), *bi = p.d_bitems.as<int2>();
-        __half *aph = ap.as<__half>(), *bph = bp.as<__half>();
-        int *aex = ae.as<int>(), *bex = be.as<int>();
-        int64_t ks = p.k_scales;
-        void *args[] = {&aj, &ai, &na, &bj, &bi, &nb, &A, &B, &aph, &bph, &aex, &bex, &alpha, &skip, &step, &err, &km,
-                        &ks};
-        KV_CUDA(cudaLaunchCooperativeKernel((const void *)k_slice_coop, dim3((unsigned)std::min(na + nb, grid)),
-                                            dim3(256), args, 0, c.stream));
-        ++n;
-    } else if (na + nb > 0) {
-        if (bal) {
-            KV_CUDA(cudaMemsetAsync(kmax.p, 0, 2 * (size_t)p.k_scales * sizeof(unsigned long long), c.stream));
-            k_kmax<<<(unsigned)(na + nb), 256, 0, c.stream>>>(p.d_ajobs.as<SliceJob>(), p.d_aitems.as<int2>(), na,
-                                                              p.d_bjobs.as<SliceJob>(), p.d_bitems.as<int2>(), A, B,
-                                                              km, p.k_scales, skip, step);
+    const int nkmax = bal ? (int)(2 * p.k_scales) : 0;
+    SliceArgs a{p.d_ajobs.as<SliceJob>(), p.d_bjobs.as<SliceJob>(), p.d_aitems.as<int2>(), p.d_bitems.as<int2>(),
+                p.na_items, p.nb_items, A, B, ap.as<__half>(), bp.as<__half>(), ae.as<int>(), be.as<int>(), alpha, step,
+                err, bal ? context_kmax(nkmax) : nullptr, p.k_scales};
+    const int items = p.na_items + p.nb_items;
+    if (items > 0) {
+        // two K steps of 8 a warp where the longest K allows
+        int GW = 1;
+        while (GW < kSliceWarps && GW * 16 < p.max_k) GW *= 2;
+        const int per = kSliceWarps / GW, ctas = (items + per - 1) / per;
+        const SliceLimits lim = slice_limits(c.device);
+        const bool main = &c == &main_ctx();
+        // Little work: one cluster (its barrier is cheaper than a grid's: 8.8
+        // against 12.5 us at D = 32), at most two rounds of four steps a warp, six
+        // on a worker stream where it also saves a launch; more: the whole
+        // chip, on the main stream in one cooperative launch (that stream's
+        // kernels never overlap, so its grid barrier waits on no other launch)
+        const int64_t rounds = (int64_t)((ctas + lim.cluster - 1) / lim.cluster) * ((p.max_k + 32 * GW - 1) / (32 * GW));
+        if (!a.kmax) {
+            k_slice_put<<<(unsigned)ctas, 32 * kSliceWarps, 0, c.stream>>>(a, GW, skip);
             KV_CUDA(cudaGetLastError());
             ++n;
+        } else if (rounds <= (main ? 2 : 6)) {
+            int size = 1;
+            while (size < lim.cluster && size < ctas) size *= 2;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)size);
+            cfg.blockDim = dim3(32 * kSliceWarps);
+            cfg.stream = c.stream;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = (unsigned)size;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            KV_CUDA(cudaLaunchKernelEx(&cfg, k_slice_cluster, a, GW, skip));
+            ++n;
+        } else if (main && lim.grid > 0) {
+            void *args[] = {&a, &GW, &skip};
+            KV_CUDA(cudaLaunchCooperativeKernel((const void *)k_slice_coop, dim3((unsigned)std::min(ctas, lim.grid)),
+                                                dim3(32 * kSliceWarps), args, 0, c.stream));
+            ++n;
+        } else {
+            k_slice_max<<<(unsigned)ctas, 32 * kSliceWarps, 0, c.stream>>>(a, GW, skip);
+            k_slice_put<<<(unsigned)ctas, 32 * kSliceWarps, 0, c.stream>>>(a, GW, skip);
+            KV_CUDA(cudaGetLastError());
+            n += 2;
         }
-        k_slice_ab<<<(unsigned)(na + nb), 256, 0, c.stream>>>(
-            p.d_ajobs.as<SliceJob>(), p.d_aitems.as<int2>(), na, p.d_bjobs.as<SliceJob>(), p.d_bitems.as<int2>(), A, B,
-            ap.as<__half>(), bp.as<__half>(), ae.as<int>(), be.as<int>(), alpha, skip, step, err, km, p.k_scales);
-        KV_CUDA(cudaGetLastError());
-        ++n;
     }
     // persistent: one CTA per SM at most (the kernel holds all of an SM's tensor memory)
     const int ntiles = p.tc_tiles;
     k_gemm_tc<<<(unsigned)std::min(ntiles, c.num_sms), NTHREADS, SMEM_BYTES, c.stream>>>(
-        p.d_tctiles.as<TcTile>(), ntiles, p.d_xsegs.as<SegX>(), p.d_maps.as<int2>(), p.d_pairs.as<TcPair>(), ap.as<__half>(), bp.as<__half>(), ae.as<int>(),
-        be.as<int>(), C, skip, err, step, p.write_inactive ? 1 : 0, g_stall_test ? (1ll << 10) : WAIT_LIMIT,
-        g_stall_test);
+        p.d_tctiles.as<TcTile>(), ntiles, p.d_xsegs.as<SegX>(), p.d_maps.as<int2>(), p.d_pairs.as<TcPair>(),
+        ap.as<__half>(), bp.as<__half>(), ae.as<int>(), be.as<int>(), C, skip, err, step, p.write_inactive ? 1 : 0,
+        g_stall_test ? (1ll << 10) : WAIT_LIMIT, g_stall_test, a.kmax, nkmax);
     KV_CUDA(cudaGetLastError());
     counted(n + 1);
     // the slices are freed stream-ordered after the GEMM
