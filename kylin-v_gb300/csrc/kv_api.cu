@@ -126,6 +126,9 @@ void context_close(Context &c) {
     if (c.kmax) cudaFreeAsync(c.kmax, c.stream);
     c.kmax = nullptr;
     c.kmax_n = 0;
+    if (c.slices) cudaFreeAsync(c.slices, c.stream);
+    c.slices = nullptr;
+    c.slices_n = 0;
     KV_CUDA(cudaStreamSynchronize(c.stream));
     KV_CUDA(cudaStreamDestroy(c.stream));
     c.stream = nullptr;

@@ -44,13 +44,10 @@ void DevBuf::release() {
     }
 }
 
-void upload_bytes(void *dst, const void *src, size_t n) {
+// n bytes (at most a chunk) of the staging ring, free for the caller until its
+// copy has been issued
+static char *ring_reserve(size_t n) {
     auto &c = ctx();
-    if (!c.ring || n > Context::kRingChunk) {
-        KV_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, c.stream));
-        KV_CUDA(cudaStreamSynchronize(c.stream));  // pageable source: keep the copy safe
-        return;
-    }
     if (c.ring_used + n > Context::kRingChunk) {
         // leave the chunk: fence its copies, move on, wait for the next chunk's old copies
         KV_CUDA(cudaEventRecord(c.ring_ev[c.ring_cur], c.stream));
@@ -61,9 +58,36 @@ void upload_bytes(void *dst, const void *src, size_t n) {
         c.ring_live[c.ring_cur] = false;
     }
     char *stage = c.ring + (size_t)c.ring_cur * Context::kRingChunk + c.ring_used;
-    std::memcpy(stage, src, n);
     c.ring_used += (n + 255) & ~size_t(255);
+    return stage;
+}
+
+void upload_bytes(void *dst, const void *src, size_t n) {
+    auto &c = ctx();
+    if (!c.ring || n > Context::kRingChunk) {
+        KV_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, c.stream));
+        KV_CUDA(cudaStreamSynchronize(c.stream));  // pageable source: keep the copy safe
+        return;
+    }
+    char *stage = ring_reserve(n);
+    std::memcpy(stage, src, n);
     KV_CUDA(cudaMemcpyAsync(dst, stage, n, cudaMemcpyHostToDevice, c.stream));
+}
+
+DevBuf UploadPack::upload() {
+    DevBuf b(std::max<size_t>(1, total));
+    for (auto &x : parts) x.dst->p = b.as<char>() + x.off;
+    if (total == 0) return b;
+    if (!ctx().ring || total > Context::kRingChunk) {
+        for (auto &x : parts)
+            if (x.n) upload_bytes(b.as<char>() + x.off, x.src, x.n);
+        return b;
+    }
+    char *stage = ring_reserve(total);
+    for (auto &x : parts)
+        if (x.n) std::memcpy(stage + x.off, x.src, x.n);
+    KV_CUDA(cudaMemcpyAsync(b.p, stage, total, cudaMemcpyHostToDevice, ctx().stream));
+    return b;
 }
 
 void Meta::layout() {
@@ -1003,8 +1027,10 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     const size_t cb = mixed ? sizeof(float2) : sizeof(double2);
     DevBuf T(std::max<int64_t>(1, P.t_elems) * sizeof(double2));
     DevBuf Us(std::max<int64_t>(1, P.t_elems) * cb);
-    DevBuf S(std::max<int64_t>(1, P.s_elems) * sizeof(double));
-    DevBuf status(std::max<size_t>(1, 2 * P.secs.size()) * sizeof(int));  // sweeps, then QR ranks
+    // singular values, then sweeps and QR ranks per sector: one buffer, read back at once
+    const size_t s_bytes = (size_t)P.s_elems * sizeof(double), st_bytes = 2 * P.secs.size() * sizeof(int);
+    DevBuf S(std::max<size_t>(16, s_bytes + st_bytes));
+    DevSpan status{S.as<char>() + s_bytes};
     svd_gather(P, A.data(), T.as<double2>());
     bool qr_ranks = false;
     if (mixed) {
@@ -1040,11 +1066,14 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     }
     std::vector<double> sv(P.s_elems);
     std::vector<int> st(2 * P.secs.size());
-    if (P.s_elems)
-        KV_CUDA(cudaMemcpyAsync(sv.data(), S.p, P.s_elems * sizeof(double), cudaMemcpyDeviceToHost, ctx().stream));
-    if (!st.empty())
-        KV_CUDA(cudaMemcpyAsync(st.data(), status.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
-    KV_CUDA(cudaStreamSynchronize(ctx().stream));
+    {
+        std::vector<char> back(s_bytes + st_bytes);
+        if (!back.empty())
+            KV_CUDA(cudaMemcpyAsync(back.data(), S.p, back.size(), cudaMemcpyDeviceToHost, ctx().stream));
+        KV_CUDA(cudaStreamSynchronize(ctx().stream));
+        if (s_bytes) std::memcpy(sv.data(), back.data(), s_bytes);
+        if (st_bytes) std::memcpy(st.data(), back.data() + s_bytes, st_bytes);
+    }
     {
         auto &c = ctx();
         for (size_t i = 0; i < P.secs.size(); ++i) {
@@ -1129,7 +1158,7 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     std::vector<int> kc(nsec, 0);  // columns rebuilt per sector
     std::vector<SvdPolish> pol;
     std::vector<int> pol_of_sector(nsec, -1);
-    DevBuf X, Gm, Wb, cst, cdiag;
+    DevBuf X, Gm, Wb, cfail;
     // The mixed rebuild sums over k in order: the last bit of its result decides,
     // through the next FP32 SVD's cut-offs, which noise-level states a one-site
     // sweep keeps (populations of D = 64 chains move by up to 7e-8 a step with
@@ -1156,12 +1185,12 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
                 item_row0.push_back(r0);
             }
         launch_gemm_fp64(gram, X.as<double2>(), X.as<double2>(), Gm.as<double2>(), 1.0, nullptr);
-        svd_chol(dp, (int)pl_list.size(), Gm.as<double2>(), cst.as<int>(), cdiag.as<double>(), shift);
+        svd_chol(dp, (int)pl_list.size(), Gm.as<double2>(), cfail.as<double2>(), shift);
         svd_trsm(dp, item_pol, item_row0, Gm.as<double2>(), X.as<double2>(), kmax);
     };
     if (mixed) {
         const double s_cut = out.kept_s.empty() ? 0.0 : out.kept_s.back();
-        int64_t x_elems = 0, g_elems = 0, w_elems = 0;
+        int64_t x_elems = 0, g_elems = 0, w_elems = 0, n_elems = 0;
         for (int s_ = 0; s_ < nsec; ++s_) {
             const SvdSector &sc = P.secs[s_];
             const int ns = std::min(sc.m, sc.n);
@@ -1172,7 +1201,8 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
             const int xr = side == 0 ? sc.m : sc.n;  // rows of the kept factor
             const int wr = side == 0 ? sc.n : sc.m;  // rows of the other side's vectors
             pol_of_sector[s_] = (int)pol.size();
-            pol.push_back({x_elems, g_elems, w_elems, s_, xr, k, k});
+            pol.push_back({x_elems, g_elems, w_elems, s_, xr, k, k, n_elems});
+            n_elems += k;
             x_elems += (int64_t)xr * k;
             g_elems += (int64_t)k * k;
             w_elems += (int64_t)wr * k;
@@ -1181,9 +1211,9 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
         X = DevBuf(std::max<int64_t>(1, x_elems) * sizeof(double2));
         Gm = DevBuf(std::max<int64_t>(1, g_elems) * sizeof(double2));
         Wb = DevBuf(std::max<int64_t>(1, w_elems) * sizeof(double2));
-        cst = DevBuf(std::max<size_t>(1, pol.size()) * sizeof(int));
-        cdiag = DevBuf(std::max<size_t>(1, pol.size()) * sizeof(double));
-        KV_CUDA(cudaMemsetAsync(cst.p, 0, std::max<size_t>(1, pol.size()) * sizeof(int), ctx().stream));
+        cfail = DevBuf(std::max<size_t>(1, pol.size()) * sizeof(double2));
+        KV_CUDA(cudaMemsetAsync(cfail.p, 0, std::max<size_t>(1, pol.size()) * sizeof(double2), ctx().stream));
+        DevBuf norms(std::max<int64_t>(1, n_elems) * sizeof(double));
         svd_extract(dpol, (int)pol.size(), P, Us.as<float2>(), S.as<double>(), Wb.as<double2>());
         // X = A_s W (L->R, K = n) or A_s^H W (R->L, K = m), A_s from T:
         // A_s[i, j] = T[i + j p] (T = A_s) or conj(T[j + i p]) (T = A_s^H)
@@ -1202,18 +1232,16 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
         // refined singular values: x_j = A w_j / s~_j, so s_j = s~_j |x_j|.  W's
         // FP32 error enters |A w_j| only at second order (the columns of X are
         // orthogonal to that order), which is what the truncation needs.
-        svd_col_norm2(dpol, (int)pol.size(), X.as<double2>(), Gm.as<double2>());
-        std::vector<std::vector<double2>> diag(pol.size());
-        for (size_t i = 0; i < pol.size(); ++i) {
-            diag[i].resize(pol[i].k);
-            KV_CUDA(cudaMemcpyAsync(diag[i].data(), Gm.as<double2>() + pol[i].g_off, pol[i].k * sizeof(double2),
-                                    cudaMemcpyDeviceToHost, ctx().stream));
-        }
+        svd_col_norm2(dpol, (int)pol.size(), X.as<double2>(), norms.as<double>());
+        std::vector<double> n2(n_elems);
+        if (n_elems)
+            KV_CUDA(cudaMemcpyAsync(n2.data(), norms.p, n_elems * sizeof(double), cudaMemcpyDeviceToHost,
+                                    ctx().stream));
         KV_CUDA(cudaStreamSynchronize(ctx().stream));
         std::vector<double> svr = sv;
         for (size_t i = 0; i < pol.size(); ++i) {
             const SvdSector &sc = P.secs[pol[i].sector];
-            for (int j = 0; j < pol[i].k; ++j) svr[sc.s_off + j] = sv[sc.s_off + j] * std::sqrt(diag[i][j].x);
+            for (int j = 0; j < pol[i].k; ++j) svr[sc.s_off + j] = sv[sc.s_off + j] * std::sqrt(n2[pol[i].n_off + j]);
         }
         out.kept_s.clear();
         kfin = truncate(svr, nullptr, nullptr);
@@ -1352,9 +1380,8 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
             sa_subtract(X.as<double2>(), Pb.as<double2>(), x_elems);
         }
         Gm = DevBuf(std::max<int64_t>(1, g_elems) * sizeof(double2));
-        cst = DevBuf(std::max<size_t>(1, pl.size()) * sizeof(int));
-        cdiag = DevBuf(std::max<size_t>(1, pl.size()) * sizeof(double));
-        KV_CUDA(cudaMemsetAsync(cst.p, 0, std::max<size_t>(1, pl.size()) * sizeof(int), ctx().stream));
+        cfail = DevBuf(std::max<size_t>(1, pl.size()) * sizeof(double2));
+        KV_CUDA(cudaMemsetAsync(cfail.p, 0, std::max<size_t>(1, pl.size()) * sizeof(double2), ctx().stream));
         DevBuf dpl = upload_vec(pl);
         polish_pass(pl, dpl, 0.0);
         polish_pass(pl, dpl, 0.0);
@@ -1429,20 +1456,17 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
     }
     svd_scatter_dense(du, side == 0 ? X.as<double2>() : Y.as<double2>(), out.U->data());
     svd_scatter_dense(dv, side == 0 ? Y.as<double2>() : X.as<double2>(), out.V->data());
-    std::vector<int> ch(pol.size());
-    std::vector<double> chd(pol.size());
+    std::vector<double2> ch(pol.size());
     if (!ch.empty()) {
-        KV_CUDA(cudaMemcpyAsync(ch.data(), cst.p, ch.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
-        KV_CUDA(cudaMemcpyAsync(chd.data(), cdiag.p, chd.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                                ctx().stream));
+        KV_CUDA(cudaMemcpyAsync(ch.data(), cfail.p, ch.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx().stream));
         KV_CUDA(cudaStreamSynchronize(ctx().stream));
         for (size_t i = 0; i < ch.size(); ++i) {
-            if (ch[i] == 0) continue;
+            if (ch[i].x == 0.0) continue;
             const SvdSector &sc = P.secs[pol[i].sector];
             std::string msg = "Cholesky re-orthonormalisation failed: sector m=" + std::to_string(sc.m) +
                               " n=" + std::to_string(sc.n) + " kept=" + std::to_string(pol[i].k) +
                               " transposed=" + std::to_string(sc.transposed) + " l2r=" + std::to_string(l2r) +
-                              " pivot=" + std::to_string(ch[i] - 1) + " value=" + std::to_string(chd[i]) + " s=[";
+                              " pivot=" + std::to_string((int)ch[i].x - 1) + " value=" + std::to_string(ch[i].y) + " s=[";
             for (int j = 0; j < std::min(sc.q, 12); ++j) msg += std::to_string(sv[sc.s_off + j]) + " ";
             throw Error(KV_ENONFINITE, msg + "]");
         }

@@ -87,6 +87,9 @@ struct Context {
     // balancing maxima of the tensor-core GEMM's slicing (kv_tc.cu), zero between calls
     int *kmax = nullptr;
     int64_t kmax_n = 0;
+    // its sliced panels, up to a bound (kv_tc.cu)
+    char *slices = nullptr;
+    int64_t slices_n = 0;
     // charge sectors through the mixed/FP64 SVD: count, columns, rank
     // reached by the QR reduction (else min(rows, columns)), Jacobi sweeps
     struct SvdStats {
@@ -146,6 +149,29 @@ DevBuf upload_vec(const std::vector<T> &v) {
     if (!v.empty()) upload_bytes(b.p, v.data(), v.size() * sizeof(T));
     return b;
 }
+
+// A device array inside some buffer.
+struct DevSpan {
+    char *p = nullptr;
+    template <class T> T *as() const { return reinterpret_cast<T *>(p); }
+};
+
+// Several host arrays uploaded with one allocation and one copy.
+struct UploadPack {
+    struct Part {
+        const void *src;
+        size_t n, off;
+        DevSpan *dst;
+    };
+    std::vector<Part> parts;
+    size_t total = 0;
+    template <class T>
+    void add(DevSpan &d, const std::vector<T> &v) {
+        parts.push_back({v.data(), v.size() * sizeof(T), total, &d});
+        total += (v.size() * sizeof(T) + 255) & ~size_t(255);
+    }
+    DevBuf upload();  // the buffer holding them all; the spans point into it
+};
 
 // ------------------------------------------------------------ block tensors
 struct BlockMeta {
@@ -350,7 +376,8 @@ void fp64_tiles(GemmPlan &g);  // one tile per output block -> tiles of about eq
 struct GemmPlan {
     std::vector<GemmTile> tiles;
     std::vector<GemmSeg> segs;
-    DevBuf d_tiles, d_segs;
+    DevBuf d_lists;  // the arrays below
+    DevSpan d_tiles, d_segs;
     double ref_flops = 0.0;  // sum of 8*M*N*K over the reference's zgemm pairs
     int max_k = 0;
     int tile_m = 0, tile_n = 0;
@@ -369,15 +396,17 @@ struct GemmPlan {
     int tc_tiles = 0, na_items = 0, nb_items = 0;
     int64_t a_planes = 0, b_planes = 0, a_exps = 0, b_exps = 0;
     // items: (job, first of 8 rows) per slicing CTA
-    DevBuf d_tctiles, d_xsegs, d_maps, d_pairs, d_ajobs, d_bjobs, d_aitems, d_bitems;
+    DevSpan d_tctiles, d_xsegs, d_maps, d_pairs, d_ajobs, d_bjobs, d_aitems, d_bitems;
     void upload() {
         if (tile_m == kMixedTileM && tile_n == kMixedTileN) {
             plan_mixed(*this);
             return;
         }
         if (tile_m == kFp64Block) fp64_tiles(*this);
-        d_tiles = upload_vec(tiles);
-        d_segs = upload_vec(segs);
+        UploadPack u;
+        u.add(d_tiles, tiles);
+        u.add(d_segs, segs);
+        d_lists = u.upload();
     }
 };
 
@@ -406,12 +435,19 @@ struct MixPlan {
     std::vector<MixJob> jobs;
     std::vector<MixItem> items;
     int chunk = kMixChunk;
-    DevBuf d_terms, d_jobs, d_items;
+    DevBuf d_lists;  // the arrays below
+    DevSpan d_terms, d_jobs, d_items;
     bool write_inactive = true;  // as GemmPlan::write_inactive, per output block
     // profiling: algorithmic bytes of a launch at Lanczos step s (s clamped to
     // the last entry step), filled on first use
     mutable std::vector<double> prof_bytes;
-    void upload() { d_terms = upload_vec(terms); d_jobs = upload_vec(jobs); d_items = upload_vec(items); }
+    void upload() {
+        UploadPack u;
+        u.add(d_terms, terms);
+        u.add(d_jobs, jobs);
+        u.add(d_items, items);
+        d_lists = u.upload();
+    }
 };
 
 // Launch step meaning "every segment / term is active".

@@ -63,33 +63,10 @@ struct Arena {
     }
 };
 
-// DevBufs pointing into the arena.  Every view is cleared when the set goes
-// out of scope -- on return and when an exception leaves the scope -- so a
-// plan's destructor never hands an arena address to cudaFreeAsync.
-struct Views {
-    std::vector<DevBuf *> held;
-    Views() = default;
-    Views(const Views &) = delete;
-    Views &operator=(const Views &) = delete;
-    void view(DevBuf &d, void *p, size_t n) {
-        held.push_back(&d);
-        d.p = p;
-        d.bytes = n;
-    }
-    ~Views() {
-        for (DevBuf *d : held) {
-            d->p = nullptr;
-            d->bytes = 0;
-        }
-    }
-};
-
 template <class T>
-void put(Arena &ar, Views &vw, DevBuf &d, const std::vector<T> &v) {
-    const size_t n = std::max<size_t>(1, v.size()) * sizeof(T);
-    void *p = ar.take(n);
-    vw.view(d, p, n);
-    if (!v.empty()) upload_bytes(p, v.data(), v.size() * sizeof(T));
+void put(Arena &ar, DevSpan &d, const std::vector<T> &v) {
+    d.p = static_cast<char *>(ar.take(std::max<size_t>(1, v.size()) * sizeof(T)));
+    if (!v.empty()) upload_bytes(d.p, v.data(), v.size() * sizeof(T));
 }
 
 // product<> of two arena-resident operands into an arena-resident output
@@ -106,9 +83,8 @@ void arena_product(Arena &ar, const Meta &A, const double2 *a, const Meta &B, co
         t.tm = (short)std::min(16, t.M);
         t.tn = (short)std::min(16, t.N);
     }
-    Views vw;
-    put(ar, vw, P.gemm.d_tiles, P.gemm.tiles);
-    put(ar, vw, P.gemm.d_segs, P.gemm.segs);
+    put(ar, P.gemm.d_tiles, P.gemm.tiles);
+    put(ar, P.gemm.d_segs, P.gemm.segs);
     launch_gemm_fp64(P.gemm, a, b, c, 1.0, nullptr);
 }
 
@@ -139,10 +115,9 @@ cplx expectation_noalloc(const std::vector<DTensor *> &bra, const std::vector<DT
         MixPlanFull M = plan_mix(t1, w[i]->meta, 1, nullptr, false, kMixChunkCoarse);
         double2 *t2_d = static_cast<double2 *>(ar.take(std::max<int64_t>(1, M.out.nelem) * sizeof(double2)));
         {
-            Views vw;
-            put(ar, vw, M.mix.d_terms, M.mix.terms);
-            put(ar, vw, M.mix.d_jobs, M.mix.jobs);
-            put(ar, vw, M.mix.d_items, M.mix.items);
+            put(ar, M.mix.d_terms, M.mix.terms);
+            put(ar, M.mix.d_jobs, M.mix.jobs);
+            put(ar, M.mix.d_items, M.mix.items);
             launch_mix(M.mix, t1_d, w[i]->data(), t2_d, nullptr);
         }
         Meta next;

@@ -920,8 +920,8 @@ __global__ void k_svd_extract(const SvdPolish *__restrict__ pol, const SvdSector
 }
 
 // Squared norms of the columns of each polish factor X (rows x k, row stride
-// ldx), written as G[g_off + j].x: one CTA per factor, one warp per column.
-__global__ void k_col_norm2(const SvdPolish *__restrict__ pol, const double2 *__restrict__ X, double2 *__restrict__ G) {
+// ldx), written as norms[n_off + j]: one CTA per factor, one warp per column.
+__global__ void k_col_norm2(const SvdPolish *__restrict__ pol, const double2 *__restrict__ X, double *__restrict__ norms) {
     const SvdPolish d = pol[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int j = warp; j < d.k; j += nw) {
@@ -931,14 +931,13 @@ __global__ void k_col_norm2(const SvdPolish *__restrict__ pol, const double2 *__
             a += v.x * v.x + v.y * v.y;
         }
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
-        if (lane == 0) G[d.g_off + j] = make_double2(a, 0.0);
+        if (lane == 0) norms[d.n_off + j] = a;
     }
 }
 
 // In place: G (k x k, row-major, Hermitian positive definite) -> upper R with
 // G = R^H R (lower triangle left as is).  One CTA per sector, column-wise.
-__global__ void k_chol(const SvdPolish *__restrict__ pol, double2 *__restrict__ G, int *status, double *diagv,
-                       double shift) {
+__global__ void k_chol(const SvdPolish *__restrict__ pol, double2 *__restrict__ G, double2 *fail, double shift) {
     const SvdPolish d = pol[blockIdx.x];
     const int k = d.k;
     double2 *g = G + d.g_off;
@@ -953,10 +952,8 @@ __global__ void k_chol(const SvdPolish *__restrict__ pol, double2 *__restrict__ 
     for (int j = 0; j < k; ++j) {
         if (threadIdx.x == 0) {
             double r = g[(int64_t)j * k + j].x;
-            if ((!(r > 0.0) || !isfinite(r)) && status[blockIdx.x] == 0) {
-                status[blockIdx.x] = j + 1;  // first failing pivot (1-based) for the error report
-                diagv[blockIdx.x] = r;
-            }
+            // the first failing pivot (1-based) and its value, for the error report
+            if ((!(r > 0.0) || !isfinite(r)) && fail[blockIdx.x].x == 0.0) fail[blockIdx.x] = make_double2(j + 1, r);
             if (!(r > 0.0) || !isfinite(r)) r = 1e-300;
             diag = sqrt(r);
             g[(int64_t)j * k + j] = make_double2(diag, 0.0);
@@ -1299,16 +1296,16 @@ void svd_extract(const DevBuf &pol, int npol, const SvdPlan &p, const float2 *Us
     KV_CUDA(cudaGetLastError());
 }
 
-void svd_col_norm2(const DevBuf &pol, int npol, const double2 *X, double2 *G) {
+void svd_col_norm2(const DevBuf &pol, int npol, const double2 *X, double *norms) {
     if (npol == 0) return;
-    k_col_norm2<<<npol, 256, 0, ctx().stream>>>(pol.as<SvdPolish>(), X, G);
+    k_col_norm2<<<npol, 256, 0, ctx().stream>>>(pol.as<SvdPolish>(), X, norms);
     counted();
     KV_CUDA(cudaGetLastError());
 }
 
-void svd_chol(const DevBuf &pol, int npol, double2 *G, int *status, double *diagv, double shift) {
+void svd_chol(const DevBuf &pol, int npol, double2 *G, double2 *fail, double shift) {
     if (npol == 0) return;
-    k_chol<<<npol, 256, 0, ctx().stream>>>(pol.as<SvdPolish>(), G, status, diagv, shift);
+    k_chol<<<npol, 256, 0, ctx().stream>>>(pol.as<SvdPolish>(), G, fail, shift);
     counted();
     KV_CUDA(cudaGetLastError());
 }
@@ -1320,7 +1317,11 @@ void svd_trsm(const DevBuf &pol, const std::vector<int> &item_pol, const std::ve
     constexpr int kTrsmSmemMax = 200 * 1024;
     KV_REQUIRE(smem <= kTrsmSmemMax, KV_EINVAL, "SVD polish: kept dimension of one sector too large");
     trsm_smem_raise(ctx().device, kTrsmSmemMax);  // once per device, to the largest size allowed here
-    DevBuf ip = upload_vec(item_pol), ir = upload_vec(item_row0);
+    DevSpan ip, ir;
+    UploadPack u;
+    u.add(ip, item_pol);
+    u.add(ir, item_row0);
+    DevBuf items = u.upload();
     k_trsm_rows<<<(unsigned)item_pol.size(), 32 * kTrsmRows, smem, ctx().stream>>>(pol.as<SvdPolish>(), ip.as<int>(),
                                                                                   ir.as<int>(), G, X);
     counted();

@@ -44,8 +44,14 @@ struct SvdPlan {
     std::vector<SvdGather> gathers;
     int64_t t_elems = 0, s_elems = 0;
     int max_q = 0;
-    DevBuf d_secs, d_gathers;
-    void upload() { d_secs = upload_vec(secs); d_gathers = upload_vec(gathers); }
+    DevBuf d_lists;  // the arrays below
+    DevSpan d_secs, d_gathers;
+    void upload() {
+        UploadPack u;
+        u.add(d_secs, secs);
+        u.add(d_gathers, gathers);
+        d_lists = u.upload();
+    }
 };
 
 // FP64 polish of the kept factor of one sector (mixed mode): W (the FP32
@@ -55,6 +61,7 @@ struct SvdPlan {
 struct SvdPolish {
     int64_t x_off, g_off, w_off;
     int sector, rows, k, ldx;
+    int64_t n_off = 0;  // its columns' norms
 };
 // one output block copied from a dense row-major factor M (ld columns);
 // ctrans: the block is taken from M^H
@@ -87,9 +94,10 @@ bool svd_qrjacobi_f32(const SvdPlan &p, const double2 *T64, float2 *Us, double *
 void svd_extract(const DevBuf &pol, int npol, const SvdPlan &p, const float2 *Us, const double *S, double2 *W);
 // rows of X per triangular-solve CTA (one warp per row)
 constexpr int kTrsmRows = 8;
-// squared column norms of each polish factor X into G[g_off + j].x
-void svd_col_norm2(const DevBuf &pol, int npol, const double2 *X, double2 *G);
-void svd_chol(const DevBuf &pol, int npol, double2 *G, int *status, double *diagv, double shift);
+// squared column norms of each polish factor X into norms[n_off + j]
+void svd_col_norm2(const DevBuf &pol, int npol, const double2 *X, double *norms);
+// fail[i] = (first failing pivot, 1-based, or 0; its value) of factor i
+void svd_chol(const DevBuf &pol, int npol, double2 *G, double2 *fail, double shift);
 void svd_trsm(const DevBuf &pol, const std::vector<int> &item_pol, const std::vector<int> &item_row0,
               const double2 *G, double2 *X, int kmax);
 void svd_scatter_dense(const std::vector<SvdDense> &d, const double2 *M, double2 *out);

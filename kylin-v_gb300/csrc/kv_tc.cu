@@ -1161,14 +1161,16 @@ void plan_mixed(GemmPlan &g) {
     g.tc_tiles = (int)tiles.size();
     g.na_items = (int)aitems.size();
     g.nb_items = (int)bitems.size();
-    g.d_tctiles = upload_vec(tiles);
-    g.d_xsegs = upload_vec(xsegs);
-    g.d_maps = upload_vec(maps);
-    g.d_pairs = upload_vec(pairs);
-    g.d_ajobs = upload_vec(ajobs);
-    g.d_bjobs = upload_vec(bjobs);
-    g.d_aitems = upload_vec(aitems);
-    g.d_bitems = upload_vec(bitems);
+    UploadPack u;
+    u.add(g.d_tctiles, tiles);
+    u.add(g.d_xsegs, xsegs);
+    u.add(g.d_maps, maps);
+    u.add(g.d_pairs, pairs);
+    u.add(g.d_ajobs, ajobs);
+    u.add(g.d_bjobs, bjobs);
+    u.add(g.d_aitems, aitems);
+    u.add(g.d_bitems, bitems);
+    g.d_lists = u.upload();
 }
 
 // Per device: the cooperative slicing grid (every CTA resident at once; 0:
@@ -1223,6 +1225,26 @@ static int *context_kmax(int64_t n) {
     return c.kmax;
 }
 
+// The context's workspace for sliced panels, at least `bytes` of it; null beyond
+// kKeepSlices (such panels are allocated per call).  A context's calls follow
+// one another on its stream, so one workspace serves them all; it is freed with
+// the context.  Four stream-ordered allocations and frees per GEMM were a
+// third of the host's time per call, and contended between worker threads.
+constexpr int64_t kKeepSlices = 64ll << 20;
+static char *context_slices(int64_t bytes) {
+    Context &c = ctx();
+    if (bytes > kKeepSlices) return nullptr;
+    if (c.slices_n < bytes) {
+        if (c.slices) KV_CUDA(cudaFreeAsync(c.slices, c.stream));
+        c.slices = nullptr;
+        c.slices_n = 0;
+        const int64_t want = std::min(kKeepSlices, std::max<int64_t>(2 * bytes, 1 << 20));
+        KV_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&c.slices), (size_t)want, c.stream));
+        c.slices_n = want;
+    }
+    return c.slices;
+}
+
 void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, double2 *C, double alpha,
                        const int *skip, int step) {
     if (p.tiles.empty()) return;
@@ -1230,14 +1252,24 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
                "internal: GEMM plan not prepared for the tensor-core path");
     auto &c = ctx();
     int *err = device_err_word(c.device);
-    DevBuf ap(std::max<int64_t>(1, p.a_planes) * sizeof(__half)), bp(std::max<int64_t>(1, p.b_planes) * sizeof(__half));
-    DevBuf ae(std::max<int64_t>(1, p.a_exps) * sizeof(int)), be(std::max<int64_t>(1, p.b_exps) * sizeof(int));
+    auto up = [](int64_t b) { return (b + 255) & ~(int64_t)255; };
+    const int64_t o_bp = up(p.a_planes * (int64_t)sizeof(__half)), o_ae = o_bp + up(p.b_planes * (int64_t)sizeof(__half)),
+                  o_be = o_ae + up(p.a_exps * (int64_t)sizeof(int)),
+                  bytes = o_be + up(p.b_exps * (int64_t)sizeof(int)) + 256;
+    DevBuf large;  // panels beyond the context's workspace
+    char *ws = context_slices(bytes);
+    if (!ws) {
+        large.alloc((size_t)bytes);
+        ws = large.as<char>();
+    }
+    __half *const aph = reinterpret_cast<__half *>(ws), *const bph = reinterpret_cast<__half *>(ws + o_bp);
+    int *const aex = reinterpret_cast<int *>(ws + o_ae), *const bex = reinterpret_cast<int *>(ws + o_be);
     int n = 0;
     const bool bal = p.balance_k && p.k_scales > 0 && p.na_items > 0 && p.nb_items > 0;
     const int nkmax = bal ? (int)(2 * p.k_scales) : 0;
     SliceArgs a{p.d_ajobs.as<SliceJob>(), p.d_bjobs.as<SliceJob>(), p.d_aitems.as<int2>(), p.d_bitems.as<int2>(),
-                p.na_items, p.nb_items, A, B, ap.as<__half>(), bp.as<__half>(), ae.as<int>(), be.as<int>(), alpha, step,
-                err, bal ? context_kmax(nkmax) : nullptr, p.k_scales};
+                p.na_items, p.nb_items, A, B, aph, bph, aex, bex, alpha, step, err,
+                 bal ? context_kmax(nkmax) : nullptr, p.k_scales};
     const int items = p.na_items + p.nb_items;
     if (items > 0) {
         // two K steps of 8 a warp where the longest K allows
@@ -1287,11 +1319,10 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
     const int ntiles = p.tc_tiles;
     k_gemm_tc<<<(unsigned)std::min(ntiles, c.num_sms), NTHREADS, SMEM_BYTES, c.stream>>>(
         p.d_tctiles.as<TcTile>(), ntiles, p.d_xsegs.as<SegX>(), p.d_maps.as<int2>(), p.d_pairs.as<TcPair>(),
-        ap.as<__half>(), bp.as<__half>(), ae.as<int>(), be.as<int>(), C, skip, err, step, p.write_inactive ? 1 : 0,
-        g_stall_test ? (1ll << 10) : WAIT_LIMIT, g_stall_test, a.kmax, nkmax);
+        aph, bph, aex, bex, C, skip, err, step, p.write_inactive ? 1 : 0, g_stall_test ? (1ll << 10) : WAIT_LIMIT, g_stall_test, a.kmax, nkmax);
     KV_CUDA(cudaGetLastError());
     counted(n + 1);
-    // the slices are freed stream-ordered after the GEMM
+    // large panels are freed stream-ordered after the GEMM
 }
 
 // KV_ETIMEOUT if a tensor-core wait gave up, else KV_ENONFINITE if an operand
