@@ -120,6 +120,37 @@ cudaEvent_t prof_event();
 // reached by a state (launches at iteration k >= that were skipped)
 void prof_resolve(int (*iters_of)(const KrylovState *, void *), void *arg);
 
+// ------------------------------------------------ dependent launches
+// A kernel launched by launch_dependent may start while its predecessor on the
+// stream finishes: it does its set-up (plan lists, tensor memory, barriers) and
+// calls dependency_wait before it touches anything an earlier launch wrote or
+// reads.  Every such kernel calls it on every path, so a launch that has
+// completed implies that all before it have.  allow_dependents lets the
+// successor start once every CTA of this launch has begun.
+#ifdef __CUDACC__
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// cluster: CTAs per cluster (0: none)
+template <class... P, class... A>
+void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, unsigned cluster, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx().stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster ? 2 : 1;
+    KV_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+#endif
+
 // Stream-ordered device buffer (cudaMallocAsync on the library stream).
 struct DevBuf {
     void *p = nullptr;

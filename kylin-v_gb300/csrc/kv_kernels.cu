@@ -50,10 +50,12 @@ __global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ t
                                                   const double2 *__restrict__ B, double2 *__restrict__ C, double alpha,
                                                   const int *skip, int step, int write_inactive, int cover,
                                                   int serial_k) {
-    if (skip && *skip) return;
+    allow_dependents();
     __shared__ GemmSeg sg[kSegBatch];
     __shared__ double2 red[NT];
     const GemmTile t = tiles[blockIdx.x];
+    dependency_wait();
+    if (skip && *skip) return;
     const int tid = threadIdx.x;
     const int tm = t.tm, tn = t.tn, mn = tm * tn, KS = serial_k ? 1 : NT / mn;
     const int ks = tid / mn, m = (tid % mn) / tn, n = tid % tn;
@@ -212,14 +214,16 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
                                                         const double2 *__restrict__ in, const double2 *__restrict__ W,
                                                         double2 *__restrict__ out, const int *skip, int step,
                                                         int write_inactive) {
+    allow_dependents();
     __shared__ MixWarp sm[kMixWarps];
-    if (skip && *skip) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * kMixWarps + warp;
+    const MixItem it = items[min(item, nitems - 1)];
+    const MixJob jb = jobs[it.job];
+    dependency_wait();
+    if (skip && *skip) return;
     if (item >= nitems) return;  // warp-uniform, as every branch on the item below
     MixWarp &mw = sm[warp];
-    const MixItem it = items[item];
-    const MixJob jb = jobs[it.job];
     const int nt_all = jb.term_end - jb.term_begin, nout = jb.so * jb.wr;
     const int64_t e1 = min(jb.count, it.start + chunk);
     bool listed = nt_all <= kMixTerms && nout <= kMixOuts && jb.count < (1ll << 31);
@@ -412,24 +416,22 @@ void launch_gemm_fp64(const GemmPlan &p, const double2 *A, const double2 *B, dou
     const int cover = p.tile_m == kFp64Coarse ? kFp64Coarse : 0;
     const unsigned n = (unsigned)p.tiles.size();
     auto launch = [&](auto kernel, int threads) {
-        kernel<<<n, threads, 0, ctx().stream>>>(p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C, alpha, skip,
-                                                step, p.write_inactive ? 1 : 0, cover, p.serial_k ? 1 : 0);
+        launch_dependent(kernel, n, (unsigned)threads, 0, 0, p.d_tiles.as<GemmTile>(), p.d_segs.as<GemmSeg>(), A, B, C,
+                         alpha, skip, step, p.write_inactive ? 1 : 0, cover, p.serial_k ? 1 : 0);
     };
     if (p.fp64_threads == 32) launch(k_gemm_fp64<32>, 32);
     else if (p.fp64_threads == 64) launch(k_gemm_fp64<64>, 64);
     else launch(k_gemm_fp64<256>, 256);
     counted();
-    KV_CUDA(cudaGetLastError());
 }
 
 void launch_mix(const MixPlan &p, const double2 *in, const double2 *W, double2 *out, const int *skip, int step) {
     if (p.items.empty()) return;
     const int n = (int)p.items.size();
-    k_mix<<<(unsigned)((n + kMixWarps - 1) / kMixWarps), 32 * kMixWarps, 0, ctx().stream>>>(
-        p.d_items.as<MixItem>(), n, p.chunk, p.d_jobs.as<MixJob>(), p.d_terms.as<MixTerm>(), in, W, out, skip, step,
-        p.write_inactive ? 1 : 0);
+    launch_dependent(k_mix, (unsigned)((n + kMixWarps - 1) / kMixWarps), 32 * kMixWarps, 0, 0, p.d_items.as<MixItem>(),
+                     n, p.chunk, p.d_jobs.as<MixJob>(), p.d_terms.as<MixTerm>(), in, W, out, skip, step,
+                     p.write_inactive ? 1 : 0);
     counted();
-    KV_CUDA(cudaGetLastError());
 }
 
 void launch_permute(const double2 *in, double2 *out, const std::vector<int64_t> &desc, int nblocks) {

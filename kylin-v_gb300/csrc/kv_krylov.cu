@@ -118,6 +118,8 @@ __device__ __forceinline__ void raise_stop(int *stop) {
 
 __global__ void __launch_bounds__(KT) k_start(KrylovState *st, const double2 *psi, double2 *v0, int64_t n,
                                               const double2 *parts, int nparts, int *stop) {
+    allow_dependents();
+    dependency_wait();
     const double n2 = reduce_partials(parts, nparts).x;
     __shared__ double s_inv;
     if (threadIdx.x == 0) {
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(kStepGrid) k_lanczos_step(KrylovState *st, int
                                                             int nparts, double tol, int max_iter, int *stop) {
     __shared__ double red[kMaxLocal][16];
     __shared__ double2 out;
+    allow_dependents();
     cooperative_groups::grid_group g = cooperative_groups::this_grid();
     LanczosStep<kStepGrid / 32, cooperative_groups::grid_group> s{g, (int)blockIdx.x, (int)gridDim.x, nparts, red, &out};
     s.run(st, k, hv, vprev, vk, vnext, n_prev, n_k, n_next, P0, P1, tol, max_iter, stop);
@@ -370,6 +373,8 @@ __global__ void __launch_bounds__(NT) k_lanczos_cluster(KrylovState *st, int k, 
                                                                   double tol, int max_iter, int *stop) {
     __shared__ double red[kMaxLocal][16];
     __shared__ double2 out;
+    allow_dependents();
+    dependency_wait();
     cooperative_groups::cluster_group g = cooperative_groups::this_cluster();
     LanczosStep<NT / 32, cooperative_groups::cluster_group> s{g, (int)blockIdx.x, (int)gridDim.x, nparts, red, &out};
     s.run(st, k, hv, vprev, vk, vnext, n_prev, n_k, n_next, P0, P1, tol, max_iter, stop);
@@ -406,6 +411,8 @@ __device__ __forceinline__ int part_exponent(double2 v) {
 
 __global__ void __launch_bounds__(32) k_tridiag_exp(KrylovState *st, int reverse) {
     static_assert(kMaxKrylov <= 32, "one lane per Krylov vector");
+    allow_dependents();
+    dependency_wait();
     const int lane = threadIdx.x;
     const int n = st->iters;
     if (n <= 0) return;
@@ -463,6 +470,8 @@ __global__ void __launch_bounds__(32) k_tridiag_exp(KrylovState *st, int reverse
 
 __global__ void __launch_bounds__(KT) k_combine(const KrylovState *st, double2 *const *V, double2 *out,
                                                 KrylovLens nl) {
+    allow_dependents();
+    dependency_wait();
     const int m = st->iters;
     if (m <= 0) return;
     const int64_t n = nl.n[m - 1];
@@ -489,7 +498,7 @@ void krylov_start(KrylovState *st, const double2 *psi, double2 *v0, int64_t n, d
     const int np = reduce_parts();
     k_norm_part<<<np, KT, 0, ctx().stream>>>(psi, n, parts);
     counted();
-    k_start<<<np, KT, 0, ctx().stream>>>(st, psi, v0, n, parts, np, stop);
+    launch_dependent(k_start, (unsigned)np, KT, 0, 0, st, psi, v0, n, parts, np, stop);
     counted();
     KV_CUDA(cudaGetLastError());
 }
@@ -562,22 +571,13 @@ void krylov_step(KrylovState *st, int k, double2 *hv, const double2 *vprev, cons
     int64_t n_prev = k > 0 ? nl.n[k - 1] : 0, n_k = nl.n[k], n_next = nl.n[k + 1];
     const bool main = &ctx() == &main_ctx();
     if (n_next <= (main ? kClusterMain : kClusterWorker)) {
-        cudaLaunchConfig_t cfg = {};
         const int full = lanczos_cluster(ctx().device);
         int size = 1;  // a CTA per virtual one, up to the largest cluster
         while (size < full && (int64_t)size * KT < n_next) size *= 2;
         const bool many = (int64_t)size * KT < n_next;
-        cfg.gridDim = dim3(size);
-        cfg.blockDim = dim3(many ? kClusterMany : kClusterOne);
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = size;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        KV_CUDA(cudaLaunchKernelEx(&cfg, many ? k_lanczos_cluster<kClusterMany> : k_lanczos_cluster<kClusterOne>, st, k, hv, vprev, vk, vnext, n_prev, n_k, n_next, P0, P1,
-                                   np, tol, max_iter, stop));
+        launch_dependent(many ? k_lanczos_cluster<kClusterMany> : k_lanczos_cluster<kClusterOne>, (unsigned)size,
+                         many ? kClusterMany : kClusterOne, 0, (unsigned)size, st, k, hv, vprev, vk, vnext, n_prev, n_k,
+                         n_next, P0, P1, np, tol, max_iter, stop);
         counted();
         return;
     }
@@ -606,15 +606,15 @@ void krylov_step(KrylovState *st, int k, double2 *hv, const double2 *vprev, cons
 }
 
 void tridiag_exp(KrylovState *st, int reverse) {
-    k_tridiag_exp<<<1, 32, 0, ctx().stream>>>(st, reverse);
+    launch_dependent(k_tridiag_exp, 1, 32, 0, 0, st, reverse);
     counted();
     KV_CUDA(cudaGetLastError());
 }
 
 void krylov_finish(KrylovState *st, double2 *const *dV, double2 *out, const KrylovLens &nl, int reverse) {
-    k_tridiag_exp<<<1, 32, 0, ctx().stream>>>(st, reverse);
+    launch_dependent(k_tridiag_exp, 1, 32, 0, 0, st, reverse);
     counted();
-    k_combine<<<reduce_parts(), KT, 0, ctx().stream>>>(st, dV, out, nl);
+    launch_dependent(k_combine, (unsigned)reduce_parts(), KT, 0, 0, st, dV, out, nl);
     counted();
     KV_CUDA(cudaGetLastError());
 }

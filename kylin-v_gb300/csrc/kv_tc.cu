@@ -354,6 +354,7 @@ __device__ __forceinline__ void slice_walk(const SliceArgs &a, int GW, int cta, 
 // grid barriers before): D = 32 12.5 -> 8.8, D = 128 two-site 30.2 -> 24.1 and
 // over 8 x 8 blocks 28.2 -> 13.1, D = 512 204 -> 127.
 __global__ void __launch_bounds__(32 * kSliceWarps) k_slice_coop(SliceArgs a, int GW, const int *skip) {
+    allow_dependents();
     if (skip && *skip) return;  // uniform over the grid: nothing in this launch writes it
     if (a.kmax) {
         slice_walk<true>(a, GW, (int)blockIdx.x, (int)gridDim.x);
@@ -362,6 +363,8 @@ __global__ void __launch_bounds__(32 * kSliceWarps) k_slice_coop(SliceArgs a, in
     slice_walk<false>(a, GW, (int)blockIdx.x, (int)gridDim.x);
 }
 __global__ void __launch_bounds__(32 * kSliceWarps) k_slice_cluster(SliceArgs a, int GW, const int *skip) {
+    allow_dependents();
+    dependency_wait();
     if (skip && *skip) return;
     if (a.kmax) {
         slice_walk<true>(a, GW, (int)blockIdx.x, (int)gridDim.x);
@@ -370,10 +373,14 @@ __global__ void __launch_bounds__(32 * kSliceWarps) k_slice_cluster(SliceArgs a,
     slice_walk<false>(a, GW, (int)blockIdx.x, (int)gridDim.x);
 }
 __global__ void __launch_bounds__(32 * kSliceWarps) k_slice_max(SliceArgs a, int GW, const int *skip) {
+    allow_dependents();
+    dependency_wait();
     if (skip && *skip) return;
     slice_walk<true>(a, GW, (int)blockIdx.x, (int)gridDim.x);
 }
 __global__ void __launch_bounds__(32 * kSliceWarps) k_slice_put(SliceArgs a, int GW, const int *skip) {
+    allow_dependents();
+    dependency_wait();
     if (skip && *skip) return;
     slice_walk<false>(a, GW, (int)blockIdx.x, (int)gridDim.x);
 }
@@ -547,10 +554,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const TcTile *__restric
                                                     double2 *__restrict__ C, const int *skip, int *err, int step,
                                                     int write_inactive, long long wait_limit, int no_copies,
                                                     int *kmax, int nkmax) {
-    if (skip && *skip) return;
-    // the balancing maxima are used up: zero for the next call's slicing
-    for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < nkmax; i += (int)(gridDim.x * blockDim.x))
-        kmax[i] = 0;
+    allow_dependents();
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + SMEM_ALIGN - 1) & ~(uintptr_t)(SMEM_ALIGN - 1));
     uint8_t *sA = smem;
@@ -582,6 +586,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const TcTile *__restric
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
+    dependency_wait();
+    if (skip && *skip) ntiles = 0;  // uniform over the grid: no role has a tile
+    else
+        // the balancing maxima are used up: zero for the next call's slicing
+        for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < nkmax; i += (int)(gridDim.x * blockDim.x))
+            kmax[i] = 0;
 
     if (warp == 0) {
         // ------------------------------------------------ producer
@@ -1285,23 +1295,12 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
         // kernels never overlap, so its grid barrier waits on no other launch)
         const int64_t rounds = (int64_t)((ctas + lim.cluster - 1) / lim.cluster) * ((p.max_k + 32 * GW - 1) / (32 * GW));
         if (!a.kmax) {
-            k_slice_put<<<(unsigned)ctas, 32 * kSliceWarps, 0, c.stream>>>(a, GW, skip);
-            KV_CUDA(cudaGetLastError());
+            launch_dependent(k_slice_put, (unsigned)ctas, 32 * kSliceWarps, 0, 0, a, GW, skip);
             ++n;
         } else if (rounds <= (main ? 2 : 6)) {
             int size = 1;
             while (size < lim.cluster && size < ctas) size *= 2;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)size);
-            cfg.blockDim = dim3(32 * kSliceWarps);
-            cfg.stream = c.stream;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)size;
-            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            KV_CUDA(cudaLaunchKernelEx(&cfg, k_slice_cluster, a, GW, skip));
+            launch_dependent(k_slice_cluster, (unsigned)size, 32 * kSliceWarps, 0, (unsigned)size, a, GW, skip);
             ++n;
         } else if (main && lim.grid > 0) {
             void *args[] = {&a, &GW, &skip};
@@ -1309,18 +1308,17 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
                                                 dim3(32 * kSliceWarps), args, 0, c.stream));
             ++n;
         } else {
-            k_slice_max<<<(unsigned)ctas, 32 * kSliceWarps, 0, c.stream>>>(a, GW, skip);
-            k_slice_put<<<(unsigned)ctas, 32 * kSliceWarps, 0, c.stream>>>(a, GW, skip);
-            KV_CUDA(cudaGetLastError());
+            launch_dependent(k_slice_max, (unsigned)ctas, 32 * kSliceWarps, 0, 0, a, GW, skip);
+            launch_dependent(k_slice_put, (unsigned)ctas, 32 * kSliceWarps, 0, 0, a, GW, skip);
             n += 2;
         }
     }
     // persistent: one CTA per SM at most (the kernel holds all of an SM's tensor memory)
     const int ntiles = p.tc_tiles;
-    k_gemm_tc<<<(unsigned)std::min(ntiles, c.num_sms), NTHREADS, SMEM_BYTES, c.stream>>>(
-        p.d_tctiles.as<TcTile>(), ntiles, p.d_xsegs.as<SegX>(), p.d_maps.as<int2>(), p.d_pairs.as<TcPair>(),
-        aph, bph, aex, bex, C, skip, err, step, p.write_inactive ? 1 : 0, g_stall_test ? (1ll << 10) : WAIT_LIMIT, g_stall_test, a.kmax, nkmax);
-    KV_CUDA(cudaGetLastError());
+    launch_dependent(k_gemm_tc, (unsigned)std::min(ntiles, c.num_sms), NTHREADS, SMEM_BYTES, 0,
+                     p.d_tctiles.as<TcTile>(), ntiles, p.d_xsegs.as<SegX>(), p.d_maps.as<int2>(),
+                     p.d_pairs.as<TcPair>(), aph, bph, aex, bex, C, skip, err, step, p.write_inactive ? 1 : 0,
+                     g_stall_test ? (1ll << 10) : WAIT_LIMIT, g_stall_test, a.kmax, nkmax);
     counted(n + 1);
     // large panels are freed stream-ordered after the GEMM
 }
