@@ -45,7 +45,7 @@ __device__ __forceinline__ double flip_sign(double v, int flip) {
 }
 
 template <int NT>
-__global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ tiles,
+__global__ void __launch_bounds__(NT, NT == 32 ? 8 : 1024 / NT) k_gemm_fp64(const GemmTile *__restrict__ tiles,
                                                   const GemmSeg *__restrict__ segs, const double2 *__restrict__ A,
                                                   const double2 *__restrict__ B, double2 *__restrict__ C, double alpha,
                                                   const int *skip, int step, int write_inactive, int cover,
@@ -85,35 +85,39 @@ __global__ void __launch_bounds__(NT) k_gemm_fp64(const GemmTile *__restrict__ t
                         const int64_t da = akc ? 1 : lda, db = bnc ? ldb : 1;
                         const double2 *pa = A + sg[i].a_off + (akc ? (int64_t)gm * lda : gm);
                         const double2 *pb = B + sg[i].b_off + (bnc ? gn : (int64_t)gn * ldb);
-                        // UL operand pairs are read ahead of the UL being multiplied
-                        constexpr int UL = NT == 32 ? 8 : 4;
-                        const int64_t sa = (int64_t)KS * da, sb = (int64_t)KS * db;
-                        const double2 *qa = pa + first * da, *qb = pb + first * db;
                         int k = first;
-                        if (k + (UL - 1) * KS < K) {
-                            double2 a[UL], b[UL];
+                        if constexpr (NT == 32) {
+                            // a warp alone on its chain: UL operand pairs are read
+                            // ahead of the UL being multiplied
+                            constexpr int UL = 8;
+                            const int64_t sa = (int64_t)KS * da, sb = (int64_t)KS * db;
+                            const double2 *qa = pa + first * da, *qb = pb + first * db;
+                            if (k + (UL - 1) * KS < K) {
+                                double2 a[UL], b[UL];
 #pragma unroll
-                            for (int u = 0; u < UL; ++u) { a[u] = qa[u * sa]; b[u] = qb[u * sb]; }
-                            for (; k + (UL - 1) * KS < K; k += UL * KS) {
-                                double2 an[UL], bn[UL];
-                                qa += UL * sa;
-                                qb += UL * sb;
-                                const bool more = k + (2 * UL - 1) * KS < K;
+                                for (int u = 0; u < UL; ++u) { a[u] = qa[u * sa]; b[u] = qb[u * sb]; }
+                                for (; k + (UL - 1) * KS < K; k += UL * KS) {
+                                    double2 an[UL], bn[UL];
+                                    qa += UL * sa;
+                                    qb += UL * sb;
+                                    const bool more = k + (2 * UL - 1) * KS < K;
 #pragma unroll
-                                for (int u = 0; u < UL; ++u) {
-                                    an[u] = more ? qa[u * sa] : make_double2(0.0, 0.0);
-                                    bn[u] = more ? qb[u * sb] : make_double2(0.0, 0.0);
-                                }
+                                    for (int u = 0; u < UL; ++u) {
+                                        an[u] = more ? qa[u * sa] : make_double2(0.0, 0.0);
+                                        bn[u] = more ? qb[u * sb] : make_double2(0.0, 0.0);
+                                    }
 #pragma unroll
-                                for (int u = 0; u < UL; ++u) {
-                                    a[u].y = flip_sign(a[u].y, fa);
-                                    b[u].y = flip_sign(b[u].y, fb);
-                                    cfma(acc, a[u], b[u]);
-                                    a[u] = an[u];
-                                    b[u] = bn[u];
+                                    for (int u = 0; u < UL; ++u) {
+                                        a[u].y = flip_sign(a[u].y, fa);
+                                        b[u].y = flip_sign(b[u].y, fb);
+                                        cfma(acc, a[u], b[u]);
+                                        a[u] = an[u];
+                                        b[u] = bn[u];
+                                    }
                                 }
                             }
                         }
+#pragma unroll 2
                         for (; k < K; k += KS) {
                             double2 a = pa[k * da], b = pb[k * db];
                             a.y = flip_sign(a.y, fa);
