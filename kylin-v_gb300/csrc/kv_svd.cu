@@ -15,7 +15,11 @@
 // The host applies the reference's global truncation and the scatter kernel
 // writes the kept columns into the U and S.V^H block tensors; the SA split's
 // new directions come from k_sa_basis / k_sa_subtract / k_sa_scatter.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <mutex>
+
 #include "kv_internal.h"
 #include "kv_jacobi.cuh"
 #include "kv_svd.h"
@@ -318,16 +322,34 @@ __device__ __forceinline__ int qrj_jacobi(float2 *sw, int ldw, int p, int r, flo
     return converged ? sweep : -sweep;
 }
 
-// Exchange columns of qrj_jacobi_reg: r/2 + 1 columns of the GJ * E packed
-// elements a group holds (rows padded past p), the column stride 8 (mod 16)
-// float2 so that the four 8-lane pieces one warp moves at a time fall in two
-// shared-memory wavefronts, and their norms.  rows: the launch's 8 * EPL.
+// Exchange columns of qrj_jacobi_reg: one slot of the GJ * E packed elements
+// a group holds (rows padded past p) per group of the CTA, the column stride
+// 8 (mod 16) float2 so that the four 8-lane pieces one warp moves at a time
+// fall in two shared-memory wavefronts, and the columns' norms; `bufs` of them.
+// rows: the launch's 8 * EPL.
 __host__ __device__ constexpr int qrj_xch_stride(int rows) { return ((rows + 15) / 16) * 16 + 8; }
-__host__ __device__ constexpr size_t qrj_xch_bytes(int rows, int kmax) {
-    return (size_t)(kmax / 2 + 2) * ((size_t)qrj_xch_stride(rows) * sizeof(float2) + sizeof(float));
+__host__ __device__ constexpr size_t qrj_xch_bytes(int rows, int slots, int bufs) {
+    return (size_t)bufs * slots * ((size_t)qrj_xch_stride(rows) * sizeof(float2) + sizeof(float));
+}
+// groups (column pairs) a CTA of a cluster of C holds for a rank up to kmax
+__host__ __device__ constexpr int qrj_slots(int kmax, int C) { return ((kmax + 1) / 2 + C - 1) / C; }
+
+// the address of this CTA's shared-memory object in CTA `rank` of the cluster, and stores to it
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, float2 v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
-// The same Jacobi with the columns held in registers for a whole sweep.
+// The same Jacobi with the columns held in registers for a whole sweep, dealt
+// over the CTAs of a cluster (each holds all of M; the result's columns 2g, 2g+1
+// are in the CTA of group g).
 // Ordering: odd-even transposition with every pair swapped after its
 // rotation, on the N = r + (r & 1) positions (column r is a zero column when r
 // is odd): even rounds pair positions (2g, 2g+1), odd rounds (2g+1, 2g+2);
@@ -336,30 +358,50 @@ __host__ __device__ constexpr size_t qrj_xch_bytes(int rows, int kmax) {
 // in even rounds and (2g+1, 2g+2) in odd ones (group n-1 idles in odd rounds
 // holding positions (2n-1, 0)); after each round one column per group moves
 // to a neighbouring group: even -> odd Y_g <- Y_{g+1 mod n}; odd -> even
-// X_g <- X_{g-1}, X_0 <- Y_{n-1}, Y_{n-1} <- X_{n-1}.  The moving columns go
-// through shared memory, one store and one load per element for every lane
-// (a warp moves four 8-row pieces at a time, two wavefronts).  The streamed
-// form reads and writes both columns of every pair each round; this moves
-// one.  On return column 2g holds X and 2g+1 holds Y of group g (positions of
-// the even layout): the caller sorts all N columns.  xch: qrj_xch_bytes(GJ E,
-// r) of shared memory.
+// X_g <- X_{g-1}, X_0 <- Y_{n-1}, Y_{n-1} <- X_{n-1}.  Every group receives one
+// column a round: its sender stores it in the receiver's slot, in the
+// receiver's CTA (a warp moves four 8-row pieces at a time, two wavefronts;
+// only a CTA's last or first group stores to another CTA).  Slots are doubled
+// where they fit (bufs = 2), so a round has one barrier: a slot is written again
+// two rounds after it was read.
+// On return column 2g holds X and 2g+1 holds Y of group g (positions of the even
+// layout).  slots: qrj_slots of the launch.
 template <int GJ, int E>
-__device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r, unsigned char *xch, int *rotated,
-                                              int max_sweeps, float tol2, float zt) {
+__device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r, unsigned char *xch, int slots,
+                                              int bufs, int *rot, int max_sweeps, float tol2, float zt) {
     constexpr int H = E / 2;
     static_assert(GJ * E <= 128 && GJ <= 32 && E % 2 == 0, "row cover");
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    auto barrier = [&] {
+        __syncwarp();
+        if (C > 1) cl.sync();
+        else __syncthreads();
+    };
     // Each lane holds rows gjl + k GJ (k < E) of its two columns as H pairs of
     // rows (2h, 2h+1), real and imaginary parts apart (XR[h] = (re, re), XI[h]
     // = (im, im)), so the complex dot products and rotations are packed FP32
     // pairs with no swapping of halves.
     constexpr int ps = qrj_xch_stride(GJ * E);
-    float2 *xd = reinterpret_cast<float2 *>(xch);  // [n + 1] exchange columns of stride ps
-    const int qe = r + (r & 1), n = qe / 2;
-    float *xn = reinterpret_cast<float *>(xd + (n + 1) * ps);  // [n + 1] their norms
+    const int qe = r + (r & 1), n = qe / 2, gpc = (n + C - 1) / C;  // gpc <= slots
+    float2 *xd = reinterpret_cast<float2 *>(xch);           // [bufs][slots] columns of stride ps
+    float *xn = reinterpret_cast<float *>(xd + (size_t)bufs * slots * ps);  // [bufs][slots] their norms
     const int tid = threadIdx.x, lane = tid & 31;
-    const int g = tid / GJ, gjl = tid % GJ;  // group, lane in the group
+    const int gl = tid / GJ, gjl = tid % GJ;  // group within the CTA, lane in the group
+    const int g = rank * gpc + gl;
     const unsigned jmask = GJ == 32 ? 0xFFFFFFFFu : (((1u << GJ) - 1u) << (lane & ~(GJ - 1)));
-    const bool act = g < n;
+    const bool act = gl < gpc && g < n;
+    // where this group's moving column goes after even and odd rounds
+    const int de = g == 0 ? n - 1 : g - 1, dodd = g >= n - 1 ? 0 : g + 1;
+    auto slot_of = [&](int d, uint32_t &col, uint32_t &nrm) {
+        const int c = act ? d / gpc : rank, sl = act ? d % gpc : 0;
+        col = cluster_addr(xd + sl * ps + gjl, c);
+        nrm = cluster_addr(xn + sl, c);
+    };
+    uint32_t ce, co, ne, no;
+    slot_of(de, ce, ne);
+    slot_of(dodd, co, no);
     float2 XR[H], XI[H], YR[H], YI[H];
 #pragma unroll
     for (int h = 0; h < H; ++h) {
@@ -379,6 +421,8 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
         for (int o = GJ / 2; o > 0; o >>= 1) v += __shfl_xor_sync(jmask, v, o, GJ);
         return v;
     };
+    if (tid == 0) rot[0] = rot[1] = 0;
+    barrier();  // every CTA's flags are cleared before one is set
     float nx = 0.f, ny = 0.f;
     int sweep = 0;
     bool converged = r < 2;
@@ -395,8 +439,7 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
             nx = gsum(a.x + a.y);
             ny = gsum(b.x + b.y);
         }
-        if (tid == 0) *rotated = 0;
-        __syncthreads();
+        bool rotated = false;
         for (int t = 0; t < qe; ++t) {
             const bool odd = t & 1;
             // ---- rotate this group's pair: c = <X, Y> = sum conj(x) y
@@ -421,7 +464,7 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
                     const float cs = rsqrtf(fmaf(tn, tn, 1.f));
                     const float sn = tn * cs;
                     const float s_re = sn * cr * rac, s_im = sn * ci * rac;
-                    if (gjl == 0) *rotated = 1;
+                    rotated = true;
                     nx = nx - tn * ac;
                     ny = ny + tn * ac;
                     // x' = cs x - conj(s) y, y' = cs y + s x, s = s_re + i s_im
@@ -437,77 +480,58 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
                     }
                 }
             }
-            // ---- move one column per group through the exchange columns
-            // (column c at xd + c * ps, the lanes' packed pairs as they are held;
-            // norms at xn[c]): store, barrier, load, barrier (the next round's
-            // stores wait for every load)
-            float2 *mine = xd + g * ps + gjl;
-            if (!odd) {
-                // Y_g <- Y_{(g+1) mod n}
-                if (act) {
+            // ---- move one column per group (the lanes' packed pairs as they are held)
+            const int b = bufs == 2 ? (t & 1) : 0;
+            if (act) {
+                const bool send_y = !odd || g == n - 1;
+                const uint32_t to = (odd ? co : ce) + (uint32_t)(b * slots * ps * (int)sizeof(float2));
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    st_cluster(to + 2 * h * GJ * sizeof(float2), send_y ? YR[h] : XR[h]);
+                    st_cluster(to + (2 * h + 1) * GJ * sizeof(float2), send_y ? YI[h] : XI[h]);
+                }
+                if (gjl == 0) st_cluster((odd ? no : ne) + (uint32_t)(b * slots * (int)sizeof(float)), send_y ? ny : nx);
+                if (odd && g == n - 1) {
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
-                        mine[2 * h * GJ] = YR[h];
-                        mine[(2 * h + 1) * GJ] = YI[h];
+                        YR[h] = XR[h];
+                        YI[h] = XI[h];
                     }
-                    if (gjl == 0) xn[g] = ny;
+                    ny = nx;
                 }
-                __syncthreads();
-                if (act) {
-                    const int src = g + 1 < n ? g + 1 : 0;
-                    const float2 *from = xd + src * ps + gjl;
+            }
+            if (t == qe - 1 && rotated && gjl == 0) {
+                if (C > 1)
+                    for (int c = 0; c < C; ++c) cl.map_shared_rank(rot, c)[sweep & 1] = 1;
+                else rot[sweep & 1] = 1;
+            }
+            barrier();
+            // the next sweep's flag: every thread has read it (at the end of the
+            // previous sweep) before this barrier, and it is set after later ones
+            if (t == 0 && tid == 0) rot[(sweep + 1) & 1] = 0;
+            if (act) {
+                const float2 *from = xd + ((size_t)b * slots + gl) * ps + gjl;
+                const float v = xn[b * slots + gl];
+                if (!odd) {
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
                         YR[h] = from[2 * h * GJ];
                         YI[h] = from[(2 * h + 1) * GJ];
                     }
-                    ny = xn[src];
-                }
-            } else {
-                // X_g <- X_{g-1}, X_0 <- Y_{n-1} (column n), Y_{n-1} <- X_{n-1}
-                if (act) {
-#pragma unroll
-                    for (int h = 0; h < H; ++h) {
-                        mine[2 * h * GJ] = XR[h];
-                        mine[(2 * h + 1) * GJ] = XI[h];
-                    }
-                    if (g == n - 1) {
-                        float2 *tail = xd + n * ps + gjl;
-#pragma unroll
-                        for (int h = 0; h < H; ++h) {
-                            tail[2 * h * GJ] = YR[h];
-                            tail[(2 * h + 1) * GJ] = YI[h];
-                        }
-                    }
-                    if (gjl == 0) {
-                        xn[g] = nx;
-                        if (g == n - 1) xn[n] = ny;
-                    }
-                }
-                __syncthreads();
-                if (act) {
-                    if (g == n - 1) {
-#pragma unroll
-                        for (int h = 0; h < H; ++h) {
-                            YR[h] = XR[h];
-                            YI[h] = XI[h];
-                        }
-                        ny = nx;
-                    }
-                    const int src = g == 0 ? n : g - 1;
-                    const float2 *from = xd + src * ps + gjl;
+                    ny = v;
+                } else {
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
                         XR[h] = from[2 * h * GJ];
                         XI[h] = from[(2 * h + 1) * GJ];
                     }
-                    nx = xn[src];
+                    nx = v;
                 }
             }
-            __syncthreads();
+            if (bufs < 2) barrier();
         }
-        converged = (*rotated == 0);
-        __syncthreads();
+        converged = rot[sweep & 1] == 0;  // the same in every CTA
+        if (bufs < 2) barrier();
     }
     if (act) {
 #pragma unroll
@@ -739,21 +763,28 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
     return r;
 }
 
+// The launch gives each sector a cluster of CTAs: every one reduces its own copy
+// of the sector (the same bits), then the register-resident Jacobi's groups are
+// dealt over them; the streamed form runs on the first alone.  slots, bufs: the
+// exchange columns per CTA and buffers of them (slots = 0: no register form).
 template <int EPL>
 __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict__ secs,
                                                     const double2 *__restrict__ T64, float2 *__restrict__ Us,
                                                     double *__restrict__ S, int *status, int *ranks, int max_sweeps,
-                                                    float tol, float qr_floor, int use_reg) {
+                                                    float tol, float qr_floor, int slots, int bufs) {
+    namespace cg = cooperative_groups;
     constexpr int NT = 512, NW = NT / 32;
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank(), sec = (int)blockIdx.x / C;
     extern __shared__ float2 sw[];
-    __shared__ int rotated;
-    const SvdSector s = secs[blockIdx.x];
+    __shared__ int rot[2];
+    const SvdSector s = secs[sec];
     const int p = s.p, q = s.q, ldw = q + 1, kmax = min(p, q);
     float2 *alph = sw + p * ldw;                          // [kmax] conj(alpha_k)
     float *cn = reinterpret_cast<float *>(alph + kmax);   // [kmax + 1] column norms^2 (Jacobi), then norms
     int *piv = reinterpret_cast<int *>(cn + kmax + 1);    // [kmax] pivot rows
     int *done = piv + kmax;                               // [p] row already pivoted
-    // [qrj_xch_bytes(8 EPL, kmax)] exchange columns of the register-resident Jacobi (use_reg)
+    // [qrj_xch_bytes(8 EPL, slots, bufs)] exchange columns of the register-resident Jacobi
     unsigned char *xch = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(done + p) + 15) & ~static_cast<uintptr_t>(15));
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -762,10 +793,11 @@ __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict_
     float fro2 = 0.f;
     const int r = qrj_reduce(s, T64, sw, ldw, alph, piv, done, qr_floor, &up, &fro2);
     if (r < 0) {  // a non-finite sector: its singular values are NaN (reported by the host)
+        if (rank != 0) return;
         for (int j = tid; j < q; j += NT) S[s.s_off + j] = nan("");
         if (tid == 0) {
-            status[blockIdx.x] = 0;
-            ranks[blockIdx.x] = 0;
+            status[sec] = 0;
+            ranks[sec] = 0;
         }
         return;
     }
@@ -774,29 +806,38 @@ __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict_
     // (r/2 pairs a round), the register capacity per lane follows EPL
     const float zt = 1e-14f * fro2;  // (1e-7 ||T||_F)^2: numerically zero columns
     const float tol2 = tol * tol;
-    int sweeps;
-    int ncol = r;  // columns holding the result (r + 1 when the register form ran on odd r)
+    int sweeps = 0;
+    int ncol = r;            // columns holding the result (r + 1 when the register form ran on odd r)
+    int j0 = 0, j1 = r;      // this CTA's columns of them
+    bool shared = false;     // the columns are dealt over the cluster
+    bool reg = false;        // the register form
+    if constexpr (EPL > 0) reg = slots > 0 && r <= 128 && (r > 32 || EPL >= 8);
+    if (!reg && rank != 0) return;  // no other CTA waits for this one or stores to it
     if constexpr (EPL > 0) {
-        constexpr int E32 = EPL >= 4 ? EPL / 4 : 1;
-        if (use_reg && r <= 128 && (r > 32 || E32 >= 2)) {
+        constexpr int E32 = EPL >= 4 ? EPL / 4 : 1, R32 = E32 >= 2 ? E32 : 2;
+        if (reg) {
             ncol = r + (r & 1);
-            if (r <= 32) sweeps = qrj_jacobi_reg<32, (E32 >= 2 ? E32 : 2)>(sw, ldw, p, r, xch, &rotated, max_sweeps, tol2, zt);
-            else if (r <= 64) sweeps = qrj_jacobi_reg<16, EPL / 2>(sw, ldw, p, r, xch, &rotated, max_sweeps, tol2, zt);
-            else sweeps = qrj_jacobi_reg<8, EPL>(sw, ldw, p, r, xch, &rotated, max_sweeps, tol2, zt);
+            shared = C > 1;
+            const int gpc = (ncol / 2 + C - 1) / C;
+            j0 = min(ncol, 2 * gpc * rank);
+            j1 = min(ncol, 2 * gpc * (rank + 1));
+            if (r <= 32) sweeps = qrj_jacobi_reg<32, R32>(sw, ldw, p, r, xch, slots, bufs, rot, max_sweeps, tol2, zt);
+            else if (r <= 64) sweeps = qrj_jacobi_reg<16, EPL / 2>(sw, ldw, p, r, xch, slots, bufs, rot, max_sweeps, tol2, zt);
+            else sweeps = qrj_jacobi_reg<8, EPL>(sw, ldw, p, r, xch, slots, bufs, rot, max_sweeps, tol2, zt);
         } else if (r <= 32) {
-            sweeps = qrj_jacobi<32, E32>(sw, ldw, p, r, cn, &rotated, max_sweeps, tol2, zt);
+            sweeps = qrj_jacobi<32, E32>(sw, ldw, p, r, cn, rot, max_sweeps, tol2, zt);
         } else if (r <= 64) {
-            sweeps = qrj_jacobi<16, EPL / 2>(sw, ldw, p, r, cn, &rotated, max_sweeps, tol2, zt);
+            sweeps = qrj_jacobi<16, EPL / 2>(sw, ldw, p, r, cn, rot, max_sweeps, tol2, zt);
         } else {
-            sweeps = qrj_jacobi<8, EPL>(sw, ldw, p, r, cn, &rotated, max_sweeps, tol2, zt);
+            sweeps = qrj_jacobi<8, EPL>(sw, ldw, p, r, cn, rot, max_sweeps, tol2, zt);
         }
     } else {
-        sweeps = qrj_jacobi<8, 0>(sw, ldw, p, r, cn, &rotated, max_sweeps, tol2, zt);
+        sweeps = qrj_jacobi<8, 0>(sw, ldw, p, r, cn, rot, max_sweeps, tol2, zt);
     }
 
     // ---- sorted singular values and normalised columns (of ncol columns the
     // r largest: a zero column beyond r sorts last)
-    for (int j = warp; j < ncol; j += NW) {
+    for (int j = j0 + warp; j < j1; j += NW) {
         float a = 0.f;
         for (int i = lane; i < p; i += 32) {
             const float2 x = sw[i * ldw + j];
@@ -804,25 +845,32 @@ __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict_
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
-        if (lane == 0) cn[j] = sqrtf(a);
+        if (!shared) {
+            if (lane == 0) cn[j] = sqrtf(a);
+        } else if (lane < C) {
+            cl.map_shared_rank(cn, lane)[j] = sqrtf(a);
+        }
     }
-    __syncthreads();
-    for (int j = warp; j < ncol; j += NW) {
+    __syncwarp();
+    if (shared) cl.sync();  // also the last access to another CTA's memory
+    else __syncthreads();
+    for (int j = j0 + warp; j < j1; j += NW) {
         const float sj = cn[j];
-        int rank = 0;
-        for (int i = 0; i < ncol; ++i) rank += (cn[i] > sj) || (cn[i] == sj && i < j);
-        if (rank >= r) continue;  // warp-uniform
+        int pos = 0;
+        for (int i = 0; i < ncol; ++i) pos += (cn[i] > sj) || (cn[i] == sj && i < j);
+        if (pos >= r) continue;  // warp-uniform
         const float inv = sj > 0.f ? 1.f / sj : 0.f;
         for (int i = lane; i < p; i += 32) {
             const float2 x = sw[i * ldw + j];
-            Us[s.t_off + (int64_t)rank * p + i] = make_float2(x.x * inv, x.y * inv);
+            Us[s.t_off + (int64_t)pos * p + i] = make_float2(x.x * inv, x.y * inv);
         }
-        if (lane == 0) S[s.s_off + rank] = (double)sj * up;
+        if (lane == 0) S[s.s_off + pos] = (double)sj * up;
     }
+    if (rank != 0) return;
     for (int j = r + tid; j < q; j += NT) S[s.s_off + j] = 0.0;  // every one of the sector's q slots
     if (tid == 0) {
-        status[blockIdx.x] = sweeps;
-        ranks[blockIdx.x] = r;
+        status[sec] = sweeps;
+        ranks[sec] = r;
     }
 }
 
@@ -1261,15 +1309,41 @@ bool svd_qrjacobi_f32(const SvdPlan &p, const double2 *T64, float2 *Us, double *
         max_p = std::max(max_p, sc.p);
     }
     if (smem > (size_t)limit) return false;
-    // the register-resident Jacobi where its exchange columns also fit
+    // The register-resident Jacobi where its exchange columns also fit, on a
+    // cluster of CTAs a sector: a round's rotations and column moves bound one
+    // SM, and a bond's sectors leave most SMs idle.  QRJ_CLUSTER_MEASURED
+    const int nsec = (int)p.secs.size(), sms = ctx().num_sms;
     const int rows = max_p <= 32 ? 32 : max_p <= 64 ? 64 : 128;  // 8 EPL of the kernel launched below
-    size_t xch = 0;
-    for (auto &sc : p.secs) xch = std::max(xch, qrj_smem(sc.p, sc.q) + 16 + qrj_xch_bytes(rows, std::min(sc.p, sc.q)));
-    const int use_reg = max_p <= 128 && xch <= (size_t)limit ? 1 : 0;
-    if (use_reg) smem = xch;
+    int C = 1, slots = 0, bufs = 1;
+    if (max_p <= 128) {
+        int kmax = 1;
+        for (auto &sc : p.secs) kmax = std::max(kmax, std::min(sc.p, sc.q));
+        while (C < 4 && 2 * C * nsec <= sms && kmax >= 32 * C) C *= 2;
+        for (bufs = 2; bufs >= 1; --bufs) {
+            size_t need = 0;
+            const int sl = qrj_slots(kmax, C);
+            for (auto &sc : p.secs) need = std::max(need, qrj_smem(sc.p, sc.q) + 16 + qrj_xch_bytes(rows, sl, bufs));
+            if (need > (size_t)limit) continue;
+            slots = sl;
+            smem = need;
+            break;
+        }
+        if (slots == 0) C = bufs = 1;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nsec * C));
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx().stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     auto launch = [&](auto kernel) {
-        kernel<<<(unsigned)p.secs.size(), 512, smem, ctx().stream>>>(p.d_secs.as<SvdSector>(), T64, Us, S, status,
-                                                                     ranks, max_sweeps, tol, qr_floor, use_reg);
+        KV_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const SvdSector *)p.d_secs.as<SvdSector>(), T64, Us, S, status, ranks,
+                                   max_sweeps, tol, qr_floor, slots, bufs));
     };
     // elements per lane from the longest column of the launch (8 lanes a pair)
     if (max_p <= 32) launch(k_svd_qrj<4>);
