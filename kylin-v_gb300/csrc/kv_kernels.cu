@@ -323,25 +323,70 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
 }
 
 // ------------------------------------------------------------ permute
-// desc per block (16 int64): in_off, out_off, size, rank, shape[6], perm[6]
-__global__ void k_permute(const int64_t *__restrict__ desc, const double2 *__restrict__ in,
-                          double2 *__restrict__ out) {
+// desc per block (16 int64): in_off, out_off, size, rank, shape[6], perm[6].
+// A CTA takes kPermChunk elements of a block at a time (blockIdx.y, striding
+// over the grid), so a tensor of one large block uses the whole chip; 32-bit
+// index divisions; an identity permutation is a copy.  A latency-bound copy for
+// small blocks: 98 -> 9 us for one of 96 x 5 x 12 x 96 x 5 elements a CTA walked
+// alone.
+constexpr int kPermChunk = 1024;
+__global__ void __launch_bounds__(256) k_permute(const int64_t *__restrict__ desc, const double2 *__restrict__ in,
+                                                 double2 *__restrict__ out) {
     const int64_t *d = desc + 16 * blockIdx.x;
     const int64_t in_off = d[0], out_off = d[1], size = d[2];
     const int rank = (int)d[3];
-    int64_t sd[kMaxRank], od[kMaxRank], osh[kMaxRank];
-    sd[rank - 1] = 1;
-    for (int i = rank - 2; i >= 0; --i) sd[i] = sd[i + 1] * d[4 + i + 1];
-    for (int i = 0; i < rank; ++i) osh[i] = d[4 + d[10 + i]];
-    od[rank - 1] = 1;
-    for (int i = rank - 2; i >= 0; --i) od[i] = od[i + 1] * osh[i + 1];
-    for (int64_t e = threadIdx.x; e < size; e += blockDim.x) {
-        int64_t dst = 0;
-        for (int j = 0; j < rank; ++j) {
-            int ax = (int)d[10 + j];
-            dst += ((e / sd[ax]) % d[4 + ax]) * od[j];
+    if ((int64_t)blockIdx.y * kPermChunk >= size) return;
+    // strides of the input's axes, and the output stride of each input axis (0 past the rank)
+    unsigned sd[kMaxRank], sh[kMaxRank];
+    int64_t od[kMaxRank];
+    bool same = true;
+    {
+        int64_t st = 1;
+#pragma unroll
+        for (int i = kMaxRank - 1; i >= 0; --i) {
+            sh[i] = i < rank ? (unsigned)d[4 + i] : 1u;
+            sd[i] = (unsigned)st;
+            od[i] = 0;
+            st *= sh[i];
         }
-        out[out_off + dst] = in[in_off + e];
+        int64_t ost = 1;
+        for (int j = rank - 1; j >= 0; --j) {
+            const int ax = (int)d[10 + j];
+            same = same && ax == j;
+#pragma unroll
+            for (int i = 0; i < kMaxRank; ++i)
+                if (i == ax) {
+                    od[i] = ost;
+                    ost *= sh[i];
+                }
+        }
+    }
+    const bool wide = size >= (1ll << 31);
+    for (int64_t c0 = (int64_t)blockIdx.y * kPermChunk; c0 < size; c0 += (int64_t)gridDim.y * kPermChunk) {
+        const int64_t c1 = min(size, c0 + kPermChunk);
+        for (int64_t e = c0 + threadIdx.x; e < c1; e += 256) {
+            int64_t dst = e;
+            if (!same) {
+                dst = 0;
+                if (wide) {
+                    int64_t rem = e;
+                    for (int i = rank - 1; i >= 0; --i) {
+                        dst += (rem % sh[i]) * od[i];
+                        rem /= sh[i];
+                    }
+                } else {
+                    unsigned rem = (unsigned)e;
+#pragma unroll
+                    for (int i = 0; i < kMaxRank; ++i)
+                        if (i < rank) {
+                            const unsigned x = rem / sd[i];
+                            rem -= x * sd[i];
+                            dst += x * od[i];
+                        }
+                }
+            }
+            out[out_off + dst] = in[in_off + e];
+        }
     }
 }
 
@@ -441,7 +486,12 @@ void launch_mix(const MixPlan &p, const double2 *in, const double2 *W, double2 *
 void launch_permute(const double2 *in, double2 *out, const std::vector<int64_t> &desc, int nblocks) {
     if (nblocks == 0) return;
     DevBuf d = upload_vec(desc);
-    k_permute<<<nblocks, 256, 0, ctx().stream>>>(d.as<int64_t>(), in, out);
+    int64_t most = 1;
+    for (int b = 0; b < nblocks; ++b) most = std::max(most, desc[16 * (size_t)b + 2]);
+    // enough CTAs a block for its chunks, no more in all than eight waves of the chip need
+    const int64_t chunks = (most + kPermChunk - 1) / kPermChunk;
+    const unsigned gy = (unsigned)std::min<int64_t>(chunks, std::max<int64_t>(1, 64ll * ctx().num_sms / nblocks));
+    k_permute<<<dim3((unsigned)nblocks, gy), 256, 0, ctx().stream>>>(d.as<int64_t>(), in, out);
     counted();
     KV_CUDA(cudaGetLastError());
     // d is freed stream-ordered after the kernel

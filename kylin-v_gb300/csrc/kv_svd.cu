@@ -1029,20 +1029,27 @@ __global__ void k_chol(const SvdPolish *__restrict__ pol, double2 *__restrict__ 
 
 // X <- X R^{-1} row by row (R upper, from k_chol): y_c = (x_c - sum_{a<c} y_a R[a,c]) / R[c,c].
 // One warp per row (kTrsmRows rows per CTA): the solved y live in shared
-// memory, lanes split each inner sum, a shuffle tree reduces it.
+// memory, lanes split each inner sum, a shuffle tree reduces it (the real
+// parts in the lower lanes, the imaginary ones in the upper, after the first
+// level: a warp's FP64 instruction costs the same for half its lanes).  The
+// diagonal's reciprocals are taken once per CTA.
 __global__ void __launch_bounds__(32 * kTrsmRows) k_trsm_rows(const SvdPolish *__restrict__ pol,
                                                               const int *__restrict__ item_pol,
                                                               const int *__restrict__ item_row0,
                                                               const double2 *__restrict__ G, double2 *__restrict__ X) {
-    extern __shared__ double2 ys[];  // [kTrsmRows][kmax]
+    extern __shared__ double2 ys[];  // [kTrsmRows][k] solved rows, then [k] reciprocals
     const SvdPolish d = pol[item_pol[blockIdx.x]];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = item_row0[blockIdx.x] + warp;
-    if (row >= d.rows) return;  // warp-uniform
     const int k = d.k;
     const double2 *r = G + d.g_off;
+    double *rd = reinterpret_cast<double *>(ys + (int64_t)kTrsmRows * k);
+    for (int c = threadIdx.x; c < k; c += blockDim.x) rd[c] = 1.0 / r[(int64_t)c * k + c].x;
+    __syncthreads();
+    if (row >= d.rows) return;  // warp-uniform
     double2 *x = X + d.x_off + (int64_t)row * d.ldx;
     double2 *y = ys + (int64_t)warp * k;
+    const bool hi = lane >= 16;
     for (int c = 0; c < k; ++c) {
         double sr = 0.0, si = 0.0;
         for (int a = lane; a < c; a += 32) {
@@ -1050,14 +1057,14 @@ __global__ void __launch_bounds__(32 * kTrsmRows) k_trsm_rows(const SvdPolish *_
             sr += ya.x * rac.x - ya.y * rac.y;
             si += ya.x * rac.y + ya.y * rac.x;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xFFFFFFFFu, sr, o);
-            si += __shfl_xor_sync(0xFFFFFFFFu, si, o);
-        }
-        if (lane == 0) {
-            const double2 v = x[c];
-            const double inv = 1.0 / r[(int64_t)c * k + c].x;
-            y[c] = make_double2((v.x - sr) * inv, (v.y - si) * inv);
+        double t = hi ? si : sr;
+        t += __shfl_xor_sync(0xFFFFFFFFu, hi ? sr : si, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+        // lane 0: the real part of y_c, lane 16: the imaginary part
+        if ((lane & 15) == 0) {
+            const double v = reinterpret_cast<const double *>(x + c)[hi ? 1 : 0];
+            reinterpret_cast<double *>(y + c)[hi ? 1 : 0] = (v - t) * rd[c];
         }
         __syncwarp();
     }
@@ -1311,7 +1318,9 @@ bool svd_qrjacobi_f32(const SvdPlan &p, const double2 *T64, float2 *Us, double *
     if (smem > (size_t)limit) return false;
     // The register-resident Jacobi where its exchange columns also fit, on a
     // cluster of CTAs a sector: a round's rotations and column moves bound one
-    // SM, and a bond's sectors leave most SMs idle.  QRJ_CLUSTER_MEASURED
+    // SM, and a bond's sectors leave most SMs idle.  Measured, the whole split of
+    // 17 sectors of 128 x 128: one CTA 1985 us, two 1727, four 1631, eight 1799 (a
+    // larger cluster's barrier costs more than its shorter round saves).
     const int nsec = (int)p.secs.size(), sms = ctx().num_sms;
     const int rows = max_p <= 32 ? 32 : max_p <= 64 ? 64 : 128;  // 8 EPL of the kernel launched below
     int C = 1, slots = 0, bufs = 1;
@@ -1387,8 +1396,8 @@ void svd_chol(const DevBuf &pol, int npol, double2 *G, double2 *fail, double shi
 void svd_trsm(const DevBuf &pol, const std::vector<int> &item_pol, const std::vector<int> &item_row0,
               const double2 *G, double2 *X, int kmax) {
     if (item_pol.empty()) return;
-    const size_t smem = (size_t)kTrsmRows * std::max(1, kmax) * sizeof(double2);
-    constexpr int kTrsmSmemMax = 200 * 1024;
+    const size_t smem = (size_t)std::max(1, kmax) * (kTrsmRows * sizeof(double2) + sizeof(double));
+    constexpr int kTrsmSmemMax = 200 * 1024 * 17 / 16;  // kept dimensions up to 1600
     KV_REQUIRE(smem <= kTrsmSmemMax, KV_EINVAL, "SVD polish: kept dimension of one sector too large");
     trsm_smem_raise(ctx().device, kTrsmSmemMax);  // once per device, to the largest size allowed here
     DevSpan ip, ir;

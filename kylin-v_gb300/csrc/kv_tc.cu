@@ -554,7 +554,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const TcTile *__restric
                                                     double2 *__restrict__ C, const int *skip, int *err, int step,
                                                     int write_inactive, long long wait_limit, int no_copies,
                                                     int *kmax, int nkmax) {
-    allow_dependents();
+    // no allow_dependents: its successors' CTAs gain nothing by waiting beside a
+    // CTA that holds the SM (D = 512 Lanczos exponential 9.93 ms with, 9.81 without)
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + SMEM_ALIGN - 1) & ~(uintptr_t)(SMEM_ALIGN - 1));
     uint8_t *sA = smem;
