@@ -46,8 +46,18 @@ namespace {
 constexpr int NT = 256, NW = NT / 32;
 constexpr int kXStage = 4096;  // longest pivot row staged in shared memory
 
-__device__ __forceinline__ double2 ldg2(const double2 *p) { return __ldcg(p); }
-__device__ __forceinline__ void stg2(double2 *p, double2 v) { __stcg(p, v); }
+// Data that other CTAs of the cluster read or write goes through L2; a sector of
+// one CTA (ONE) keeps it in the SM's L1.
+template <bool ONE, class T>
+__device__ __forceinline__ T ldg(const T *p) {
+    if constexpr (ONE) return *p;
+    else return __ldcg(p);
+}
+template <bool ONE, class T>
+__device__ __forceinline__ void stg(T *p, T v) {
+    if constexpr (ONE) *p = v;
+    else __stcg(p, v);
+}
 
 // sums of two / four values over groups of G lanes, every lane of the group
 // receiving them: at the first levels a lane passes on half of its values, so
@@ -102,6 +112,26 @@ __device__ __forceinline__ double widen(float x) {
     return __hiloint2double((u & (int)0x80000000) | ((E - 127 + 1023) << 20) | (m >> 3), m << 29);
 }
 
+// 1 / sqrt(x) and 1 / x for normal x > 0 away from the range's ends: two Newton
+// steps on an FP32 start, about ten FP64 instructions each in place of some
+// thirty (64 clocks a warp each), to within two units in the last place
+__device__ __forceinline__ double newton_rsqrt(double x) {
+    int e;
+    float m = mantissa(x, e);
+    if (e & 1) m *= 2.f;
+    e = (e - (e & 1)) / 2;
+    double y = __hiloint2double(__double2hiint(widen(rsqrtf(m))) - (e << 20), __double2loint(widen(rsqrtf(m))));
+    y = fma(y * 0.5, fma(-x * y, y, 1.0), y);
+    return fma(y * 0.5, fma(-x * y, y, 1.0), y);
+}
+__device__ __forceinline__ double newton_reciprocal(double x) {
+    int e;
+    const double r = widen(__fdividef(1.f, mantissa(x, e)));
+    double y = __hiloint2double(__double2hiint(r) - (e << 20), __double2loint(r));
+    y = fma(y, fma(-x, y, 1.0), y);
+    return fma(y, fma(-x, y, 1.0), y);
+}
+
 // The Jacobi rotation of a column pair with |x|^2 = a, |y|^2 = b, x^H y = c
 // != 0 (x' = cs x - conj(s) y, y' = s x + cs y): tau = t c/|c| with
 // t = sign(z) / (|z| + sqrt(1 + z^2)), z = (b - a) / (2|c|), in FP32; then
@@ -128,14 +158,9 @@ __device__ __forceinline__ void rotation(double a, double b, double cr, double c
         ti = widen(t * fi * rn);
     }
     const double w = fma(tr, tr, fma(ti, ti, 1.0));  // in [1, 2]
-    int ew;
-    const float fw = mantissa(w, ew);
-    double y = widen(rsqrtf(fw * pow2f(ew)));
-    y = fma(y * 0.5, fma(-w * y, y, 1.0), y);
-    y = fma(y * 0.5, fma(-w * y, y, 1.0), y);
-    cs = y;
-    sr = y * tr;
-    si = y * ti;
+    cs = newton_rsqrt(w);
+    sr = cs * tr;
+    si = cs * ti;
 }
 
 struct Svd64Sector {
@@ -152,7 +177,7 @@ struct Cand {
     int row, bad;
 };
 
-template <int G, int EPL>
+template <int G, int EPL, bool ONE>
 __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ secs, const double2 *__restrict__ T,
                                               double2 *U, double2 *M, double *S, double2 *alph, double *nrm,
                                               int *done, Cand *cand, int *flags, int *status,
@@ -163,6 +188,13 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
     __shared__ double wv[NW];
     __shared__ int wi[NW], wbad[NW];
     __shared__ double2 sc[2];  // v0 and (beta, nu) of the step
+    __shared__ Cand own[2];    // ONE: the candidates
+    auto sync = [&] {
+        if constexpr (ONE) __syncthreads();
+        else cl.sync();
+    };
+    auto ldg2 = [](const double2 *p) { return ldg<ONE>(p); };
+    auto stg2 = [](double2 *p, double2 v) { stg<ONE>(p, v); };
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int sec = blockIdx.x / C;
     const Svd64Sector s = secs[sec];
@@ -193,10 +225,10 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                 bad |= wbad[x];
                 if (wv[x] > bv || (wv[x] == bv && wi[x] < bi)) { bv = wv[x]; bi = wi[x]; }
             }
-            Cand *o = cd + slot * 16 + rank;
-            __stcg(&o->v, bv);
-            __stcg(&o->row, bi);
-            __stcg(&o->bad, bad);
+            Cand *o = ONE ? own + slot : cd + slot * 16 + rank;
+            stg<ONE>(&o->v, bv);
+            stg<ONE>(&o->row, bi);
+            stg<ONE>(&o->bad, bad);
         }
     };
 
@@ -220,7 +252,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         if (rank == 0 && tid < 4) fl[tid] = 0;
         publish(bv, bi, bad, 0);
     }
-    cl.sync();
+    sync();
 
     // ---- pivoted Householder on the rows
     int r = 0;
@@ -229,10 +261,10 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         double mv = -1.0;
         int ip = 0x7FFFFFFF, bad = 0;
         for (int x = 0; x < C; ++x) {  // the same in every CTA
-            const Cand *o = cd + (k & 1) * 16 + x;
-            const double v = __ldcg(&o->v);
-            const int i = __ldcg(&o->row);
-            bad |= __ldcg(&o->bad);
+            const Cand *o = ONE ? own + (k & 1) : cd + (k & 1) * 16 + x;
+            const double v = ldg<ONE>(&o->v);
+            const int i = ldg<ONE>(&o->row);
+            bad |= ldg<ONE>(&o->bad);
             if (v > mv || (v == mv && i < ip)) { mv = v; ip = i; }
         }
         if (bad) { nonfinite = true; break; }
@@ -246,12 +278,25 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         // beta = 2 / |v|^2 = 1 / (|u| (|u| + |u_0|))
         if (warp == 0) {
             const double2 x0 = ldg2(xr + k);
-            const double nu = sqrt(mv), a0 = sqrt(fma(x0.x, x0.x, x0.y * x0.y));
-            const double ia = a0 > 0.0 ? 1.0 / a0 : 0.0;
+            const double n0 = fma(x0.x, x0.x, x0.y * x0.y);
+            double nu, a0, ia, beta;
+            if (mv > 1e-140 && mv < 1e140 && (n0 == 0.0 || n0 > 1e-280)) {
+                const double y = newton_rsqrt(mv);
+                nu = mv * y;
+                nu = fma(0.5 * y, fma(-nu, nu, mv), nu);
+                ia = n0 > 0.0 ? newton_rsqrt(n0) : 0.0;
+                a0 = n0 * ia;
+                beta = newton_reciprocal(nu * (nu + a0));
+            } else {
+                nu = sqrt(mv);
+                a0 = sqrt(n0);
+                ia = a0 > 0.0 ? 1.0 / a0 : 0.0;
+                beta = 1.0 / (nu * (nu + a0));
+            }
             const double pr = a0 > 0.0 ? x0.x * ia : 1.0, pi = -x0.y * ia;  // e^{i phi}
             if (lane == 0) {
                 sc[0] = make_double2(pr * (a0 + nu), pi * (a0 + nu));
-                sc[1] = make_double2(1.0 / (nu * (nu + a0)), 0.0);
+                sc[1] = make_double2(beta, 0.0);
                 if (ip % C == rank) {
                     al[k] = make_double2(-pr * nu, pi * nu);  // conj(alpha): the pivot row's entry k
                     dn[ip] = k;
@@ -292,7 +337,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
             if (ta > bv) { bv = ta; bi = i; }
         }
         publish(bv, bi, isbad, (k + 1) & 1);
-        cl.sync();
+        sync();
     }
     if (nonfinite) {  // uniform over the cluster: reported by the host
         if (rank == 0)
@@ -309,7 +354,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
             stg2(m + (int64_t)c * p + i, v);
         }
     }
-    cl.sync();
+    sync();
 
     // ---- one-sided Jacobi on M's r columns: a round's pairs two (G = 16) or
     // one (G = 32) a warp, dealt over the CTAs first
@@ -320,7 +365,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
     int sweep = 0;
     bool converged = r < 2;
     for (; sweep < max_sweeps && !converged; ++sweep) {
-        if (rank == 0 && tid == 0) __stcg(fl + (sweep + 1) % 3, 0);  // last read two sweeps ago
+        if (rank == 0 && tid == 0) stg<ONE>(fl + (sweep + 1) % 3, 0);  // last read two sweeps ago
         bool rotated = false;
         for (int rr = 0; rr < m1; ++rr) {
             for (int wt = rank + C * warp; wt * PW < np; wt += C * NW) {  // warp-uniform
@@ -394,11 +439,11 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                     }
                 }
             }
-            if (rr == m1 - 1 && rotated) __stcg(fl + sweep % 3, 1);
+            if (rr == m1 - 1 && rotated) stg<ONE>(fl + sweep % 3, 1);
             __syncwarp();
-            cl.sync();
+            sync();
         }
-        converged = __ldcg(fl + sweep % 3) == 0;  // the same in every CTA
+        converged = ldg<ONE>(fl + sweep % 3) == 0;  // the same in every CTA
     }
     if (rank == 0 && tid == 0) status[sec] = converged ? sweep : -sweep;
 
@@ -412,17 +457,17 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
             }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
-        if (lane == 0) __stcg(nv + j, sqrt(a));
+        if (lane == 0) stg<ONE>(nv + j, sqrt(a));
     }
-    cl.sync();
+    sync();
     int zeros = 0;  // columns of norm zero, the same in every warp
     for (int j0 = 0; j0 < kmax; j0 += 32)
-        zeros += __popc(__ballot_sync(0xFFFFFFFFu, j0 + lane < kmax && !(__ldcg(nv + min(j0 + lane, kmax - 1)) > 0.0)));
+        zeros += __popc(__ballot_sync(0xFFFFFFFFu, j0 + lane < kmax && !(ldg<ONE>(nv + min(j0 + lane, kmax - 1)) > 0.0)));
     for (int j = rank + C * warp; j < kmax; j += C * NW) {
-        const double sj = __ldcg(nv + j);
+        const double sj = ldg<ONE>(nv + j);
         int pos = 0;
         for (int i = lane; i < kmax; i += 32) {
-            const double si = __ldcg(nv + i);
+            const double si = ldg<ONE>(nv + i);
             pos += (si > sj) || (si == sj && i < j);
         }
 #pragma unroll
@@ -438,7 +483,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
     if (rank == 0)
         for (int j = kmax + tid; j < q; j += NT) S[s.s_off + j] = 0.0;
     if (zeros == 0) return;  // uniform over the cluster
-    cl.sync();
+    sync();
     if (rank != 0) return;
     // ---- the last `zeros` vectors: unit vectors e_i made orthogonal (twice)
     // to all before them, i the row those leave the most of e_i in
@@ -513,9 +558,13 @@ bool svd64_setup(int dev) {
     KV_REQUIRE(dev >= 0 && dev < kMaxDevices, KV_EINVAL, "device index out of range");
     std::lock_guard<std::mutex> lk(mu);
     if (state[dev] == 0) {
-        const void *ks[] = {(const void *)k_svd64<16, 4>, (const void *)k_svd64<16, 8>, (const void *)k_svd64<16, 16>,
-                            (const void *)k_svd64<16, 0>, (const void *)k_svd64<32, 2>, (const void *)k_svd64<32, 4>,
-                            (const void *)k_svd64<32, 8>, (const void *)k_svd64<32, 0>};
+        const void *ks[] = {(const void *)k_svd64<16, 4, false>, (const void *)k_svd64<16, 8, false>,
+                            (const void *)k_svd64<16, 16, false>, (const void *)k_svd64<16, 0, false>,
+                            (const void *)k_svd64<32, 2, false>, (const void *)k_svd64<32, 4, false>,
+                            (const void *)k_svd64<32, 8, false>, (const void *)k_svd64<32, 0, false>};
+        for (const void *k : {(const void *)k_svd64<16, 4, true>, (const void *)k_svd64<16, 8, true>,
+                              (const void *)k_svd64<16, 16, true>, (const void *)k_svd64<16, 0, true>})
+            KV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kXBytes));
         int ok = 1;
         for (const void *k : ks) {
             KV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kXBytes));
@@ -574,11 +623,20 @@ void svd_fp64(const SvdPlan &P, const double2 *T, double2 *U, double *S, int *st
         C *= 2;
         wide = C * 4 >= pairs;
     }
-    DevBuf ds = upload_vec(secs);
-    DevBuf M(std::max<int64_t>(1, P.t_elems) * sizeof(double2));
-    DevBuf al(std::max<int64_t>(1, k_elems) * sizeof(double2)), nv(std::max<int64_t>(1, k_elems) * sizeof(double));
-    DevBuf dn(std::max<int64_t>(1, r_elems) * sizeof(int));
-    DevBuf cd((size_t)nsec * 32 * sizeof(Cand)), fl((size_t)nsec * 4 * sizeof(int));
+    // one allocation: sectors, M, diagonal entries, norms, row flags, candidates, sweep flags
+    size_t bytes = 0;
+    auto carve = [&](size_t n) {
+        const size_t o = bytes;
+        bytes += (n + 255) & ~size_t(255);
+        return o;
+    };
+    const size_t o_ds = carve(secs.size() * sizeof(Svd64Sector)), o_m = carve((size_t)P.t_elems * sizeof(double2)),
+                 o_al = carve((size_t)k_elems * sizeof(double2)), o_nv = carve((size_t)k_elems * sizeof(double)),
+                 o_dn = carve((size_t)r_elems * sizeof(int)), o_cd = carve((size_t)nsec * 32 * sizeof(Cand)),
+                 o_fl = carve((size_t)nsec * 4 * sizeof(int));
+    DevBuf ws(bytes);
+    char *wp = ws.as<char>();
+    upload_bytes(wp + o_ds, secs.data(), secs.size() * sizeof(Svd64Sector));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nsec * C));
     cfg.blockDim = dim3(NT);
@@ -591,21 +649,28 @@ void svd_fp64(const SvdPlan &P, const double2 *T, double2 *U, double *S, int *st
     cfg.attrs = at;
     cfg.numAttrs = 1;
     auto launch = [&](auto kernel) {
-        KV_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const Svd64Sector *)ds.as<Svd64Sector>(), T, U, M.as<double2>(), S,
-                                   al.as<double2>(), nv.as<double>(), dn.as<int>(), cd.as<Cand>(),
-                                   fl.as<int>(), status, max_sweeps, tol));
+        KV_CUDA(cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const Svd64Sector *>(wp + o_ds), T, U,
+                                   reinterpret_cast<double2 *>(wp + o_m), S, reinterpret_cast<double2 *>(wp + o_al),
+                                   reinterpret_cast<double *>(wp + o_nv), reinterpret_cast<int *>(wp + o_dn),
+                                   reinterpret_cast<Cand *>(wp + o_cd), reinterpret_cast<int *>(wp + o_fl), status,
+                                   max_sweeps, tol));
     };
     // a column's elements stay in registers between the sums and the rotation up to 256 rows
-    if (wide) {
-        if (max_p <= 64) launch(k_svd64<32, 2>);
-        else if (max_p <= 128) launch(k_svd64<32, 4>);
-        else if (max_p <= 256) launch(k_svd64<32, 8>);
-        else launch(k_svd64<32, 0>);
+    if (C == 1) {
+        if (max_p <= 64) launch(k_svd64<16, 4, true>);
+        else if (max_p <= 128) launch(k_svd64<16, 8, true>);
+        else if (max_p <= 256) launch(k_svd64<16, 16, true>);
+        else launch(k_svd64<16, 0, true>);
+    } else if (wide) {
+        if (max_p <= 64) launch(k_svd64<32, 2, false>);
+        else if (max_p <= 128) launch(k_svd64<32, 4, false>);
+        else if (max_p <= 256) launch(k_svd64<32, 8, false>);
+        else launch(k_svd64<32, 0, false>);
     } else {
-        if (max_p <= 64) launch(k_svd64<16, 4>);
-        else if (max_p <= 128) launch(k_svd64<16, 8>);
-        else if (max_p <= 256) launch(k_svd64<16, 16>);
-        else launch(k_svd64<16, 0>);
+        if (max_p <= 64) launch(k_svd64<16, 4, false>);
+        else if (max_p <= 128) launch(k_svd64<16, 8, false>);
+        else if (max_p <= 256) launch(k_svd64<16, 16, false>);
+        else launch(k_svd64<16, 0, false>);
     }
     counted();
 }
