@@ -62,13 +62,11 @@ __device__ __forceinline__ void stg(T *p, T v) {
 // sums of two / four values over groups of G lanes, every lane of the group
 // receiving them: at the first levels a lane passes on half of its values, so
 // the four sums cost 2 + 1 + ... additions instead of 4 a level
-template <int G>
-__device__ __forceinline__ void group_sum2(double &a, double &b) {
+__device__ __forceinline__ void group_sum2(double &a, double &b, int G) {
     const int lane = threadIdx.x & 31;
     const bool hi = lane & 1;
     double keep = hi ? b : a, give = hi ? a : b;
     keep += __shfl_xor_sync(0xFFFFFFFFu, give, 1);
-#pragma unroll
     for (int o = 2; o < G; o <<= 1) keep += __shfl_xor_sync(0xFFFFFFFFu, keep, o);
     const double other = __shfl_xor_sync(0xFFFFFFFFu, keep, 1);
     a = hi ? other : keep;
@@ -232,22 +230,30 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         }
     };
 
-    // ---- rows i = rank, rank + C, ... belong to this CTA, row i to warp (i / C) % NW
+    // ---- rows i = rank, rank + C, ... belong to this CTA.  A group of lanes takes
+    // a row, as many as the row's length keeps busy: a warp's FP64 instruction
+    // costs the same for idle lanes.
+    auto lanes_for = [](int n) { return n > 64 ? 32 : n > 24 ? 16 : n > 8 ? 8 : 4; };
     {
         double bv = -1.0;
         int bi = 0x7FFFFFFF, bad = 0;
-        for (int i = rank + C * warp; i < p; i += C * NW) {
+        const int GQ = lanes_for(q), RW = 32 / GQ, sub = lane / GQ, gl = lane % GQ;
+        for (int base = warp * RW; rank + C * base < p; base += NW * RW) {  // warp-uniform
+            const int i = rank + C * (base + sub);
             double a = 0.0;
-            for (int c = lane; c < q; c += 32) {
-                const double2 v = t[i + (int64_t)c * p];
-                w[(int64_t)i * q + c] = v;
-                a = fma(v.x, v.x, fma(v.y, v.y, a));
+            if (i < p)
+                for (int c = gl; c < q; c += GQ) {
+                    const double2 v = t[i + (int64_t)c * p];
+                    w[(int64_t)i * q + c] = v;
+                    a = fma(v.x, v.x, fma(v.y, v.y, a));
+                }
+            __syncwarp();
+            for (int o = GQ / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+            if (i < p) {
+                if (gl == 0) dn[i] = -1;
+                if (!isfinite(a)) bad = 1;
+                if (a > bv || (a == bv && i < bi)) { bv = a; bi = i; }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
-            if (lane == 0) dn[i] = -1;
-            if (!isfinite(a)) bad = 1;
-            if (a > bv) { bv = a; bi = i; }
         }
         if (rank == 0 && tid < 4) fl[tid] = 0;
         publish(bv, bi, bad, 0);
@@ -308,33 +314,41 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         const double beta = sc[1].x;
         double bv = -1.0;
         int bi = 0x7FFFFFFF, isbad = 0;
-        for (int i = rank + C * warp; i < p; i += C * NW) {
-            if (dn[i] >= 0) continue;  // warp-uniform
-            double2 *wr = w + (int64_t)i * q;
+        const int GQ = lanes_for(q - k), RW = 32 / GQ, sub = lane / GQ, gl = lane % GQ;
+        for (int base = warp * RW; rank + C * base < p; base += NW * RW) {  // warp-uniform
+            const int i = rank + C * (base + sub);
+            const bool live = i < p && dn[i] < 0;
+            if (!__any_sync(0xFFFFFFFFu, live)) continue;
+            double2 *wr = w + (int64_t)(live ? i : rank) * q;
             double sr = 0.0, si = 0.0;  // sum_c w_c v_c, v_c = conj(x_c) for c > k, v_k = v0
-            for (int c = k + lane; c < q; c += 32) {
-                const double2 xc = staged ? xs[c] : ldg2(xr + c);
-                const double2 vc = c == k ? v0 : make_double2(xc.x, -xc.y);
-                const double2 a = wr[c];
-                sr = fma(a.x, vc.x, fma(-a.y, vc.y, sr));
-                si = fma(a.x, vc.y, fma(a.y, vc.x, si));
-            }
-            group_sum2<32>(sr, si);
+            if (live)
+                for (int c = k + gl; c < q; c += GQ) {
+                    const double2 xc = staged ? xs[c] : ldg2(xr + c);
+                    const double2 vc = c == k ? v0 : make_double2(xc.x, -xc.y);
+                    const double2 a = wr[c];
+                    sr = fma(a.x, vc.x, fma(-a.y, vc.y, sr));
+                    si = fma(a.x, vc.y, fma(a.y, vc.x, si));
+                }
+            __syncwarp();
+            group_sum2(sr, si, GQ);
             const double fr = beta * sr, fi = beta * si;
             double ta = 0.0;
-            for (int c = k + lane; c < q; c += 32) {
-                const double2 xc = staged ? xs[c] : ldg2(xr + c);
-                const double2 cv = c == k ? make_double2(v0.x, -v0.y) : xc;  // conj(v_c)
-                double2 a = wr[c];
-                a.x = fma(-fr, cv.x, fma(fi, cv.y, a.x));
-                a.y = fma(-fr, cv.y, fma(-fi, cv.x, a.y));
-                wr[c] = a;
-                if (c > k) ta = fma(a.x, a.x, fma(a.y, a.y, ta));
+            if (live)
+                for (int c = k + gl; c < q; c += GQ) {
+                    const double2 xc = staged ? xs[c] : ldg2(xr + c);
+                    const double2 cv = c == k ? make_double2(v0.x, -v0.y) : xc;  // conj(v_c)
+                    double2 a = wr[c];
+                    a.x = fma(-fr, cv.x, fma(fi, cv.y, a.x));
+                    a.y = fma(-fr, cv.y, fma(-fi, cv.x, a.y));
+                    wr[c] = a;
+                    if (c > k) ta = fma(a.x, a.x, fma(a.y, a.y, ta));
+                }
+            __syncwarp();
+            for (int o = GQ / 2; o > 0; o >>= 1) ta += __shfl_xor_sync(0xFFFFFFFFu, ta, o);
+            if (live) {
+                if (!isfinite(ta)) isbad = 1;
+                if (ta > bv || (ta == bv && i < bi)) { bv = ta; bi = i; }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ta += __shfl_xor_sync(0xFFFFFFFFu, ta, o);
-            if (!isfinite(ta)) isbad = 1;
-            if (ta > bv) { bv = ta; bi = i; }
         }
         publish(bv, bi, isbad, (k + 1) & 1);
         sync();
@@ -519,7 +533,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                     sr = fma(a.x, b.x, fma(a.y, b.y, sr));
                     si = fma(a.x, b.y, fma(-a.y, b.x, si));
                 }
-                group_sum2<32>(sr, si);
+                group_sum2(sr, si, 32);
                 __syncthreads();
                 for (int i = tid; i < p; i += NT) {
                     const double2 a = ldg2(w + (int64_t)c * p + i);
@@ -563,7 +577,9 @@ bool svd64_setup(int dev) {
                             (const void *)k_svd64<32, 2, false>, (const void *)k_svd64<32, 4, false>,
                             (const void *)k_svd64<32, 8, false>, (const void *)k_svd64<32, 0, false>};
         for (const void *k : {(const void *)k_svd64<16, 4, true>, (const void *)k_svd64<16, 8, true>,
-                              (const void *)k_svd64<16, 16, true>, (const void *)k_svd64<16, 0, true>})
+                              (const void *)k_svd64<16, 16, true>, (const void *)k_svd64<16, 0, true>,
+                              (const void *)k_svd64<32, 2, true>, (const void *)k_svd64<32, 4, true>,
+                              (const void *)k_svd64<32, 8, true>, (const void *)k_svd64<32, 0, true>})
             KV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kXBytes));
         int ok = 1;
         for (const void *k : ks) {
@@ -656,7 +672,12 @@ void svd_fp64(const SvdPlan &P, const double2 *T, double2 *U, double *S, int *st
                                    max_sweeps, tol));
     };
     // a column's elements stay in registers between the sums and the rotation up to 256 rows
-    if (C == 1) {
+    if (C == 1 && wide) {
+        if (max_p <= 64) launch(k_svd64<32, 2, true>);
+        else if (max_p <= 128) launch(k_svd64<32, 4, true>);
+        else if (max_p <= 256) launch(k_svd64<32, 8, true>);
+        else launch(k_svd64<32, 0, true>);
+    } else if (C == 1) {
         if (max_p <= 64) launch(k_svd64<16, 4, true>);
         else if (max_p <= 128) launch(k_svd64<16, 8, true>);
         else if (max_p <= 256) launch(k_svd64<16, 16, true>);
