@@ -373,8 +373,8 @@ MixPlanFull plan_mix(const Meta &lm, const Meta &W, int lead, const std::vector<
             R.term_coef[at] = f.coef;
         }
     }
-    const int64_t share = R.out.nelem / (32 * std::max(1, ctx().num_sms));
-    R.mix.chunk = (int)std::max<int64_t>(min_chunk, std::min<int64_t>(kMixChunkMax, share / 32 * 32));
+    const int64_t share = R.out.nelem / (24 * std::max(1, ctx().num_sms));
+    R.mix.chunk = (int)std::max<int64_t>(min_chunk, std::min<int64_t>(kMixChunkMax, (share + 63) / 64 * 64));
     for (size_t b = 0; b < nout; ++b) {
         MixJob j;
         j.out_off = R.out.blocks[b].off;

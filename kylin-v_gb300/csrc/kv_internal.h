@@ -453,10 +453,11 @@ struct MixJob {
     int term_begin, term_end;
 };
 // Output elements of one job handled by one warp of the mixing kernel: so that
-// the plan's elements make about 32 items an SM, within these bounds
+// the plan's elements make about 24 items an SM (three CTAs of eight warps: one
+// wave), within these bounds
 // (kMixChunkCoarse: the least where the item list's size is part of a scratch
 // bound).
-constexpr int kMixChunk = 64, kMixChunkCoarse = 256, kMixChunkMax = 2048;
+constexpr int kMixChunk = 64, kMixChunkCoarse = 256, kMixChunkMax = 4096;
 struct MixItem {  // a chunk of one job handled by one warp
     int job;
     int64_t start;

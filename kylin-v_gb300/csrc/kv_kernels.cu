@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 1024 / NT) k_gemm_fp64(cons
 // For finite inputs the sums equal the four-multiply-add product's over all
 // entries up to the sign of a zero.
 // Measured (us a launch, against one thread an element over all entries): D =
-// 128 two-site blocks 35.6 -> 23.8, D = 512 213 -> 79.
+// 128 two-site blocks 35.6 -> 16.4, D = 512 213 -> 76.
 constexpr int kMixWarps = 8;    // warps (items) per CTA
 constexpr int kMixTerms = 16;   // terms, outputs (k2, r) and nonzero entries a warp's list holds;
 constexpr int kMixOuts = 16;    // larger jobs take mix_direct
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
         return;
     }
     const unsigned rest = (unsigned)jb.rest, no = (unsigned)nout, ee = (unsigned)e1;
-    if (rest >= 32) {  // row by row: each entry is read once for up to 4 elements a lane
+    if (rest > 64) {  // row by row: each entry is read once for up to 4 elements a lane
         for (unsigned e = (unsigned)it.start; e < ee;) {
             const unsigned row = e / rest, n0 = e - row * rest, k = row / no, o = row - k * no;
             const unsigned len = min(min(rest - n0, ee - e), 128u);
@@ -306,6 +306,46 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
             for (int j = 0; j < 4; ++j)
                 if (lane + 32 * j < len) y[lane + 32 * j] = acc[j];
             e += len;
+        }
+        return;
+    }
+    if (rest > 16) {  // two rows at a time, up to 64 elements of each: four loads in flight a lane
+        const unsigned r1 = (ee - 1) / rest;
+        for (unsigned row = (unsigned)it.start / rest; row <= r1; row += 2) {
+            unsigned k[2];
+            int i0[2], cnt[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                k[u] = (row + u) / no;
+                const unsigned o = row + u - k[u] * no;
+                i0[u] = mw.start[o];
+                cnt[u] = row + u <= r1 ? mw.start[o + 1] - i0[u] : 0;
+            }
+            double2 acc[2][2] = {};
+            const int most = max(cnt[0], cnt[1]);
+            for (int t = 0; t < most; ++t) {
+                double2 v[2][2] = {};
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (t < cnt[u]) {
+                        const double2 *x = in + mw.list[i0[u] + t].off + (int64_t)k[u] * mw.list[i0[u] + t].kst;
+                        if (lane < rest) v[u][0] = x[lane];
+                        if (lane + 32 < rest) v[u][1] = x[lane + 32];
+                    }
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (t < cnt[u]) {
+                        mix_add(acc[u][0], mw.list[i0[u] + t], v[u][0], t == 0);
+                        if (rest > 32) mix_add(acc[u][1], mw.list[i0[u] + t], v[u][1], t == 0);
+                    }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const unsigned n = lane + 32 * j, e = (row + u) * rest + n;
+                    if (n < rest && e >= (unsigned)it.start && e < ee) out[jb.out_off + e] = acc[u][j];
+                }
         }
         return;
     }
