@@ -588,7 +588,7 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
 // sector holding Inf or NaN.  alph, piv: [min(p, q)]; done: [p].  512 threads.
 __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__restrict__ T64, float2 *sw, int ldw,
                                           float2 *alph, int *piv, int *done, float qr_floor, double *up,
-                                          float *fro2_out) {
+                                          float *fro2_out, int C, int rank, float2 *rows) {
     constexpr int NT = 512, NW = NT / 32;
     constexpr int GQ = 16;  // lanes per row (two rows at a time)
     __shared__ float wbest[2][NW];
@@ -661,12 +661,19 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
     const float thr2 = qr_floor * qr_floor * fro2;
     *fro2_out = fro2;
 
-    // ---- pivoted Householder on the rows
+    // ---- pivoted Householder on the rows: CTA `rank` of C updates rows rank,
+    // rank + C, ...  After a step each CTA sends its best candidate row and norm
+    // to all (slots of rows: [2][C][q]), so every CTA picks the same next pivot
+    // row and has it at hand; rows' arithmetic does not depend on who does it.
+    __shared__ float cbest[2][8];
+    __shared__ int cbesti[2][8];
+    if (C > 1) cooperative_groups::this_cluster().sync();  // every CTA runs before one stores to it
     int r = 0;
     for (int k = 0; k < kmax; ++k) {
         const int cur = k & 1;
-        float mv = lane < NW ? wbest[cur][lane] : -1.f;
-        int mi = lane < NW ? wbesti[cur][lane] : 0x7FFFFFFF;
+        const bool sent = C > 1 && k > 0;  // the candidates came from every CTA
+        float mv = sent ? (lane < C ? cbest[cur][lane] : -1.f) : lane < NW ? wbest[cur][lane] : -1.f;
+        int mi = sent ? (lane < C ? cbesti[cur][lane] : 0x7FFFFFFF) : lane < NW ? wbesti[cur][lane] : 0x7FFFFFFF;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const float ov = __shfl_xor_sync(0xFFFFFFFFu, mv, o);
@@ -676,7 +683,7 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
         if (!(mv > thr2) || mi >= p) break;  // uniform: every warp computed the same maximum
         r = k + 1;
         const int ip = mi;
-        const float2 *xr = sw + ip * ldw;
+        const float2 *xr = sent ? rows + ((size_t)cur * C + ip % C) * q : sw + ip * ldw;
         // u = conj(x), alpha = -e^{i phi} |u| (phi = arg u_0), v = u - alpha e_0,
         // beta = 2 / |v|^2 = 1 / (|u| (|u| + |u_0|));  x H = conj(alpha) e_0^T
         const float nu = sqrtf(mv);
@@ -692,8 +699,8 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
         }
         float gbv = -1.f;
         int gbi = 0x7FFFFFFF;
-        for (int i0 = gq; i0 < p; i0 += 2 * ngq) {
-            const int iA = i0, iB = i0 + ngq;
+        for (int l0 = gq; rank + C * l0 < p; l0 += 2 * ngq) {
+            const int iA = rank + C * l0, iB = rank + C * (l0 + ngq);
             // group-uniform: every lane of the group has the same rows
             const bool lA = iA != ip && !done[iA];
             const bool lB = iB < p && iB != ip && !done[iB];
@@ -753,6 +760,42 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
         }
         if (lane == 0) { wbest[cur ^ 1][warp] = gbv; wbesti[cur ^ 1][warp] = gbi; }
         __syncthreads();
+        if (C > 1) {
+            float mv2 = lane < NW ? wbest[cur ^ 1][lane] : -1.f;
+            int mi2 = lane < NW ? wbesti[cur ^ 1][lane] : 0x7FFFFFFF;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ov = __shfl_xor_sync(0xFFFFFFFFu, mv2, o);
+                const int oi = __shfl_xor_sync(0xFFFFFFFFu, mi2, o);
+                if (ov > mv2 || (ov == mv2 && oi < mi2)) { mv2 = ov; mi2 = oi; }
+            }
+            const int to = tid / (NT / C), e0 = tid % (NT / C);  // NT / C threads send to each CTA
+            if (mi2 < p) {
+                const uint32_t dst = cluster_addr(rows + ((size_t)(cur ^ 1) * C + rank) * q, to);
+                for (int c = k + 1 + e0; c < q; c += NT / C)
+                    st_cluster(dst + (uint32_t)(c * sizeof(float2)), sw[mi2 * ldw + c]);
+            }
+            if (e0 == 0) {
+                st_cluster(cluster_addr(&cbest[cur ^ 1][rank], to), mv2);
+                st_cluster(cluster_addr(&cbesti[cur ^ 1][rank], to), __int_as_float(mi2));
+            }
+            __syncwarp();
+            cooperative_groups::this_cluster().sync();
+        }
+    }
+    if (C > 1) {  // every CTA gets every row
+        cooperative_groups::this_cluster().sync();
+        for (int to = 0; to < C; ++to) {
+            if (to == rank) continue;
+            const uint32_t dst = cluster_addr(sw, to);
+            const int nr = (p - rank + C - 1) / C;
+            for (int e = tid; e < nr * r; e += NT) {
+                const int at = (rank + C * (e / r)) * ldw + e % r;
+                st_cluster(dst + (uint32_t)(at * sizeof(float2)), sw[at]);
+            }
+        }
+        __syncwarp();
+        cooperative_groups::this_cluster().sync();
     }
     // pivot rows: conj(alpha_k) at position k, zeros after it (within the r columns kept)
     for (int e = tid; e < r * r; e += NT) {
@@ -763,9 +806,9 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
     return r;
 }
 
-// The launch gives each sector a cluster of CTAs: every one reduces its own copy
-// of the sector (the same bits), then the register-resident Jacobi's groups are
-// dealt over them; the streamed form runs on the first alone.  slots, bufs: the
+// The launch gives each sector a cluster of CTAs: each holds the sector, the
+// reduction's row updates are dealt over them (qrj_reduce), then the
+// register-resident Jacobi's groups; the streamed form runs on the first alone.  slots, bufs: the
 // exchange columns per CTA and buffers of them (slots = 0: no register form).
 template <int EPL>
 __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict__ secs,
@@ -791,7 +834,15 @@ __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict_
 
     double up = 1.0;
     float fro2 = 0.f;
-    const int r = qrj_reduce(s, T64, sw, ldw, alph, piv, done, qr_floor, &up, &fro2);
+    // The reduction's candidate rows use the exchange columns' memory; where they
+    // do not fit every CTA reduces the whole sector alone.  A step's row updates
+    // bound one SM more than the cluster barrier that dealing them adds: the split
+    // of 17 sectors of 128 x 128 takes 1651 us with every CTA reducing alone, 1580
+    // with the rows dealt (1587 if only sectors of more than 64 rows are).
+    const bool deal = C > 1 && slots > 0 &&
+                      (size_t)2 * C * q * sizeof(float2) <= qrj_xch_bytes(8 * (EPL > 0 ? EPL : 1), slots, bufs);
+    const int r = qrj_reduce(s, T64, sw, ldw, alph, piv, done, qr_floor, &up, &fro2, deal ? C : 1, deal ? rank : 0,
+                             reinterpret_cast<float2 *>(xch));
     if (r < 0) {  // a non-finite sector: its singular values are NaN (reported by the host)
         if (rank != 0) return;
         for (int j = tid; j < q; j += NT) S[s.s_off + j] = nan("");
@@ -894,7 +945,7 @@ __global__ void __launch_bounds__(512, 1) k_svd_qr_g(const SvdSector *__restrict
     int *done = piv + kmax;
     double up = 1.0;
     float fro2 = 0.f;
-    const int r = qrj_reduce(s, T64, sw, ldw, alph, piv, done, qr_floor, &up, &fro2);
+    const int r = qrj_reduce(s, T64, sw, ldw, alph, piv, done, qr_floor, &up, &fro2, 1, 0, nullptr);
     float2 *out = T32 + s.t_off;
     const int64_t pq = (int64_t)p * q;
     if (r < 0) {
@@ -1320,7 +1371,8 @@ bool svd_qrjacobi_f32(const SvdPlan &p, const double2 *T64, float2 *Us, double *
     // cluster of CTAs a sector: a round's rotations and column moves bound one
     // SM, and a bond's sectors leave most SMs idle.  Measured, the whole split of
     // 17 sectors of 128 x 128: one CTA 1985 us, two 1727, four 1631, eight 1799 (a
-    // larger cluster's barrier costs more than its shorter round saves).
+    // larger cluster's barrier costs more than its shorter round saves); four
+    // reach 1580 with the reduction's rows dealt as well.
     const int nsec = (int)p.secs.size(), sms = ctx().num_sms;
     const int rows = max_p <= 32 ? 32 : max_p <= 64 ? 64 : 128;  // 8 EPL of the kernel launched below
     int C = 1, slots = 0, bufs = 1;
