@@ -391,7 +391,7 @@ struct SegX {
 struct TcTile {
     int rows;                // rows of the A packs (a multiple of 8)
     int seg_begin, seg_end;
-    int rowmap, colmap;      // 128 and 32 entries (piece, row or column of its block; piece -1: padding)
+    int rowmap, colmap;      // rows and 32 entries (piece, row or column of its block; piece -1: padding)
     int pair, ncol;          // output of (row piece i, column piece j): pairs[pair + i * ncol + j]
 };
 struct TcPair {

@@ -689,7 +689,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_gemm_tc(const TcTile *__restric
             const int nseg = t.seg_end - t.seg_begin;
             // where this thread's row and the warp's 8 columns go (pieces start at
             // multiples of 8, so the columns belong to one): read ahead of the drain
-            const int2 rm = maps[t.rowmap + m];  // (row piece, row of its block)
+            // (row piece, row of its block)
+            const int2 rm = m < t.rows ? maps[t.rowmap + m] : make_int2(-1, 0);
             const int2 cm = maps[t.colmap + c_lo + (lane & (EPI_COLS - 1))];
             const int ncol = __popc(__ballot_sync(0xFFFFFFFFu, lane < EPI_COLS && cm.x >= 0));
             const int cpiece = __shfl_sync(0xFFFFFFFFu, cm.x, 0), col0 = __shfl_sync(0xFFFFFFFFu, cm.y, 0);
@@ -827,69 +828,147 @@ int *device_err_word(int dev) {
 namespace {
 
 struct Pack {
-    std::vector<std::array<int, 3>> pieces;  // view, first row, rows
-    int rows = 0;                            // with every piece padded to a multiple of 8
+    int begin, end;  // its pieces of the list that it was made in
+    int rows;        // with every piece padded to a multiple of 8
+};
+struct Piece {
+    int view, r0, rows, unit;  // rows r0.. of a view; unit: the view's index in the list packed
 };
 
 int pad8(int n) { return (n + 7) & ~7; }
 
-// rows of the views in order, cut into packs of at most `most` rows; unit[p] = index of each piece's view in `views`
+// rows of the views in order, cut into packs of at most `most` rows
 void make_packs(const std::vector<int> &views, const std::vector<int> &view_rows, int most, std::vector<Pack> *packs,
-                std::vector<std::vector<int>> *unit) {
-    Pack cur;
-    std::vector<int> cu;
+                std::vector<Piece> *pieces) {
+    packs->clear();
+    pieces->clear();
+    Pack cur{0, 0, 0};
     auto flush = [&] {
-        if (cur.pieces.empty()) return;
-        packs->push_back(cur);
-        unit->push_back(cu);
-        cur = Pack{};
-        cu.clear();
+        cur.end = (int)pieces->size();
+        if (cur.end > cur.begin) packs->push_back(cur);
+        cur = Pack{cur.end, cur.end, 0};
     };
     for (size_t u = 0; u < views.size(); ++u)
         for (int r = 0; r < view_rows[u];) {
             if (cur.rows == most) flush();
             const int n = std::min(view_rows[u] - r, most - cur.rows);
-            cur.pieces.push_back({views[u], r, n});
-            cu.push_back((int)u);
+            pieces->push_back({views[u], r, n, (int)u});
             cur.rows += pad8(n);
             r += n;
         }
     flush();
 }
 
+struct View {
+    int64_t key, off;
+    int rows, K, ld, trans, conj, ks;
+};
+struct OutBlock {
+    int64_t c_off;
+    int ldc, M, N, sb, se;
+};
+struct Group {
+    std::vector<int> rblk;   // row units: A views (one segment) or blocks (several)
+    std::vector<int> cview;  // column units: B views (one segment); several: (view, entry) of each segment
+    uint64_t hash;           // of cview
+    bool multi;
+};
+struct Panel {
+    int64_t pan;
+    int exp;
+    int job0, njobs;
+};
+// ids by 64-bit key, open addressing
+struct IdTable {
+    std::vector<int> slot;
+    size_t mask = 0;
+    void reset(size_t n) {
+        size_t m = 16;
+        while (m < 2 * n) m *= 2;
+        slot.assign(m, -1);
+        mask = m - 1;
+    }
+    // the slot of the id for which same(id) holds, or a free one (-1)
+    template <class F>
+    int &find(uint64_t key, F same) {
+        uint64_t h = key * 0x9E3779B97F4A7C15ull;
+        h ^= h >> 32;
+        for (size_t i = h & mask;; i = (i + 1) & mask)
+            if (slot[i] < 0 || same(slot[i])) return slot[i];
+    }
+};
+// The planner's lists, kept by each thread: operations outside the sweep plan on
+// every call, and lists grown afresh (page faults of memory that the allocator
+// had given back), a node per view and group, and maps of 128 rows for short
+// packs took 28 + 69 us of an environment update of 64 + 94 block pairs at
+// D = 128, which went from 185 to 125 us without them.  A plan larger than
+// kScratchBytes leaves nothing behind.
+constexpr size_t kScratchBytes = 4 << 20;
+struct Scratch {
+    std::vector<View> av, bv;
+    std::vector<OutBlock> blocks;
+    std::vector<int> sa, sb, zero_blocks, first, of, fill, key, rows, cols, rmap, cmap, bfirst;
+    std::vector<Group> groups;
+    size_t ngroups = 0;  // of groups in use (the others keep their lists' memory)
+    IdTable atab, btab, gtab;
+    std::vector<SliceJob> ajobs, bjobs;
+    std::vector<SegX> xsegs;
+    std::vector<TcTile> tiles;
+    std::vector<TcPair> pairs;
+    std::vector<int2> maps, aitems, bitems;
+    std::vector<Pack> rp, cp;
+    std::vector<Piece> rpc, cpc;
+    std::vector<Panel> ap, bp, bpanels;
+    void clear() {
+        av.clear(), bv.clear(), blocks.clear(), zero_blocks.clear(), bpanels.clear();
+        ajobs.clear(), bjobs.clear(), xsegs.clear(), tiles.clear(), pairs.clear(), maps.clear();
+        aitems.clear(), bitems.clear();
+        ngroups = 0;
+    }
+    size_t bytes() const {
+        return maps.size() * sizeof(int2) + pairs.size() * sizeof(TcPair) + tiles.size() * sizeof(TcTile) +
+               xsegs.size() * sizeof(SegX) + (ajobs.size() + bjobs.size()) * sizeof(SliceJob) +
+               (aitems.size() + bitems.size()) * sizeof(int2) + (sa.size() + blocks.size()) * 64;
+    }
+};
+
 }  // namespace
 
 void plan_mixed(GemmPlan &g) {
-    struct View {
-        int64_t off;
-        int rows, K, ld, trans, conj, ks = -1;
-    };
-    std::vector<View> av, bv;
-    std::unordered_map<int64_t, int> amap, bmap;
-    struct Block {
-        int64_t c_off;
-        int ldc, M, N, sb, se;
-    };
-    std::vector<Block> blocks;
+    thread_local Scratch kept;
+    Scratch &w = kept;
+    w.clear();
+    auto &av = w.av;
+    auto &bv = w.bv;
+    auto &blocks = w.blocks;
+    auto &sa = w.sa, &sb = w.sb;  // views of each segment
+    auto &groups = w.groups;
+    auto &zero_blocks = w.zero_blocks;
     for (auto &t : g.tiles)
         if (t.m0 == 0 && t.n0 == 0) blocks.push_back({t.c_off, t.ldc, t.M, t.N, t.seg_begin, t.seg_end});
     // ---- views: one per distinct (block offset, operation) of each operand
-    std::vector<int> sa(g.segs.size(), -1), sb(g.segs.size(), -1);  // views of each segment
-    amap.reserve(2 * g.segs.size());
-    bmap.reserve(2 * g.segs.size());
+    sa.assign(g.segs.size(), -1);
+    sb.assign(g.segs.size(), -1);
+    w.atab.reset(g.segs.size());
+    w.btab.reset(g.segs.size());
     for (auto &b : blocks)
         for (int s = b.sb; s < b.se; ++s) {
             const GemmSeg &sg = g.segs[s];
-            auto ia = amap.emplace(sg.a_off * 4 + sg.opa, (int)av.size());
-            if (ia.second)
-                av.push_back({sg.a_off, b.M, sg.K, sg.lda, (sg.opa == 1 || sg.opa == 2) ? 1 : 0,
-                              (sg.opa == 1 || sg.opa == 3) ? 1 : 0});
-            auto ib = bmap.emplace(sg.b_off * 4 + sg.opb, (int)bv.size());
-            if (ib.second)  // B element (n, k) at b[k*ldb + n] for opb 0 and 3
-                bv.push_back({sg.b_off, b.N, sg.K, sg.ldb, (sg.opb == 0 || sg.opb == 3) ? 1 : 0,
-                              (sg.opb == 2 || sg.opb == 3) ? 1 : 0});
-            sa[s] = ia.first->second;
-            sb[s] = ib.first->second;
+            const int64_t ka = sg.a_off * 4 + sg.opa, kb = sg.b_off * 4 + sg.opb;
+            int &ia = w.atab.find((uint64_t)ka, [&](int i) { return av[i].key == ka; });
+            if (ia < 0) {
+                ia = (int)av.size();
+                av.push_back({ka, sg.a_off, b.M, sg.K, sg.lda, (sg.opa == 1 || sg.opa == 2) ? 1 : 0,
+                              (sg.opa == 1 || sg.opa == 3) ? 1 : 0, -1});
+            }
+            int &ib = w.btab.find((uint64_t)kb, [&](int i) { return bv[i].key == kb; });
+            if (ib < 0) {  // B element (n, k) at b[k*ldb + n] for opb 0 and 3
+                ib = (int)bv.size();
+                bv.push_back({kb, sg.b_off, b.N, sg.K, sg.ldb, (sg.opb == 0 || sg.opb == 3) ? 1 : 0,
+                              (sg.opb == 2 || sg.opb == 3) ? 1 : 0, -1});
+            }
+            sa[s] = ia;
+            sb[s] = ib;
             KV_REQUIRE(av[sa[s]].rows == b.M && bv[sb[s]].rows == b.N && av[sa[s]].K == sg.K && bv[sb[s]].K == sg.K,
                        KV_EINVAL, "internal: inconsistent block views in a mixed-precision plan");
         }
@@ -926,60 +1005,55 @@ void plan_mixed(GemmPlan &g) {
         KV_REQUIRE(g.k_scales < (1ll << 31), KV_EINVAL, "mixed-precision plan too large");
     }
     // ---- groups
-    struct Group {
-        std::vector<int> rblk;                // row units: A views (one segment) or blocks (several)
-        std::vector<int> cview;               // column units: B views (one segment); several: the views per segment
-        std::vector<int> grid;                // one segment: block of (row unit, column unit)
-        bool multi;
-    };
-    std::vector<Group> groups;
-    std::vector<int> zero_blocks;
+    auto &first = w.first, &of = w.of, &key = w.key;
     {
-        struct Hash {
-            size_t operator()(const std::vector<int> &v) const {
-                uint64_t h = 1469598103934665603ull;
-                for (int x : v) { h ^= (uint64_t)(uint32_t)x; h *= 1099511628211ull; }
-                return (size_t)h;
+        w.gtab.reset(blocks.size());
+        auto group_of = [&](bool multi) -> Group & {  // the group of `key`, a new one if there is none
+            uint64_t h = multi ? 1469598103934665603ull : 0xCBF29CE484222325ull + 2;
+            for (int x : key) { h ^= (uint64_t)(uint32_t)x; h *= 1099511628211ull; }
+            int &at = w.gtab.find(h, [&](int i) {
+                return groups[i].hash == h && groups[i].multi == multi && groups[i].cview == key;
+            });
+            if (at < 0) {
+                at = (int)w.ngroups++;
+                if (groups.size() < w.ngroups) groups.emplace_back();
+                Group &gr = groups[at];
+                gr.rblk.clear();
+                gr.cview = key;
+                gr.hash = h;
+                gr.multi = multi;
             }
+            return groups[at];
         };
-        std::unordered_map<std::vector<int>, int, Hash> single, multi;
-        std::vector<std::vector<int>> alist(av.size());  // one-segment blocks of each A view, in block order
+        // one-segment blocks by A view, in block order
+        first.assign(av.size() + 1, 0);
+        for (auto &b : blocks)
+            if (b.se - b.sb == 1) ++first[sa[b.sb] + 1];
+        for (size_t a = 0; a < av.size(); ++a) first[a + 1] += first[a];
+        of.resize(first[av.size()]);
+        w.fill.assign(first.begin(), first.end() - 1);
         for (size_t b = 0; b < blocks.size(); ++b) {
             const int n = blocks[b].se - blocks[b].sb;
             if (n == 0) zero_blocks.push_back((int)b);
-            else if (n == 1) alist[sa[blocks[b].sb]].push_back((int)b);
+            else if (n == 1) of[w.fill[sa[blocks[b].sb]]++] = (int)b;
             else {
-                std::vector<int> key;
+                key.clear();
                 for (int s = blocks[b].sb; s < blocks[b].se; ++s) {
                     key.push_back(sb[s]);
                     key.push_back(g.segs[s].entry);
                 }
-                auto it = multi.emplace(key, (int)groups.size());
-                if (it.second) {
-                    Group gr;
-                    gr.multi = true;
-                    for (int s = blocks[b].sb; s < blocks[b].se; ++s) gr.cview.push_back(sb[s]);
-                    groups.push_back(gr);
-                }
-                groups[it.first->second].rblk.push_back((int)b);
+                group_of(true).rblk.push_back((int)b);
             }
         }
         for (size_t a = 0; a < av.size(); ++a) {
-            if (alist[a].empty()) continue;
-            std::vector<int> key;
-            for (int b : alist[a]) key.push_back(sb[blocks[b].sb]);
-            auto it = single.emplace(key, (int)groups.size());
-            if (it.second) {
-                Group gr;
-                gr.multi = false;
-                gr.cview = key;
-                groups.push_back(gr);
-            }
-            Group &gr = groups[it.first->second];
-            gr.rblk.push_back((int)a);
-            gr.grid.insert(gr.grid.end(), alist[a].begin(), alist[a].end());
+            if (first[a] == first[a + 1]) continue;
+            key.clear();
+            for (int x = first[a]; x < first[a + 1]; ++x) key.push_back(sb[blocks[of[x]].sb]);
+            group_of(false).rblk.push_back((int)a);
         }
     }
+    // the block of (row unit u, column unit v) of a one-segment group
+    auto cell = [&](const Group &gr, int u, int v) -> const OutBlock & { return blocks[of[first[gr.rblk[u]] + v]]; };
     // ---- rows per tile: estimated clocks of the busiest SM.  A K panel costs
     // its operand bytes at about 45 B per clock or the MMAs' shared-memory
     // reads, a drain about 1800 clocks, a tile 600 more (measured on GB300).
@@ -1001,8 +1075,10 @@ void plan_mixed(GemmPlan &g) {
         for (int R : {128, 64, 32}) {
             const double panel = std::max(800.0, (R + BN) * NPL * BKC * 2 / 45.0);
             double sum = 0.0, top = 0.0, n = 0.0;
-            for (auto &gr : groups) {
-                const int s0 = gr.multi ? blocks[gr.rblk[0]].sb : blocks[gr.grid[0]].sb, ns = gr.multi ? (int)gr.cview.size() : 1;
+            for (size_t x = 0; x < w.ngroups; ++x) {
+                const Group &gr = groups[x];
+                const int s0 = gr.multi ? blocks[gr.rblk[0]].sb : cell(gr, 0, 0).sb;
+                const int ns = gr.multi ? (int)gr.cview.size() / 2 : 1;
                 double cost = 600.0;
                 for (int s = s0; s < s0 + ns; ++s) {
                     const int nkc = (g.segs[s].K + BKC - 1) / BKC;
@@ -1021,147 +1097,154 @@ void plan_mixed(GemmPlan &g) {
         }
     }
     // ---- packs (shared where the same pieces recur), tiles, maps, pairs
-    std::vector<SliceJob> ajobs, bjobs;
-    std::vector<SegX> xsegs;
-    std::vector<TcTile> tiles;
-    std::vector<TcPair> pairs;
-    std::vector<int2> maps;
+    auto &ajobs = w.ajobs, &bjobs = w.bjobs;
+    auto &xsegs = w.xsegs;
+    auto &tiles = w.tiles;
+    auto &pairs = w.pairs;
+    auto &maps = w.maps;
     g.a_planes = g.b_planes = g.a_exps = g.b_exps = 0;
-    struct Panel {
-        int64_t pan;
-        int exp;
-        int job0, njobs;
-    };
-    std::unordered_map<int64_t, Panel> bpanels;  // single-piece B packs by (view, first column)
-    auto add_pack = [&](const Pack &p, bool is_b) {
+    w.bfirst.assign(bv.size(), -1);  // single-piece B packs of each view in bpanels, by first column / BN
+    // rows of a pack's panel from its pieces; view_of: the view of a piece
+    auto add_pack = [&](const Piece *pc, const Piece *pe, int tall, bool is_b, auto view_of) {
         Panel o;
         const std::vector<View> &vw = is_b ? bv : av;
         std::vector<SliceJob> &jobs = is_b ? bjobs : ajobs;
-        const int tr = is_b ? BN : p.rows, K = vw[p.pieces[0][0]].K, nkc = (K + BKC - 1) / BKC;
+        const int tr = is_b ? BN : tall, K = vw[view_of(*pc)].K, nkc = (K + BKC - 1) / BKC;
         o.pan = is_b ? g.b_planes : g.a_planes;
         o.exp = (int)(is_b ? g.b_exps : g.a_exps);
         o.job0 = (int)jobs.size();
+        o.njobs = (int)(pe - pc);
         int r0 = 0;
-        for (auto &pc : p.pieces) {
-            const View &v = vw[pc[0]];
+        for (; pc != pe; ++pc) {
+            const View &v = vw[view_of(*pc)];
             KV_REQUIRE(v.K == K, KV_EINVAL, "internal: a pack's views differ in K");
-            jobs.push_back(SliceJob{v.off, o.pan, pc[1], pc[2], r0, tr, v.K, v.ld, v.trans, v.conj, o.exp + r0, nkc,
+            jobs.push_back(SliceJob{v.off, o.pan, pc->r0, pc->rows, r0, tr, v.K, v.ld, v.trans, v.conj, o.exp + r0, nkc,
                                     kAllSteps, v.ks});
-            r0 += pad8(pc[2]);
+            r0 += pad8(pc->rows);
         }
-        o.njobs = (int)jobs.size() - o.job0;
         (is_b ? g.b_planes : g.a_planes) += (int64_t)nkc * NPL * BKC * tr;
         (is_b ? g.b_exps : g.a_exps) += is_b ? BN : BM;
         return o;
     };
+    auto own_view = [](const Piece &pc) { return pc.view; };
     // a pair reads the pack's piece from step `entry` on (before that its block
     // may not hold data yet)
     auto seen = [&](const Panel &p, bool is_b, int piece, int entry) {
         SliceJob &j = (is_b ? bjobs : ajobs)[p.job0 + piece];
         j.entry = std::min(j.entry, entry);
     };
-    auto add_map = [&](const Pack &p, int n) {  // (piece, row) of each of n panel rows
+    auto add_map = [&](const Piece *pc, const Piece *pe, int n) {  // (piece, row) of each of n panel rows
         const int at = (int)maps.size();
-        for (size_t i = 0; i < p.pieces.size(); ++i) {
-            for (int r = 0; r < p.pieces[i][2]; ++r) maps.push_back(make_int2((int)i, p.pieces[i][1] + r));
-            for (int r = p.pieces[i][2]; r < pad8(p.pieces[i][2]); ++r) maps.push_back(make_int2(-1, 0));
+        maps.resize((size_t)at + n, make_int2(-1, 0));
+        int r0 = at;
+        for (int i = 0; pc != pe; ++i, ++pc) {
+            for (int r = 0; r < pc->rows; ++r) maps[r0 + r] = make_int2(i, pc->r0 + r);
+            r0 += pad8(pc->rows);
         }
-        while ((int)maps.size() < at + n) maps.push_back(make_int2(-1, 0));
         return at;
     };
-    for (auto &gr : groups) {
-        std::vector<Pack> rp, cp;
-        std::vector<std::vector<int>> ru, cu;
-        std::vector<int> rows;
+    auto &rp = w.rp, &cp = w.cp;
+    auto &rpc = w.rpc, &cpc = w.cpc;
+    auto &rows = w.rows, &cols = w.cols, &rmap = w.rmap, &cmap = w.cmap;
+    auto &ap = w.ap, &bp = w.bp;
+    for (size_t x = 0; x < w.ngroups; ++x) {
+        const Group &gr = groups[x];
+        rows.clear();
         if (!gr.multi) {
             for (int a : gr.rblk) rows.push_back(av[a].rows);
-            make_packs(gr.rblk, rows, most, &rp, &ru);
-            std::vector<int> cols;
+            make_packs(gr.rblk, rows, most, &rp, &rpc);
+            cols.clear();
             for (int v : gr.cview) cols.push_back(bv[v].rows);
-            make_packs(gr.cview, cols, BN, &cp, &cu);
-            std::vector<Panel> ap, bp;
-            std::vector<int> rmap, cmap;
-            for (auto &p : rp) { ap.push_back(add_pack(p, false)); rmap.push_back(add_map(p, BM)); }
-            for (auto &p : cp) { bp.push_back(add_pack(p, true)); cmap.push_back(add_map(p, BN)); }
-            const int nc = (int)gr.cview.size();
+            make_packs(gr.cview, cols, BN, &cp, &cpc);
+            ap.clear(), bp.clear(), rmap.clear(), cmap.clear();
+            for (auto &p : rp) {
+                ap.push_back(add_pack(rpc.data() + p.begin, rpc.data() + p.end, p.rows, false, own_view));
+                rmap.push_back(add_map(rpc.data() + p.begin, rpc.data() + p.end, p.rows));
+            }
+            for (auto &p : cp) {
+                bp.push_back(add_pack(cpc.data() + p.begin, cpc.data() + p.end, p.rows, true, own_view));
+                cmap.push_back(add_map(cpc.data() + p.begin, cpc.data() + p.end, BN));
+            }
+            const int nkc = (av[gr.rblk[0]].K + BKC - 1) / BKC;
             // kColBatch column packs meet every row pack before the next ones, so
             // the panels of the tiles in flight stay in L2 (all columns a row pack
             // at a time read B's panels from HBM once per row pack)
             constexpr size_t kColBatch = 16;
-            std::vector<std::pair<size_t, size_t>> order;
             for (size_t j0 = 0; j0 < cp.size(); j0 += kColBatch)
                 for (size_t i = 0; i < rp.size(); ++i)
-                    for (size_t j = j0; j < std::min(cp.size(), j0 + kColBatch); ++j) order.push_back({i, j});
-            for (auto [i, j] : order) {
-                TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + 1, rmap[i], cmap[j], (int)pairs.size(),
-                         (int)cp[j].pieces.size()};
-                int entry = kAllSteps;
-                for (size_t u = 0; u < ru[i].size(); ++u)
-                    for (size_t v = 0; v < cu[j].size(); ++v) {
-                        const Block &b = blocks[gr.grid[(size_t)ru[i][u] * nc + cu[j][v]]];
-                        const int e = g.segs[b.sb].entry;
-                        pairs.push_back({b.c_off, b.ldc, e});
-                        entry = std::min(entry, e);
-                        seen(ap[i], false, (int)u, e);
-                        seen(bp[j], true, (int)v, e);
+                    for (size_t j = j0; j < std::min(cp.size(), j0 + kColBatch); ++j) {
+                        TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + 1, rmap[i], cmap[j],
+                                 (int)pairs.size(), cp[j].end - cp[j].begin};
+                        int entry = kAllSteps;
+                        for (int u = rp[i].begin; u < rp[i].end; ++u)
+                            for (int v = cp[j].begin; v < cp[j].end; ++v) {
+                                const OutBlock &b = cell(gr, rpc[u].unit, cpc[v].unit);
+                                const int e = g.segs[b.sb].entry;
+                                pairs.push_back({b.c_off, b.ldc, e});
+                                entry = std::min(entry, e);
+                                seen(ap[i], false, u - rp[i].begin, e);
+                                seen(bp[j], true, v - cp[j].begin, e);
+                            }
+                        xsegs.push_back(SegX{ap[i].pan, bp[j].pan, nkc, ap[i].exp, bp[j].exp, entry});
+                        tiles.push_back(t);
                     }
-                xsegs.push_back(SegX{ap[i].pan, bp[j].pan, (av[gr.rblk[0]].K + BKC - 1) / BKC, ap[i].exp, bp[j].exp,
-                                     entry});
-                tiles.push_back(t);
-            }
             continue;
         }
         for (int b : gr.rblk) rows.push_back(blocks[b].M);
-        make_packs(gr.rblk, rows, most, &rp, &ru);  // pieces name blocks here
-        const int ns = (int)gr.cview.size(), N = bv[gr.cview[0]].rows;
+        make_packs(gr.rblk, rows, most, &rp, &rpc);  // pieces name blocks here
+        const int ns = (int)gr.cview.size() / 2, N = bv[gr.cview[0]].rows, nb = (N + BN - 1) / BN;
+        cmap.clear();
+        for (int n0 = 0; n0 < N; n0 += BN) {
+            const Piece c{0, n0, std::min(BN, N - n0), 0};
+            cmap.push_back(add_map(&c, &c + 1, BN));
+        }
         for (size_t i = 0; i < rp.size(); ++i) {
-            std::vector<Panel> ap;
-            const int rmap = add_map(rp[i], BM);
-            for (int s = 0; s < ns; ++s) {
-                Pack p = rp[i];
-                for (auto &pc : p.pieces) pc[0] = sa[blocks[pc[0]].sb + s];
-                ap.push_back(add_pack(p, false));
-            }
+            const Piece *p0 = rpc.data() + rp[i].begin, *p1 = rpc.data() + rp[i].end;
+            const int rm = add_map(p0, p1, rp[i].rows);
+            ap.clear();
+            for (int s = 0; s < ns; ++s)
+                ap.push_back(add_pack(p0, p1, rp[i].rows, false,
+                                      [&](const Piece &pc) { return sa[blocks[pc.view].sb + s]; }));
             for (int n0 = 0; n0 < N; n0 += BN) {
-                Pack c;
-                c.pieces.push_back({0, n0, std::min(BN, N - n0)});
-                TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + ns, rmap, add_map(c, BN), (int)pairs.size(),
-                         1};
+                TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + ns, rm, cmap[n0 / BN], (int)pairs.size(), 1};
                 int entry = kAllSteps;
                 for (int s = 0; s < ns; ++s) {
                     const GemmSeg &sg = g.segs[blocks[gr.rblk[0]].sb + s];
-                    const int64_t key = (int64_t)gr.cview[s] * (1 << 20) + n0 / BN;
-                    KV_REQUIRE(n0 / BN < (1 << 20), KV_EINVAL, "mixed-precision plan too large");
-                    auto it = bpanels.find(key);
-                    if (it == bpanels.end()) {
-                        c.pieces[0][0] = gr.cview[s];
-                        it = bpanels.emplace(key, add_pack(c, true)).first;
+                    const int v = gr.cview[2 * s];
+                    if (w.bfirst[v] < 0) {
+                        w.bfirst[v] = (int)w.bpanels.size();
+                        w.bpanels.resize(w.bpanels.size() + nb, Panel{0, 0, 0, 0});
                     }
-                    xsegs.push_back(SegX{ap[s].pan, it->second.pan, (sg.K + BKC - 1) / BKC, ap[s].exp, it->second.exp,
-                                         sg.entry});
-                    for (int x = 0; x < ap[s].njobs; ++x) seen(ap[s], false, x, sg.entry);
-                    seen(it->second, true, 0, sg.entry);
+                    Panel &pb = w.bpanels[w.bfirst[v] + n0 / BN];
+                    if (pb.njobs == 0) {
+                        const Piece c{v, n0, std::min(BN, N - n0), 0};
+                        pb = add_pack(&c, &c + 1, BN, true, own_view);
+                    }
+                    xsegs.push_back(SegX{ap[s].pan, pb.pan, (sg.K + BKC - 1) / BKC, ap[s].exp, pb.exp, sg.entry});
+                    for (int y = 0; y < ap[s].njobs; ++y) seen(ap[s], false, y, sg.entry);
+                    seen(pb, true, 0, sg.entry);
                     entry = std::min(entry, sg.entry);
                 }
-                for (int u : ru[i]) pairs.push_back({blocks[gr.rblk[u]].c_off, blocks[gr.rblk[u]].ldc, entry});
+                for (const Piece *u = p0; u != p1; ++u) {
+                    const OutBlock &b = blocks[gr.rblk[u->unit]];
+                    pairs.push_back({b.c_off, b.ldc, entry});
+                }
                 tiles.push_back(t);
             }
         }
     }
     for (int z : zero_blocks) {  // written as zeros (or skipped) by tiles without segments
-        const Block &b = blocks[z];
+        const OutBlock &b = blocks[z];
         for (int m0 = 0; m0 < b.M; m0 += BM)
             for (int n0 = 0; n0 < b.N; n0 += BN) {
-                Pack r, c;
-                r.pieces.push_back({0, m0, std::min(BM, b.M - m0)});
-                c.pieces.push_back({0, n0, std::min(BN, b.N - n0)});
-                const int rm = add_map(r, BM), cm = add_map(c, BN);
-                tiles.push_back(TcTile{pad8(r.pieces[0][2]), (int)xsegs.size(), (int)xsegs.size(), rm, cm,
+                const Piece r{0, m0, std::min(BM, b.M - m0), 0}, c{0, n0, std::min(BN, b.N - n0), 0};
+                const int rm = add_map(&r, &r + 1, pad8(r.rows)), cm = add_map(&c, &c + 1, BN);
+                tiles.push_back(TcTile{pad8(r.rows), (int)xsegs.size(), (int)xsegs.size(), rm, cm,
                                        (int)pairs.size(), 1});
                 pairs.push_back({b.c_off, b.ldc, kAllSteps});
             }
     }
-    std::vector<int2> aitems, bitems;
+    auto &aitems = w.aitems, &bitems = w.bitems;
     for (size_t i = 0; i < ajobs.size(); ++i)
         for (int r0 = 0; r0 < ajobs[i].rows; r0 += 8) aitems.push_back({(int)i, r0});
     for (size_t i = 0; i < bjobs.size(); ++i)
@@ -1182,6 +1265,7 @@ void plan_mixed(GemmPlan &g) {
     u.add(g.d_aitems, aitems);
     u.add(g.d_bitems, bitems);
     g.d_lists = u.upload();
+    if (w.bytes() > kScratchBytes) kept = Scratch{};
 }
 
 // Per device: the cooperative slicing grid (every CTA resident at once; 0:
