@@ -60,7 +60,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <unordered_map>
 #include <utility>
 
 #include "kv_internal.h"
