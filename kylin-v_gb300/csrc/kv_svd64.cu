@@ -6,17 +6,22 @@
 // projection of the sector matrix onto them.
 //
 // One thread-block cluster per sector:
+//  0. T is scaled by the power of two that brings its largest real or imaginary
+//     part to [0.5, 1) (undone on the singular values), so that squared norms
+//     neither overflow nor underflow whatever the amplitude of the sector.
 //  1. Pivoted Householder reduction of T's rows from the right: at step k the
 //     row with the largest trailing norm is reflected onto its position k and
 //     the reflector applied to the rows not yet pivoted, so T Q = M is
 //     row-pivoted lower triangular (p x r, r <= min(p, q); r is smaller only
-//     if the remaining rows are exactly zero) and T's left vectors are M's.
+//     if the remaining rows are shorter than 1e-130 of the largest element:
+//     kNormFloor) and T's left vectors are M's.
 //     One-sided Jacobi on such a graded triangular factor converges in fewer
 //     sweeps than on T, and a wide T loses its surplus columns (Drmac and
 //     Veselic, SIAM J. Matrix Anal. Appl. 29 (2008) 1322).
 //  2. One-sided Jacobi on M's columns, round-robin pairs, one barrier a round.
 //  3. Column norms = singular values, sorted; normalised columns = vectors.
-//     Columns of norm exactly zero are completed to an orthonormal set.
+//     Columns below the floor count as zero and are completed to an orthonormal
+//     set.
 //
 // What bounds it: the FP64 unit.  GB300 issues two FP64 thread-operations per
 // clock per SM, so a warp's FP64 instruction holds its quarter of the SM for
@@ -45,6 +50,14 @@ namespace {
 
 constexpr int NT = 256, NW = NT / 32;
 constexpr int kXStage = 4096;  // longest pivot row staged in shared memory
+
+// Squared norms (of the scaled sector) that count as zero.  Above the floor every
+// quantity of a reflection or rotation is a normal FP64 number: 1 / |u|^2 <= 1e260,
+// and the inner product of two columns at the tolerance is 1e-15 * 1e-260.  The
+// squares of such inner products underflow where both columns are short
+// (kProductFloor: a b 1e-30 >= 1e-290 above it); those pairs are compared with
+// their exponents taken out.
+constexpr double kNormFloor = 1e-260, kProductFloor = 1e-130;
 
 // Data that other CTAs of the cluster read or write goes through L2; a sector of
 // one CTA (ONE) keeps it in the SM's L1.
@@ -161,6 +174,16 @@ __device__ __forceinline__ void rotation(double a, double b, double cr, double c
     si = cs * ti;
 }
 
+// |c|^2 > tol2 a b for short columns, whose products would underflow: exponents
+// apart, mantissas in FP32 (a tolerance needs no more)
+__device__ __forceinline__ bool above_tolerance(double a, double b, double cr, double ci, double tol2) {
+    int ea, eb, er, ei;
+    const float ma = mantissa(a, ea), mb = mantissa(b, eb), mr = mantissa(cr, er), mi = mantissa(ci, ei);
+    const int ec = mr == 0.f ? ei : mi == 0.f ? er : max(er, ei);
+    const float fr = mr == 0.f ? 0.f : mr * pow2f(er - ec), fi = mi == 0.f ? 0.f : mi * pow2f(ei - ec);
+    return fmaf(fr, fr, fi * fi) * pow2f(2 * ec - ea - eb) > (float)tol2 * ma * mb;
+}
+
 struct Svd64Sector {
     int64_t t_off;   // T, the row workspace and M: p * q elements each
     int64_t s_off;   // q singular values
@@ -230,6 +253,30 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         }
     };
 
+    // ---- the power of two: the largest exponent, over the cluster by way of the
+    // second candidate slot (next written after the barrier that follows its reads)
+    int shift;
+    {
+        int mx = 0;
+        const int64_t n = (int64_t)p * q;
+        for (int64_t e = (int64_t)rank * NT + tid; e < n; e += (int64_t)C * NT) {
+            const double2 v = t[e];
+            mx = max(mx, max(__double2hiint(v.x) & 0x7FFFFFFF, __double2hiint(v.y) & 0x7FFFFFFF));
+        }
+        mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+        if (lane == 0) wi[warp] = mx;
+        __syncthreads();
+        if (tid == 0) {
+            for (int x = 1; x < NW; ++x) mx = max(mx, wi[x]);
+            stg<ONE>(ONE ? &own[1].row : &cd[16 + rank].row, mx);
+        }
+        sync();
+        mx = 0;
+        for (int x = 0; x < C; ++x) mx = max(mx, ldg<ONE>(ONE ? &own[1].row : &cd[16 + x].row));
+        const int E = mx >> 20;
+        shift = E == 0x7FF ? 0 : 1022 - max(E, 1);  // a non-finite sector is found by its row norms
+    }
+
     // ---- rows i = rank, rank + C, ... belong to this CTA.  A group of lanes takes
     // a row, as many as the row's length keeps busy: a warp's FP64 instruction
     // costs the same for idle lanes.
@@ -238,12 +285,15 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         double bv = -1.0;
         int bi = 0x7FFFFFFF, bad = 0;
         const int GQ = lanes_for(q), RW = 32 / GQ, sub = lane / GQ, gl = lane % GQ;
+        const double up = scalbn(1.0, shift);  // 2^-1024 ... 2^1021: the products are exact
         for (int base = warp * RW; rank + C * base < p; base += NW * RW) {  // warp-uniform
             const int i = rank + C * (base + sub);
             double a = 0.0;
             if (i < p)
                 for (int c = gl; c < q; c += GQ) {
-                    const double2 v = t[i + (int64_t)c * p];
+                    double2 v = t[i + (int64_t)c * p];
+                    v.x *= up;
+                    v.y *= up;
                     w[(int64_t)i * q + c] = v;
                     a = fma(v.x, v.x, fma(v.y, v.y, a));
                 }
@@ -274,7 +324,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
             if (v > mv || (v == mv && i < ip)) { mv = v; ip = i; }
         }
         if (bad) { nonfinite = true; break; }
-        if (k >= kmax || !(mv > 0.0) || ip >= p) break;
+        if (k >= kmax || !(mv > kNormFloor) || ip >= p) break;
         r = k + 1;
         const double2 *xr = w + (int64_t)ip * q;
         const bool staged = q <= kXStage;
@@ -423,8 +473,13 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                 }
                 group_sum4<G>(a, b, cr, ci);
                 const double ac2 = fma(cr, cr, ci * ci);
-                // |c|^2 <= tol^2 a b: the pair is orthogonal to the tolerance
-                if (!act || !(ac2 > tol2 * a * b)) continue;
+                // |c|^2 <= tol^2 a b: the pair is orthogonal to the tolerance; a column below the
+                // floor counts as zero (high words: no FP64 instruction)
+                const int lo = min(__double2hiint(a), __double2hiint(b));
+                if (!act || lo <= __double2hiint(kNormFloor)) continue;
+                if (lo > __double2hiint(kProductFloor) ? !(ac2 > tol2 * a * b)
+                                                       : !above_tolerance(a, b, cr, ci, tol2))
+                    continue;
                 double cs, sr, si;
                 rotation(a, b, cr, ci, cs, sr, si);
                 rotated = true;
@@ -471,7 +526,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
             }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
-        if (lane == 0) stg<ONE>(nv + j, sqrt(a));
+        if (lane == 0) stg<ONE>(nv + j, a > kNormFloor ? sqrt(a) : 0.0);
     }
     sync();
     int zeros = 0;  // columns of norm zero, the same in every warp
@@ -492,7 +547,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                 const double2 v = ldg2(m + (int64_t)j * p + i);
                 stg2(w + (int64_t)pos * p + i, make_double2(v.x * inv, v.y * inv));
             }
-        if (lane == 0) S[s.s_off + pos] = sj;
+        if (lane == 0) S[s.s_off + pos] = scalbn(sj, -shift);
     }
     if (rank == 0)
         for (int j = kmax + tid; j < q; j += NT) S[s.s_off + j] = 0.0;
