@@ -58,6 +58,9 @@ constexpr int kXStage = 4096;  // longest pivot row staged in shared memory
 // (kProductFloor: a b 1e-30 >= 1e-290 above it); those pairs are compared with
 // their exponents taken out.
 constexpr double kNormFloor = 1e-260, kProductFloor = 1e-130;
+// Below it |u_0|^2 gives no phase of modulus one to FP64 rounding (its squares are
+// subnormal); u_0 is then under 1e-20 of |u| and is left out of the reflector.
+constexpr double kPhaseFloor = 1e-300;
 
 // Data that other CTAs of the cluster read or write goes through L2; a sector of
 // one CTA (ONE) keeps it in the SM's L1.
@@ -335,21 +338,14 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         if (warp == 0) {
             const double2 x0 = ldg2(xr + k);
             const double n0 = fma(x0.x, x0.x, x0.y * x0.y);
-            double nu, a0, ia, beta;
-            if (mv > 1e-140 && mv < 1e140 && (n0 == 0.0 || n0 > 1e-280)) {
-                const double y = newton_rsqrt(mv);
-                nu = mv * y;
-                nu = fma(0.5 * y, fma(-nu, nu, mv), nu);
-                ia = n0 > 0.0 ? newton_rsqrt(n0) : 0.0;
-                a0 = n0 * ia;
-                beta = newton_reciprocal(nu * (nu + a0));
-            } else {
-                nu = sqrt(mv);
-                a0 = sqrt(n0);
-                ia = a0 > 0.0 ? 1.0 / a0 : 0.0;
-                beta = 1.0 / (nu * (nu + a0));
-            }
-            const double pr = a0 > 0.0 ? x0.x * ia : 1.0, pi = -x0.y * ia;  // e^{i phi}
+            const double y = newton_rsqrt(mv);
+            double nu = mv * y;
+            nu = fma(0.5 * y, fma(-nu, nu, mv), nu);
+            const bool phase = n0 > kPhaseFloor;
+            const double ia = phase ? newton_rsqrt(n0) : 0.0;
+            const double a0 = phase ? n0 * ia : 0.0;
+            const double beta = newton_reciprocal(nu * (nu + a0));
+            const double pr = phase ? x0.x * ia : 1.0, pi = phase ? -x0.y * ia : 0.0;  // e^{i phi}
             if (lane == 0) {
                 sc[0] = make_double2(pr * (a0 + nu), pi * (a0 + nu));
                 sc[1] = make_double2(beta, 0.0);

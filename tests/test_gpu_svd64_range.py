@@ -78,3 +78,16 @@ def test_a_faint_sector_beside_another(gpu, power):
     assert (kept, total) == (8, 13)
     x, y = dict(L.to_host().blocks)[(0, 0)], dict(R.to_host().blocks)[(0, 0)]
     assert np.abs(x @ y - a).max() <= 40 * 9 * EPS * np.linalg.svd(a, compute_uv=False)[0]
+
+
+@pytest.mark.parametrize("l2r", [True, False])
+@pytest.mark.parametrize("power", [-140, -149, -150, -151, -155, -158, -159, -160, -161, -161.5, -161.8, -163, -310])
+@pytest.mark.parametrize("m,n,at", [(6, 5, 0), (5, 6, 0), (20, 30, 7), (30, 20, 19), (9, 1, 0)])
+def test_faint_column(gpu, m, n, at, power, l2r):
+    """A column of entries whose squares are subnormal beside ordinary ones: the reflectors' phases."""
+    a = _random(np.random.default_rng([m, n]), m, n)
+    a[:, at] *= 10.0**power
+    if n == 1:
+        a[0, 0] = 1.0
+    _check(gpu, a, l2r)
+    _check(gpu, a.T.copy(), l2r)
