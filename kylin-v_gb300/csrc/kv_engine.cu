@@ -1296,6 +1296,7 @@ SvdOut op_svd(const DTensor &A, int r1, bool l2r, double thres, int max_dim, int
         // projection of the sector matrix onto them, S V^H = U^H A or U S = A V:
         // A[i, c] = T[i + c p] (L->R) or conj(T[c + i p]) (R->L), both
         // contiguous along the contracted index
+        svd_fp64_complete(P, sv, kfin, Us.as<double2>());
         std::vector<SvdScatter> orth;
         std::vector<SvdDense> dense;
         std::vector<int64_t> y_off(nsec, 0);

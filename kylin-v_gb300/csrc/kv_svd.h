@@ -102,9 +102,13 @@ void svd_trsm(const DevBuf &pol, const std::vector<int> &item_pol, const std::ve
               const double2 *G, double2 *X, int kmax);
 void svd_scatter_dense(const std::vector<SvdDense> &d, const double2 *M, double2 *out);
 // FP64 mode: the min(p, q) left singular vectors of every sector's T,
-// normalised and sorted (column-major p x min(p, q) at t_off), and the singular
-// values (kv_svd64.cu); status[sector] = Jacobi sweeps, negative: no convergence
+// normalised and sorted (column-major p x min(p, q) at t_off; those of singular
+// values of zero are not written), and the singular values (kv_svd64.cu);
+// status[sector] = Jacobi sweeps, negative: no convergence
 void svd_fp64(const SvdPlan &p, const double2 *T, double2 *U, double *S, int *status, int max_sweeps, double tol);
+// the first kept[sector] vectors of every sector, where their singular values s
+// (the host's copy of S) are zero: an orthonormal set with the others
+void svd_fp64_complete(const SvdPlan &p, const std::vector<double> &s, const std::vector<int> &kept, double2 *U);
 void svd_scatter(const std::vector<SvdScatter> &sc, const SvdPlan &p, const double2 *Us, double2 *out);
 // FP64 path: the kept vectors of each SA sector into B (after svd_fp64)
 void sa_basis(const std::vector<SaSector> &v, const SvdPlan &p, const double2 *Us, double2 *B);

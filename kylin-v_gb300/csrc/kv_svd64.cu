@@ -20,8 +20,9 @@
 //     Veselic, SIAM J. Matrix Anal. Appl. 29 (2008) 1322).
 //  2. One-sided Jacobi on M's columns, round-robin pairs, one barrier a round.
 //  3. Column norms = singular values, sorted; normalised columns = vectors.
-//     Columns below the floor count as zero and are completed to an orthonormal
-//     set.
+//     Columns below the floor count as zero, and their vectors are not written;
+//     those that a truncation keeps are completed to an orthonormal set
+//     (svd_fp64_complete).
 //
 // What bounds it: the FP64 unit.  GB300 issues two FP64 thread-operations per
 // clock per SM, so a warp's FP64 instruction holds its quarter of the SM for
@@ -525,9 +526,6 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
         if (lane == 0) stg<ONE>(nv + j, a > kNormFloor ? sqrt(a) : 0.0);
     }
     sync();
-    int zeros = 0;  // columns of norm zero, the same in every warp
-    for (int j0 = 0; j0 < kmax; j0 += 32)
-        zeros += __popc(__ballot_sync(0xFFFFFFFFu, j0 + lane < kmax && !(ldg<ONE>(nv + min(j0 + lane, kmax - 1)) > 0.0)));
     for (int j = rank + C * warp; j < kmax; j += C * NW) {
         const double sj = ldg<ONE>(nv + j);
         int pos = 0;
@@ -547,68 +545,102 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
     }
     if (rank == 0)
         for (int j = kmax + tid; j < q; j += NT) S[s.s_off + j] = 0.0;
-    if (zeros == 0) return;  // uniform over the cluster
-    sync();
-    if (rank != 0) return;
-    // ---- the last `zeros` vectors: unit vectors e_i made orthogonal (twice)
-    // to all before them, i the row those leave the most of e_i in
-    for (int j = kmax - zeros; j < kmax; ++j) {
-        double best = -1.0;
-        int bi = 0x7FFFFFFF;
-        for (int i = tid; i < p; i += NT) {
-            double a = 1.0;
-            for (int c = 0; c < j; ++c) {
-                const double2 v = ldg2(w + (int64_t)c * p + i);
-                a -= fma(v.x, v.x, v.y * v.y);
-            }
-            if (a > best) { best = a; bi = i; }
-        }
+}
+
+// Completion of a factor's orthonormal columns (svd_fp64_complete): Householder
+// reflectors H_0 ... H_{j0-1} of the j0 columns U holds, whose product Q has
+// those columns (up to phases) first; Q's columns j0 ... k-1 complete them, each
+// for itself.  Only columns that are kept are made, so it runs where a
+// truncation keeps singular values of zero (a negative cut-off, the SA split).
+// FP64 issue bounds both kernels.  Measured (the split of one 200 x 200 sector,
+// kept whole; completion vector by vector in k_svd64 before): all of it zero 132.5
+// -> 0.38 ms, half of its rows zero 110.5 -> 15.2 ms, 11.4 of it without
+// completion; nothing kept of the zero sector: 132.4 -> 0.19 ms.
+struct Fill {
+    int64_t t_off, v_off;  // U's columns; the reflectors' vectors, p x j0
+    int64_t b_off;         // j0 reflector scales
+    int p, j0;
+};
+
+__global__ void __launch_bounds__(NT) k_svd64_reflect(const Fill *__restrict__ fills, const double2 *__restrict__ U,
+                                                      double2 *V, double *beta) {
+    const Fill d = fills[blockIdx.x];
+    const int p = d.p, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double2 *v = V + d.v_off;
+    __shared__ double s_beta;
+    for (int64_t e = tid; e < (int64_t)p * d.j0; e += NT) v[e] = U[d.t_off + e];
+    __syncthreads();
+    for (int c = 0; c < d.j0; ++c) {
+        double2 *x = v + (int64_t)c * p;
+        if (warp == 0) {  // v = x - alpha e_c with alpha = -(x_c / |x_c|) |x|, beta = 2 / |v|^2
+            double a = 0.0;
+            for (int i = c + lane; i < p; i += 32) a = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, a));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-        }
-        if (lane == 0) { wv[warp] = best; wi[warp] = bi; }
-        __syncthreads();
-        for (int x = 0; x < NW; ++x)
-            if (wv[x] > best || (wv[x] == best && wi[x] < bi)) { best = wv[x]; bi = wi[x]; }
-        double2 *u = w + (int64_t)j * p;
-        for (int i = tid; i < p; i += NT) stg2(u + i, make_double2(i == bi ? 1.0 : 0.0, 0.0));
-        __syncthreads();
-        for (int pass = 0; pass < 2; ++pass)
-            for (int c = 0; c < j; ++c) {
-                double sr = 0.0, si = 0.0;  // u_c^H u, by every warp alike
-                for (int i = lane; i < p; i += 32) {
-                    const double2 a = ldg2(w + (int64_t)c * p + i), b = ldg2(u + i);
-                    sr = fma(a.x, b.x, fma(a.y, b.y, sr));
-                    si = fma(a.x, b.y, fma(-a.y, b.x, si));
-                }
-                group_sum2(sr, si, 32);
-                __syncthreads();
-                for (int i = tid; i < p; i += NT) {
-                    const double2 a = ldg2(w + (int64_t)c * p + i);
-                    double2 b = ldg2(u + i);
-                    b.x -= a.x * sr - a.y * si;
-                    b.y -= a.x * si + a.y * sr;
-                    stg2(u + i, b);
-                }
-                __syncthreads();
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+            const double2 xc = x[c];
+            const double nu = sqrt(a), n0 = fma(xc.x, xc.x, xc.y * xc.y);
+            const bool phase = n0 > kPhaseFloor;
+            const double a0 = phase ? sqrt(n0) : 0.0;
+            __syncwarp();
+            if (lane == 0) {
+                x[c] = make_double2(phase ? xc.x / a0 * (a0 + nu) : nu, phase ? xc.y / a0 * (a0 + nu) : 0.0);
+                beta[d.b_off + c] = s_beta = 1.0 / (nu * (nu + a0));
             }
-        double a = 0.0;
-        for (int i = lane; i < p; i += 32) {
-            const double2 b = ldg2(u + i);
-            a = fma(b.x, b.x, fma(b.y, b.y, a));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
-        const double inv = 1.0 / sqrt(a);
-        __syncthreads();
-        for (int i = tid; i < p; i += NT) {
-            const double2 b = ldg2(u + i);
-            stg2(u + i, make_double2(b.x * inv, b.y * inv));
         }
         __syncthreads();
+        const double b = s_beta;
+        for (int y0 = c + 1 + warp; y0 < d.j0; y0 += NW) {
+            double2 *y = v + (int64_t)y0 * p;
+            double sr = 0.0, si = 0.0;  // v^H y
+            for (int i = c + lane; i < p; i += 32) {
+                const double2 h = x[i], w = y[i];
+                sr = fma(h.x, w.x, fma(h.y, w.y, sr));
+                si = fma(h.x, w.y, fma(-h.y, w.x, si));
+            }
+            __syncwarp();
+            group_sum2(sr, si, 32);
+            sr *= b;
+            si *= b;
+            for (int i = c + lane; i < p; i += 32) {
+                const double2 h = x[i];
+                y[i].x -= h.x * sr - h.y * si;
+                y[i].y -= h.x * si + h.y * sr;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// one warp per new column: items (fill, column)
+__global__ void __launch_bounds__(NT) k_svd64_fill(const Fill *__restrict__ fills, const int2 *__restrict__ items,
+                                                   int nitems, const double2 *__restrict__ V,
+                                                   const double *__restrict__ beta, double2 *U) {
+    const int item = blockIdx.x * NW + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (item >= nitems) return;  // warp-uniform
+    const int2 it = items[item];
+    const Fill d = fills[it.x];
+    double2 *y = U + d.t_off + (int64_t)it.y * d.p;  // a lane reads only elements that it wrote
+    for (int i = lane; i < d.p; i += 32) y[i] = make_double2(i == it.y ? 1.0 : 0.0, 0.0);
+    for (int c = d.j0 - 1; c >= 0; --c) {
+        const double2 *h = V + d.v_off + (int64_t)c * d.p;
+        double sr = 0.0, si = 0.0;
+        for (int i = lane; i < d.p; i += 32) {
+            if (i < c) continue;
+            const double2 a = h[i], w = y[i];
+            sr = fma(a.x, w.x, fma(a.y, w.y, sr));
+            si = fma(a.x, w.y, fma(-a.y, w.x, si));
+        }
+        __syncwarp();
+        group_sum2(sr, si, 32);
+        const double b = beta[d.b_off + c];
+        sr *= b;
+        si *= b;
+        for (int i = lane; i < d.p; i += 32) {
+            if (i < c) continue;
+            const double2 a = h[i];
+            y[i].x -= a.x * sr - a.y * si;
+            y[i].y -= a.x * si + a.y * sr;
+        }
     }
 }
 
@@ -745,6 +777,38 @@ void svd_fp64(const SvdPlan &P, const double2 *T, double2 *U, double *S, int *st
         else launch(k_svd64<16, 0, false>);
     }
     counted();
+}
+
+void svd_fp64_complete(const SvdPlan &P, const std::vector<double> &s, const std::vector<int> &kept, double2 *U) {
+    std::vector<Fill> fills;
+    std::vector<int2> items;
+    int64_t v_elems = 0, b_elems = 0;
+    for (size_t i = 0; i < P.secs.size(); ++i) {
+        const SvdSector &sc = P.secs[i];
+        int j0 = 0;
+        while (j0 < kept[i] && s[sc.s_off + j0] > 0.0) ++j0;
+        if (j0 >= kept[i]) continue;
+        for (int j = j0; j < kept[i]; ++j) items.push_back(make_int2((int)fills.size(), j));
+        fills.push_back({sc.t_off, v_elems, b_elems, sc.p, j0});
+        v_elems += (int64_t)sc.p * j0;
+        b_elems += j0;
+    }
+    if (fills.empty()) return;
+    DevSpan df, di;
+    UploadPack u;
+    u.add(df, fills);
+    u.add(di, items);
+    DevBuf lists = u.upload();
+    DevBuf V(std::max<int64_t>(1, v_elems) * sizeof(double2)), beta(std::max<int64_t>(1, b_elems) * sizeof(double));
+    if (v_elems > 0) {
+        k_svd64_reflect<<<(unsigned)fills.size(), NT, 0, ctx().stream>>>(df.as<Fill>(), U, V.as<double2>(),
+                                                                         beta.as<double>());
+        counted();
+    }
+    k_svd64_fill<<<(unsigned)((items.size() + NW - 1) / NW), NT, 0, ctx().stream>>>(
+        df.as<Fill>(), di.as<int2>(), (int)items.size(), V.as<double2>(), beta.as<double>(), U);
+    counted();
+    KV_CUDA(cudaGetLastError());
 }
 
 }  // namespace kv

@@ -91,3 +91,43 @@ def test_faint_column(gpu, m, n, at, power, l2r):
         a[0, 0] = 1.0
     _check(gpu, a, l2r)
     _check(gpu, a.T.copy(), l2r)
+
+
+@pytest.mark.parametrize("l2r", [True, False])
+@pytest.mark.parametrize("m,n,rows", [(1, 1, 0), (5, 5, 0), (5, 9, 2), (9, 5, 4), (33, 70, 31), (70, 33, 20),
+                                      (300, 40, 39), (260, 270, 1), (100, 100, 50)])
+def test_completed_vectors(gpu, m, n, rows, l2r):
+    """All min(m, n) states kept of a sector of which only `rows` rows are not zero, and several such sectors."""
+    rng = np.random.default_rng([m, n, rows])
+    a = np.zeros((m, n), complex)
+    a[rng.permutation(m)[:rows]] = _random(rng, rows, n)
+    if not a.any():
+        k = min(m, n)
+        L, R, kept, _ = gpu.svd_impl(BlockTensor((1, -1), [((0, 0), a)]), 1, l2r, -1.0, k)
+        x, y = L.to_host().blocks[0][1], R.to_host().blocks[0][1]
+        orth, other = (x, y) if l2r else (y.conj().T, x)
+        assert kept == k and not other.any()
+        assert np.abs(orth.conj().T @ orth - np.eye(k)).max() <= 1e-14 + 40 * max(m, n) * EPS
+        return
+    _check(gpu, a, l2r)
+    _check(gpu, a.T.copy(), l2r)
+
+
+def test_dropped_vectors_cost_nothing(gpu):
+    """A sector of zeros whose states the truncation drops takes no longer than one of full rank."""
+    import time
+
+    import torch
+
+    def run(a):
+        t, best = gpu.Tensor.from_host(BlockTensor((1, -1), [((0, 0), a)])), 1e9
+        for _ in range(4):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            gpu.svd_impl(t, 1, True, 0.0, 200)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    full = run(_random(np.random.default_rng(8), 200, 200))
+    assert run(np.zeros((200, 200), complex)) <= full
