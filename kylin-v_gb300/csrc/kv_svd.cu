@@ -687,9 +687,15 @@ __device__ __forceinline__ int qrj_reduce(const SvdSector &s, const double2 *__r
         // u = conj(x), alpha = -e^{i phi} |u| (phi = arg u_0), v = u - alpha e_0,
         // beta = 2 / |v|^2 = 1 / (|u| (|u| + |u_0|));  x H = conj(alpha) e_0^T
         const float nu = sqrtf(mv);
-        const float2 x0 = xr[k];
-        const float a0 = sqrtf(x0.x * x0.x + x0.y * x0.y);
+        // |u_0| below 1e-18 (of the largest element, about one): its square is near or
+        // in the subnormals and gives a phase that is not of modulus one, so it is
+        // taken with u_0 scaled up
+        float2 x0 = xr[k];
+        const bool faint = x0.x * x0.x + x0.y * x0.y < 1e-36f;
+        if (faint) x0 = make_float2(x0.x * 0x1p100f, x0.y * 0x1p100f);
+        float a0 = sqrtf(x0.x * x0.x + x0.y * x0.y);
         const float ph_r = a0 > 0.f ? x0.x / a0 : 1.f, ph_i = a0 > 0.f ? -x0.y / a0 : 0.f;  // e^{i phi}
+        if (faint) a0 *= 0x1p-100f;
         const float2 v0 = make_float2(ph_r * (a0 + nu), ph_i * (a0 + nu));              // u_0 - alpha
         const float beta = 1.f / (nu * (nu + a0));
         if (tid == 0) {
