@@ -4,6 +4,7 @@
 #include <cmath>
 
 #include "kv_internal.h"
+#include "kv_permute.cuh"
 
 namespace kv {
 
@@ -370,63 +371,19 @@ __global__ void __launch_bounds__(32 * kMixWarps) k_mix(const MixItem *__restric
 // small blocks: 98 -> 9 us for one of 96 x 5 x 12 x 96 x 5 elements a CTA walked
 // alone.
 constexpr int kPermChunk = 1024;
+static_assert(kMaxRank == kvp::kRank, "axes of a block");
 __global__ void __launch_bounds__(256) k_permute(const int64_t *__restrict__ desc, const double2 *__restrict__ in,
                                                  double2 *__restrict__ out) {
     const int64_t *d = desc + 16 * blockIdx.x;
     const int64_t in_off = d[0], out_off = d[1], size = d[2];
     const int rank = (int)d[3];
     if ((int64_t)blockIdx.y * kPermChunk >= size) return;
-    // strides of the input's axes, and the output stride of each input axis (0 past the rank)
-    unsigned sd[kMaxRank], sh[kMaxRank];
-    int64_t od[kMaxRank];
-    bool same = true;
-    {
-        int64_t st = 1;
-#pragma unroll
-        for (int i = kMaxRank - 1; i >= 0; --i) {
-            sh[i] = i < rank ? (unsigned)d[4 + i] : 1u;
-            sd[i] = (unsigned)st;
-            od[i] = 0;
-            st *= sh[i];
-        }
-        int64_t ost = 1;
-        for (int j = rank - 1; j >= 0; --j) {
-            const int ax = (int)d[10 + j];
-            same = same && ax == j;
-#pragma unroll
-            for (int i = 0; i < kMaxRank; ++i)
-                if (i == ax) {
-                    od[i] = ost;
-                    ost *= sh[i];
-                }
-        }
-    }
+    const kvp::PermMap map = kvp::perm_map(d + 4, d + 10, rank);
     const bool wide = size >= (1ll << 31);
     for (int64_t c0 = (int64_t)blockIdx.y * kPermChunk; c0 < size; c0 += (int64_t)gridDim.y * kPermChunk) {
         const int64_t c1 = min(size, c0 + kPermChunk);
-        for (int64_t e = c0 + threadIdx.x; e < c1; e += 256) {
-            int64_t dst = e;
-            if (!same) {
-                dst = 0;
-                if (wide) {
-                    int64_t rem = e;
-                    for (int i = rank - 1; i >= 0; --i) {
-                        dst += (rem % sh[i]) * od[i];
-                        rem /= sh[i];
-                    }
-                } else {
-                    unsigned rem = (unsigned)e;
-#pragma unroll
-                    for (int i = 0; i < kMaxRank; ++i)
-                        if (i < rank) {
-                            const unsigned x = rem / sd[i];
-                            rem -= x * sd[i];
-                            dst += x * od[i];
-                        }
-                }
-            }
-            out[out_off + dst] = in[in_off + e];
-        }
+        for (int64_t e = c0 + threadIdx.x; e < c1; e += 256)
+            out[out_off + kvp::perm_index(map, rank, e, wide)] = in[in_off + e];
     }
 }
 
