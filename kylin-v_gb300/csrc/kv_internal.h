@@ -361,7 +361,9 @@ struct GemmTile {
 // block and cut by fp64_tiles when the plan is uploaded, or (task lists whose
 // size must not grow) made kFp64Coarse square, each CTA walking its tile.
 constexpr int kFp64Block = 1 << 30, kFp64Coarse = 32;
-// Tile shape of the tensor-core path (kv_tc.cu).
+// Tensor-core path (kv_tc.cu): its plans hold one entry per output block too,
+// which plan_mixed packs into tiles of this shape.
+constexpr int kMixedBlock = kFp64Block + 1;
 constexpr int kMixedTileM = 128, kMixedTileN = 32;
 
 // Tensor-core path.  An operand view is one operand block as GEMM rows x K (A:
@@ -429,7 +431,7 @@ struct GemmPlan {
     // items: (job, first of 8 rows) per slicing CTA
     DevSpan d_tctiles, d_xsegs, d_maps, d_pairs, d_ajobs, d_bjobs, d_aitems, d_bitems;
     void upload() {
-        if (tile_m == kMixedTileM && tile_n == kMixedTileN) {
+        if (tile_m == kMixedBlock) {
             plan_mixed(*this);
             return;
         }

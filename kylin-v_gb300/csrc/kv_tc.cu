@@ -807,8 +807,8 @@ int *device_err_word(int dev) {
 
 }  // namespace
 
-// Tiles, packs and slicing jobs of a tensor-core plan (GemmPlan::tiles holds the
-// output blocks; only a block's first entry, m0 = n0 = 0, is read).
+// Tiles, packs and slicing jobs of a tensor-core plan (GemmPlan::tiles holds one
+// entry per output block).
 //
 // A U(1) block-sparse product is a set of dense products cut into small blocks
 // (8 x 8 at a D = 128 bond of 17 sectors), and a 128 x 32 tile per output block
@@ -872,6 +872,9 @@ struct Group {
     uint64_t hash;           // of cview
     bool multi;
 };
+struct GroupCost {
+    int rows, col_packs, panels, drains;
+};
 struct Panel {
     int64_t pan;
     int exp;
@@ -918,6 +921,7 @@ struct Scratch {
     std::vector<Pack> rp, cp;
     std::vector<Piece> rpc, cpc;
     std::vector<Panel> ap, bp, bpanels;
+    std::vector<GroupCost> costs;
     void clear() {
         av.clear(), bv.clear(), blocks.clear(), zero_blocks.clear(), bpanels.clear();
         ajobs.clear(), bjobs.clear(), xsegs.clear(), tiles.clear(), pairs.clear(), maps.clear();
@@ -943,8 +947,7 @@ void plan_mixed(GemmPlan &g) {
     auto &sa = w.sa, &sb = w.sb;  // views of each segment
     auto &groups = w.groups;
     auto &zero_blocks = w.zero_blocks;
-    for (auto &t : g.tiles)
-        if (t.m0 == 0 && t.n0 == 0) blocks.push_back({t.c_off, t.ldc, t.M, t.N, t.seg_begin, t.seg_end});
+    for (auto &t : g.tiles) blocks.push_back({t.c_off, t.ldc, t.M, t.N, t.seg_begin, t.seg_end});
     // ---- views: one per distinct (block offset, operation) of each operand
     sa.assign(g.segs.size(), -1);
     sb.assign(g.segs.size(), -1);
@@ -1069,21 +1072,29 @@ void plan_mixed(GemmPlan &g) {
     };
     int most = BM;
     {
+        auto &gc = w.costs;
+        gc.resize(w.ngroups);
+        for (size_t x = 0; x < w.ngroups; ++x) {
+            const Group &gr = groups[x];
+            const int s0 = gr.multi ? blocks[gr.rblk[0]].sb : cell(gr, 0, 0).sb;
+            const int ns = gr.multi ? (int)gr.cview.size() / 2 : 1;
+            GroupCost c{group_rows(gr), (group_cols(gr) + BN - 1) / BN, 0, 0};
+            for (int s = s0; s < s0 + ns; ++s) {
+                const int nkc = (g.segs[s].K + BKC - 1) / BKC;
+                c.panels += nkc;
+                c.drains += (nkc + GKC - 1) / GKC;
+            }
+            gc[x] = c;
+        }
         double best = 0.0;
         const double sms = std::max(1, ctx().num_sms);
-        for (int R : {128, 64, 32}) {
+        for (int log_r : {7, 6, 5}) {
+            const int R = 1 << log_r;
             const double panel = std::max(800.0, (R + BN) * NPL * BKC * 2 / 45.0);
             double sum = 0.0, top = 0.0, n = 0.0;
-            for (size_t x = 0; x < w.ngroups; ++x) {
-                const Group &gr = groups[x];
-                const int s0 = gr.multi ? blocks[gr.rblk[0]].sb : cell(gr, 0, 0).sb;
-                const int ns = gr.multi ? (int)gr.cview.size() / 2 : 1;
-                double cost = 600.0;
-                for (int s = s0; s < s0 + ns; ++s) {
-                    const int nkc = (g.segs[s].K + BKC - 1) / BKC;
-                    cost += nkc * panel + ((nkc + GKC - 1) / GKC) * 1800.0;
-                }
-                const double tiles = (double)((group_rows(gr) + R - 1) / R) * ((group_cols(gr) + BN - 1) / BN);
+            for (const GroupCost &c : gc) {
+                const double cost = 600.0 + c.panels * panel + c.drains * 1800.0;
+                const double tiles = (double)((c.rows + R - 1) >> log_r) * c.col_packs;
                 sum += tiles * cost;
                 n += tiles;
                 top = std::max(top, cost);
@@ -1132,14 +1143,25 @@ void plan_mixed(GemmPlan &g) {
         SliceJob &j = (is_b ? bjobs : ajobs)[p.job0 + piece];
         j.entry = std::min(j.entry, entry);
     };
-    auto add_map = [&](const Piece *pc, const Piece *pe, int n) {  // (piece, row) of each of n panel rows
+    // (piece, row) of each of n panel rows; packs of one piece of the same rows share
+    // a map (a plan of many blocks that do not pack is mostly such)
+    struct {
+        int r0, rows, n, at;
+    } last[2] = {{0, -1, 0, 0}, {0, -1, 0, 0}};
+    auto add_map = [&](const Piece *pc, const Piece *pe, int n, bool is_b) {
+        auto &l = last[is_b];
+        const bool one = pe - pc == 1;
+        if (one && l.r0 == pc->r0 && l.rows == pc->rows && l.n == n) return l.at;
         const int at = (int)maps.size();
-        maps.resize((size_t)at + n, make_int2(-1, 0));
-        int r0 = at;
+        if (one) l = {pc->r0, pc->rows, n, at};
+        maps.resize((size_t)at + n);
+        int2 *m = maps.data() + at;
         for (int i = 0; pc != pe; ++i, ++pc) {
-            for (int r = 0; r < pc->rows; ++r) maps[r0 + r] = make_int2(i, pc->r0 + r);
-            r0 += pad8(pc->rows);
+            int2 *const end = m + pad8(pc->rows);
+            for (int r = pc->r0; r < pc->r0 + pc->rows; ++r) *m++ = make_int2(i, r);
+            while (m != end) *m++ = make_int2(-1, 0);
         }
+        for (int2 *const end = maps.data() + at + n; m != end; ++m) *m = make_int2(-1, 0);
         return at;
     };
     auto &rp = w.rp, &cp = w.cp;
@@ -1149,6 +1171,20 @@ void plan_mixed(GemmPlan &g) {
     for (size_t x = 0; x < w.ngroups; ++x) {
         const Group &gr = groups[x];
         rows.clear();
+        if (!gr.multi && gr.rblk.size() == 1 && gr.cview.size() == 1 && av[gr.rblk[0]].rows <= most &&
+            bv[gr.cview[0]].rows <= BN) {  // one block, one tile
+            const OutBlock &b = cell(gr, 0, 0);
+            const int e = g.segs[b.sb].entry;
+            const Piece r{gr.rblk[0], 0, b.M, 0}, c{gr.cview[0], 0, b.N, 0};
+            const Panel a1 = add_pack(&r, &r + 1, pad8(b.M), false, own_view);
+            const Panel b1 = add_pack(&c, &c + 1, BN, true, own_view);
+            ajobs[a1.job0].entry = bjobs[b1.job0].entry = e;
+            tiles.push_back({pad8(b.M), (int)xsegs.size(), (int)xsegs.size() + 1, add_map(&r, &r + 1, pad8(b.M), false),
+                             add_map(&c, &c + 1, BN, true), (int)pairs.size(), 1});
+            xsegs.push_back(SegX{a1.pan, b1.pan, (av[r.view].K + BKC - 1) / BKC, a1.exp, b1.exp, e});
+            pairs.push_back({b.c_off, b.ldc, e});
+            continue;
+        }
         if (!gr.multi) {
             for (int a : gr.rblk) rows.push_back(av[a].rows);
             make_packs(gr.rblk, rows, most, &rp, &rpc);
@@ -1158,34 +1194,36 @@ void plan_mixed(GemmPlan &g) {
             ap.clear(), bp.clear(), rmap.clear(), cmap.clear();
             for (auto &p : rp) {
                 ap.push_back(add_pack(rpc.data() + p.begin, rpc.data() + p.end, p.rows, false, own_view));
-                rmap.push_back(add_map(rpc.data() + p.begin, rpc.data() + p.end, p.rows));
+                rmap.push_back(add_map(rpc.data() + p.begin, rpc.data() + p.end, p.rows, false));
             }
             for (auto &p : cp) {
                 bp.push_back(add_pack(cpc.data() + p.begin, cpc.data() + p.end, p.rows, true, own_view));
-                cmap.push_back(add_map(cpc.data() + p.begin, cpc.data() + p.end, BN));
+                cmap.push_back(add_map(cpc.data() + p.begin, cpc.data() + p.end, BN, true));
             }
             const int nkc = (av[gr.rblk[0]].K + BKC - 1) / BKC;
             // kColBatch column packs meet every row pack before the next ones, so
             // the panels of the tiles in flight stay in L2 (all columns a row pack
             // at a time read B's panels from HBM once per row pack)
             constexpr size_t kColBatch = 16;
+            int ns = (int)xsegs.size(), nt = (int)tiles.size(), np = (int)pairs.size();
+            xsegs.resize(ns + rp.size() * cp.size());
+            tiles.resize(nt + rp.size() * cp.size());
+            pairs.resize(np + rpc.size() * cpc.size());
             for (size_t j0 = 0; j0 < cp.size(); j0 += kColBatch)
                 for (size_t i = 0; i < rp.size(); ++i)
                     for (size_t j = j0; j < std::min(cp.size(), j0 + kColBatch); ++j) {
-                        TcTile t{rp[i].rows, (int)xsegs.size(), (int)xsegs.size() + 1, rmap[i], cmap[j],
-                                 (int)pairs.size(), cp[j].end - cp[j].begin};
+                        tiles[nt++] = {rp[i].rows, ns, ns + 1, rmap[i], cmap[j], np, cp[j].end - cp[j].begin};
                         int entry = kAllSteps;
                         for (int u = rp[i].begin; u < rp[i].end; ++u)
                             for (int v = cp[j].begin; v < cp[j].end; ++v) {
                                 const OutBlock &b = cell(gr, rpc[u].unit, cpc[v].unit);
                                 const int e = g.segs[b.sb].entry;
-                                pairs.push_back({b.c_off, b.ldc, e});
+                                pairs[np++] = {b.c_off, b.ldc, e};
                                 entry = std::min(entry, e);
                                 seen(ap[i], false, u - rp[i].begin, e);
                                 seen(bp[j], true, v - cp[j].begin, e);
                             }
-                        xsegs.push_back(SegX{ap[i].pan, bp[j].pan, nkc, ap[i].exp, bp[j].exp, entry});
-                        tiles.push_back(t);
+                        xsegs[ns++] = SegX{ap[i].pan, bp[j].pan, nkc, ap[i].exp, bp[j].exp, entry};
                     }
             continue;
         }
@@ -1195,11 +1233,11 @@ void plan_mixed(GemmPlan &g) {
         cmap.clear();
         for (int n0 = 0; n0 < N; n0 += BN) {
             const Piece c{0, n0, std::min(BN, N - n0), 0};
-            cmap.push_back(add_map(&c, &c + 1, BN));
+            cmap.push_back(add_map(&c, &c + 1, BN, true));
         }
         for (size_t i = 0; i < rp.size(); ++i) {
             const Piece *p0 = rpc.data() + rp[i].begin, *p1 = rpc.data() + rp[i].end;
-            const int rm = add_map(p0, p1, rp[i].rows);
+            const int rm = add_map(p0, p1, rp[i].rows, false);
             ap.clear();
             for (int s = 0; s < ns; ++s)
                 ap.push_back(add_pack(p0, p1, rp[i].rows, false,
@@ -1237,17 +1275,23 @@ void plan_mixed(GemmPlan &g) {
         for (int m0 = 0; m0 < b.M; m0 += BM)
             for (int n0 = 0; n0 < b.N; n0 += BN) {
                 const Piece r{0, m0, std::min(BM, b.M - m0), 0}, c{0, n0, std::min(BN, b.N - n0), 0};
-                const int rm = add_map(&r, &r + 1, pad8(r.rows)), cm = add_map(&c, &c + 1, BN);
+                const int rm = add_map(&r, &r + 1, pad8(r.rows), false), cm = add_map(&c, &c + 1, BN, true);
                 tiles.push_back(TcTile{pad8(r.rows), (int)xsegs.size(), (int)xsegs.size(), rm, cm,
                                        (int)pairs.size(), 1});
                 pairs.push_back({b.c_off, b.ldc, kAllSteps});
             }
     }
     auto &aitems = w.aitems, &bitems = w.bitems;
-    for (size_t i = 0; i < ajobs.size(); ++i)
-        for (int r0 = 0; r0 < ajobs[i].rows; r0 += 8) aitems.push_back({(int)i, r0});
-    for (size_t i = 0; i < bjobs.size(); ++i)
-        for (int r0 = 0; r0 < bjobs[i].rows; r0 += 8) bitems.push_back({(int)i, r0});
+    auto add_items = [](const std::vector<SliceJob> &jobs, std::vector<int2> &items) {
+        size_t n = 0;
+        for (auto &j : jobs) n += (j.rows + 7) / 8;
+        items.resize(n);
+        int2 *o = items.data();
+        for (size_t i = 0; i < jobs.size(); ++i)
+            for (int r0 = 0; r0 < jobs[i].rows; r0 += 8) *o++ = make_int2((int)i, r0);
+    };
+    add_items(ajobs, aitems);
+    add_items(bjobs, bitems);
     KV_REQUIRE(g.a_exps < (1ll << 31) && g.b_exps < (1ll << 31) && maps.size() < (1ull << 31) &&
                    pairs.size() < (1ull << 31),
                KV_EINVAL, "mixed-precision plan too large");
@@ -1342,7 +1386,7 @@ static char *context_slices(int64_t bytes) {
 void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, double2 *C, double alpha,
                        const int *skip, int step) {
     if (p.tiles.empty()) return;
-    KV_REQUIRE(p.tile_m == BM && p.tile_n == BN && p.tc_tiles > 0, KV_EINVAL,
+    KV_REQUIRE(p.tile_m == kMixedBlock && p.tile_n == kMixedBlock && p.tc_tiles > 0, KV_EINVAL,
                "internal: GEMM plan not prepared for the tensor-core path");
     auto &c = ctx();
     int *err = device_err_word(c.device);
