@@ -380,8 +380,9 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                         cr = fma(xv[e].x, yv[e].x, fma(xv[e].y, yv[e].y, cr));
                         ci = fma(xv[e].x, yv[e].y, fma(-xv[e].y, yv[e].x, ci));
                     }
-                } else {
+                } else {  // four elements in flight a lane (the compiler's own choice: 5 to 15 % longer splits)
                     if (act)
+#pragma unroll 4
                         for (int i = gl; i < p; i += G) {
                             const double2 xi = ldg2(x + i), yi = ldg2(y + i);
                             a = fma(xi.x, xi.x, fma(xi.y, xi.y, a));
@@ -419,6 +420,7 @@ __global__ void __launch_bounds__(NT) k_svd64(const Svd64Sector *__restrict__ se
                         }
                     }
                 } else {
+#pragma unroll 4
                     for (int i = gl; i < p; i += G) {
                         const double2 xo = ldg2(x + i), yo = ldg2(y + i);
                         stg2(x + i, make_double2(fma(cs, xo.x, -fma(sr, yo.x, si * yo.y)),
