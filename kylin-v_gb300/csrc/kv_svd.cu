@@ -1375,17 +1375,21 @@ bool svd_qrjacobi_f32(const SvdPlan &p, const double2 *T64, float2 *Us, double *
     if (smem > (size_t)limit) return false;
     // The register-resident Jacobi where its exchange columns also fit, on a
     // cluster of CTAs a sector: a round's rotations and column moves bound one
-    // SM, and a bond's sectors leave most SMs idle.  Measured, the whole split of
-    // 17 sectors of 128 x 128: one CTA 1985 us, two 1727, four 1631, eight 1799 (a
-    // larger cluster's barrier costs more than its shorter round saves); four
-    // reach 1580 with the reduction's rows dealt as well.
+    // SM, and a bond's sectors leave most SMs idle.  Up to 64 columns a pair has 16
+    // lanes and a round is so short that the cluster's barrier costs more than its
+    // share saves; beyond, four CTAs are best (two where four do not fit, eight no
+    // better for few sectors and worse for many).  Measured, us a split with 1, 2, 4
+    // and 8 CTAs a sector: one sector of 48 x 48 552, 620, 588, 566; of 64 x 64 763,
+    // 833, 787, 749; of 72 x 72 1193, 1171, 1061, 1040; of 128 x 128 2661, 2222, 1994,
+    // 1937; 17 sectors of 48 x 48 636, 710, 681, 928; of 64 x 64 859, 911, 879, 1243;
+    // of 72 x 72 1358, 1332, 1211, 1887; of 128 x 128 3399, 2866, 2616, 3794.
     const int nsec = (int)p.secs.size(), sms = ctx().num_sms;
     const int rows = max_p <= 32 ? 32 : max_p <= 64 ? 64 : 128;  // 8 EPL of the kernel launched below
     int C = 1, slots = 0, bufs = 1;
     if (max_p <= 128) {
         int kmax = 1;
         for (auto &sc : p.secs) kmax = std::max(kmax, std::min(sc.p, sc.q));
-        while (C < 4 && 2 * C * nsec <= sms && kmax >= 32 * C) C *= 2;
+        while (C < 4 && 2 * C * nsec <= sms && kmax > 64) C *= 2;
         for (bufs = 2; bufs >= 1; --bufs) {
             size_t need = 0;
             const int sl = qrj_slots(kmax, C);
