@@ -41,3 +41,20 @@ def test_faint_rows_and_columns(gpu, m, n, faint, power, l2r):
         assert np.abs(orth.conj().T @ orth - np.eye(k)).max() <= 1e-12
         assert np.abs(x @ y - z).max() <= 1e-5 * s[0]
         assert np.abs(np.linalg.norm(other, axis=1) - s[:k]).max() <= max(m, n) * 1e-10 * s[0]
+
+
+@pytest.mark.parametrize("l2r", [True, False])
+@pytest.mark.parametrize("m,n", [(64, 64), (64, 90), (65, 65), (66, 100), (100, 65)])
+def test_either_side_of_the_cluster_rule(gpu, m, n, l2r):
+    """64 columns take one CTA, 65 a cluster: the bits of the same sector among so many that each gets one CTA."""
+    rng = np.random.default_rng([m, n])
+    a = rng.normal(size=(m, n)) + 1j * rng.normal(size=(m, n))
+    out = []
+    for others in (0, 159):
+        mats = [a] + [np.full((1, 1), 1.0 + q) for q in range(others)]
+        t = BlockTensor((1, -1), [((q, q), x) for q, x in enumerate(mats)])
+        L, R, _, _ = gpu.svd_impl(t, 1, l2r, 0.0, min(m, n) + others, precision=gpu.KV_MIXED_TF32)
+        out.append((dict(L.to_host().blocks)[(0, 0)], dict(R.to_host().blocks)[(0, 0)]))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    x, y = out[0]
+    assert np.abs(x @ y - a).max() <= 1e-5 * np.linalg.svd(a, compute_uv=False)[0]
