@@ -1416,16 +1416,21 @@ void launch_gemm_mixed(const GemmPlan &p, const double2 *A, const double2 *B, do
         const int per = kSliceWarps / GW, ctas = (items + per - 1) / per;
         const SliceLimits lim = slice_limits(c.device);
         const bool main = &c == &main_ctx();
-        // Little work: one cluster (its barrier is cheaper than a grid's: 8.8
-        // against 12.5 us at D = 32), at most two rounds of four steps a warp, six
-        // on a worker stream where it also saves a launch; more: the whole
-        // chip, on the main stream in one cooperative launch (that stream's
-        // kernels never overlap, so its grid barrier waits on no other launch)
+        // Little work, at most two rounds of four steps a warp: one cluster, whose
+        // barrier is cheaper than a grid's or a second launch.  More: the whole chip,
+        // on the main stream in one cooperative launch (that stream's kernels never
+        // overlap, so its grid barrier waits on no other launch).  Measured, us a step
+        // with up to 0, 1, 2, 3, 4 and 6 rounds in a cluster: one chain on the main
+        // stream, D = 32 one-site 28830, 26860, 26761, 26880, 26837, 26878; D = 96 two-site
+        // 91121, 89960, 89831, 90134, 91598, 93476; four chains on worker streams,
+        // D = 32 35412, 33615, 34018, 34548, 34728, 34295; D = 96 two-site 121025, 121727,
+        // 122222, 122440, 123079, 125065; D = 128 two-site 148949, 148314, 147041, 148498,
+        // 148834, 153003.
         const int64_t rounds = (int64_t)((ctas + lim.cluster - 1) / lim.cluster) * ((p.max_k + 32 * GW - 1) / (32 * GW));
         if (!a.kmax) {
             launch_dependent(k_slice_put, (unsigned)ctas, 32 * kSliceWarps, 0, 0, a, GW, skip);
             ++n;
-        } else if (rounds <= (main ? 2 : 6)) {
+        } else if (rounds <= 2) {
             int size = 1;
             while (size < lim.cluster && size < ctas) size *= 2;
             launch_dependent(k_slice_cluster, (unsigned)size, 32 * kSliceWarps, 0, (unsigned)size, a, GW, skip);
