@@ -4,14 +4,16 @@
 // Each charge sector's dense matrix is gathered as T (p x q, column-major;
 // T = A or T = A^H) and factorised:
 //  * FP64 mode: kv_svd64.cu;
-//  * mixed mode, one CTA a sector: T oriented so the wanted singular vectors are its columns, a
+//  * mixed mode: T oriented so the wanted singular vectors are its columns, a
 //    pivoted Householder reduction of its rows to the numerical rank, then
 //    FP32 one-sided Jacobi on the rank-r factor, all in shared memory
-//    (k_svd_qrj, the Jacobi with the columns in registers); sectors beyond
-//    shared memory take the same reduction on an L2-resident workspace
-//    (k_svd_qr_g) and the global-memory Jacobi (k_svd_jacobi_w).  The FP64
-//    rebuild of the kept factor (k_svd_extract, k_col_norm2, k_chol,
-//    k_trsm_rows with the FP64 GEMM) runs after the host's truncation.
+//    (k_svd_qrj: a cluster of up to four CTAs a sector, the reduction's rows and
+//    the Jacobi's columns dealt over them, or one CTA; the Jacobi with the columns
+//    in registers); sectors beyond shared memory take the same reduction on an
+//    L2-resident workspace (k_svd_qr_g) and the global-memory Jacobi
+//    (k_svd_jacobi_w), one CTA each.  The FP64 rebuild of the kept factor
+//    (k_svd_extract, k_col_norm2, k_chol, k_trsm_rows with the FP64 GEMM) runs
+//    after the host's truncation.
 // The host applies the reference's global truncation and the scatter kernel
 // writes the kept columns into the U and S.V^H block tensors; the SA split's
 // new directions come from k_sa_basis / k_sa_subtract / k_sa_scatter.
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(NT) k_svd_jacobi_w(const SvdSector *__restrict
                     cr += __shfl_xor_sync(gmask, cr, o, G);
                     ci += __shfl_xor_sync(gmask, ci, o, G);
                 }
-                // the rotation of kvj::make_rotation, keeping tan(theta) for the norm update:
+                // the Jacobi rotation (kv_jacobi.cuh), keeping tan(theta) for the norm update:
                 // the new squared norms are a - tan |c| and b + tan |c|
                 const float ac = sqrtf(cr * cr + ci * ci);
                 if (!(ac > tol * sqrtf(a * b))) continue;
@@ -551,12 +553,12 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
     return converged ? sweep : -sweep;
 }
 
-// QR-preconditioned one-sided Jacobi (mixed mode).  One CTA of 512 threads
-// per charge sector; the sector is held in shared memory in FP32 as p rows of
-// length q (row stride q + 1, so reads of one column by consecutive rows fall
-// in distinct banks), scaled by a power of two so that its largest element
-// lies in [0.5, 1).  The wanted singular vectors are T's left ones (its
-// column space).
+// QR-preconditioned one-sided Jacobi (mixed mode).  A cluster of C CTAs of 512
+// threads per charge sector (C = 4, 2 or 1: svd_qrjacobi_f32); every CTA holds
+// the sector in shared memory in FP32 as p rows of length q (row stride q + 1,
+// so reads of one column by consecutive rows fall in distinct banks), scaled by
+// a power of two so that its largest element lies in [0.5, 1).  The wanted
+// singular vectors are T's left ones (its column space).
 //
 //  1. Pivoted Householder from the right on T's rows: at step k the row with
 //     the largest trailing norm (positions k..q-1) is the pivot; the unitary
@@ -565,17 +567,24 @@ __device__ __forceinline__ int qrj_jacobi_reg(float2 *sw, int ldw, int p, int r,
 //     T H_1 ... H_r = [M | E]: M = T Q (p x r, Q the first r columns of the
 //     product) and E has rows of norm below qr_floor * ||T||_F, where the loop
 //     stops.  T = M Q^H + E Q'^H, so T's left singular vectors above the FP32
-//     noise level are M's.  One barrier per step: every warp finds the next
-//     pivot itself from the per-warp maxima of the previous step (double
-//     buffered), and each row's exact trailing norm is accumulated while the
-//     row is updated.  A group of 16 lanes updates two rows at once, so each
-//     pivot-row element it loads serves both.
-//  2. One-sided Jacobi on M's r columns (qrj_jacobi: round-robin pairs, 32,
-//     16 or 8 lanes a pair for r <= 32, <= 64 or more, so that a round's r/2
-//     pairs occupy most warps; each lane holds its elements of both columns in
-//     registers between the dot product and the rotation, 8 EPL rows per pair
-//     in all; tolerance `tol` on the cosine).  M is row-pivoted triangular, so
-//     it converges in fewer sweeps than T, and only r columns are rotated.
+//     noise level are M's.  One CTA alone needs one barrier per step: every
+//     warp finds the next pivot itself from the per-warp maxima of the previous
+//     step (double buffered), and each row's exact trailing norm is accumulated
+//     while the row is updated.  A group of 16 lanes updates two rows at once,
+//     so each pivot-row element it loads serves both.  In a cluster CTA i
+//     updates rows i, i + C, ...; after a step (a CTA barrier) it sends its best
+//     candidate, norm and row, to every CTA's shared memory, a cluster barrier
+//     follows, and all pick the same next pivot row.  The rows are exchanged
+//     once at the end.
+//  2. One-sided Jacobi on M's r columns.  qrj_jacobi_reg where the exchange
+//     columns fit and r <= 128: each group of 32, 16 or 8 lanes (r <= 32, <= 64
+//     or more) holds a pair of columns in registers for a whole sweep, the
+//     groups dealt over the cluster, one column a group moved and one barrier
+//     taken a round.  qrj_jacobi else, on the first CTA alone: round-robin pairs,
+//     each lane holding its elements of both columns in registers between the
+//     dot product and the rotation (8 EPL rows per pair in all).  Tolerance `tol`
+//     on the cosine.  M is row-pivoted triangular, so it converges in fewer
+//     sweeps than T, and only r columns are rotated.
 //  3. Columns sorted by norm: S = norms (descending), Us = normalised columns
 //     (column-major p x r at the sector's t_off), S = 0 in the sector's
 //     remaining slots up to q.
