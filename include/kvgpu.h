@@ -76,7 +76,15 @@ extern "C" {
 typedef struct kv_tensor_s *kv_tensor;
 typedef struct kv_tdvp_s *kv_tdvp;
 
-/* Library lifetime: select the device and create the stream / pools. */
+/* Library lifetime: select the device and create the stream / pools.
+ * Device memory that stays with the library until kv_shutdown, beside the
+ * caller's tensors: per stream (the main one and each worker of
+ * kv_sweep_batched) a workspace of sliced GEMM panels that grows to at most
+ * 64 MiB with the mixed calls made on it, and their balancing maxima (a few
+ * kB); freed blocks stay in the device pool.  Host memory: each thread's
+ * planning lists, a few MiB at most.  FP64 results are reproducible on one GPU
+ * model; sums are cut by the device's SM count and the call's block list, so
+ * models with another number of SMs round differently in the last bits. */
 int kv_init(int device);
 int kv_shutdown(void);
 const char *kv_last_error(void);
