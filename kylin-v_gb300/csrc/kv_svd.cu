@@ -851,9 +851,11 @@ __global__ void __launch_bounds__(512, 1) k_svd_qrj(const SvdSector *__restrict_
     float fro2 = 0.f;
     // The reduction's candidate rows use the exchange columns' memory; where they
     // do not fit every CTA reduces the whole sector alone.  A step's row updates
-    // bound one SM more than the cluster barrier that dealing them adds: the split
-    // of 17 sectors of 128 x 128 takes 1651 us with every CTA reducing alone, 1580
-    // with the rows dealt (1587 if only sectors of more than 64 rows are).
+    // bound one SM more than the cluster barrier that dealing them adds, from about
+    // 80 rows on, and it makes no difference below: us a split with the rows dealt
+    // and with every CTA reducing alone, one sector of 72 x 72 1056 and 1056, of 96 x
+    // 96 1487 and 1524, of 128 x 128 1993 and 2034; 17 sectors of 72 x 72 1213 and 1208,
+    // of 80 x 80 1430 and 1438, of 128 x 128 2623 and 2663.
     const bool deal = C > 1 && slots > 0 &&
                       (size_t)2 * C * q * sizeof(float2) <= qrj_xch_bytes(8 * (EPL > 0 ? EPL : 1), slots, bufs);
     const int r = qrj_reduce(s, T64, sw, ldw, alph, piv, done, qr_floor, &up, &fro2, deal ? C : 1, deal ? rank : 0,
